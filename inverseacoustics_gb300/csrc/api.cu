@@ -1232,7 +1232,7 @@ int ia_sinc_resistance_batch(ia_context *ctx, int n, const double *d_x, int F, c
     if (!ctx || n < 1 || F < 1 || !d_x || !d_k || !d_R || !(area > 0.0)) return IA_ERR_ARG;
     ia_config dc;
     if (!cfg) { ia_config_default(&dc); cfg = &dc; }
-    return sinc_resistance_batched(ctx, n, d_x, F, d_k, area, cfg->c, cfg->rho, d_R, nullptr);
+    return sinc_resistance_batched(ctx, n, d_x, F, d_k, area, cfg->c, cfg->rho, d_R);
 }
 
 int ia_radiation_modes_batch(ia_context *ctx, int n, int F, const double *d_R, int nmodes, const ia_config *cfg,

@@ -295,9 +295,9 @@ int hels_batched(ia_context *ctx, int npts, const double *pts, int order, int F,
                  double rho, double2 *Me, double2 *Qe);
 
 // ---- radiation modes (radiation.cu)
-// R (F x n x n FP64) and optionally an FP32 copy R32
+// R (F x n x n FP64), exactly symmetric
 int sinc_resistance_batched(ia_context *ctx, int n, const double *x, int F, const double *k, double area, double c,
-                            double rho, double *R, float *R32);
+                            double rho, double *R);
 // leading eigenpairs of the symmetric R, or (gram) of R R^T for a general R:
 // left singular vectors, lambda = squared singular values
 size_t radiation_modes_ws_bytes(int n, int F, int nm, const ia_config *cfg, bool gram = false);
