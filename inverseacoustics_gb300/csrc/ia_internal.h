@@ -179,6 +179,7 @@ int df_hi_batched(ia_context *ctx, size_t count, const float4 *in, float2 *out);
 #define TC_SLICES_MIN 6
 #define TC_SLICES_MAX 8
 #define TC_SLICES_DEFAULT 7
+#define TC_SLICES_FP64 10   // the FP64 path's products: rounding below an FP64 GEMM's
 struct TcPlanes {
     __nv_bfloat16 *p;   // [batch][S][rows][Kp] BF16 digits
     int *e;             // [batch][R] power-of-two scale exponents
@@ -191,6 +192,14 @@ inline bool tc_products_ok(int S, int K)
 {
     return S >= TC_SLICES_MIN && S <= TC_SLICES_MAX && (long long)S * 1024 * ((2 * K + 7) & ~7) <= (1ll << 24);
 }
+// the FP64 path's products on TC_SLICES_FP64 slices, complex and real
+inline bool tc_fp64_ok(int K) { return (long long)TC_SLICES_FP64 * 1024 * ((2 * K + 7) & ~7) <= (1ll << 24); }
+inline bool tc_real_ok(int K) { return (long long)TC_SLICES_FP64 * 1024 * ((K + 7) & ~7) <= (1ll << 24); }
+size_t tc_planes_real_bytes(int R, int K, int batch);
+int tc_slice_real(ia_context *ctx, bool role_b, Op op, const double *X, int ld, long long sX, int R, int K, int batch,
+                  TcPlanes &out, WsCursor &cur);
+int tc_gemm_real(ia_context *ctx, const TcPlanes &A, const TcPlanes &B, int M, int N, double alpha, double beta,
+                 double *C, int ldc, long long sC, int batch, int *info);
 // role_b false: A (M x K) = op(X); true: B (K x N) = op(X); R = M or N
 int tc_slice(ia_context *ctx, bool role_b, Op op, const double2 *X, int ld, long long sX, int R, int K, int S,
              int batch, TcPlanes &out, WsCursor &cur);

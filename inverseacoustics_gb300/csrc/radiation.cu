@@ -307,6 +307,37 @@ static int prod64(ia_context *ctx, bool df, Op opa, int M, int N, int K, const d
     return rgemm_batched<double>(ctx, opa, M, N, K, 1.0, A, lda, sA, B, ldb, sB, 0.0, C, ldc, sC, batch);
 }
 
+// The FP64 path's subspace products on the tensor cores: the operator (R, and
+// R^T for gram) is cut into slice planes once per call, a block of vectors per
+// product.  On the FP64 pipe the 11 products of 16 bins (1280 x 1280 x 40) ran
+// 4.0 ms each, 84 % of the call; on slices 0.27 ms (two waves of 128-row
+// tiles, bound by the MMAs' shared-memory operand reads).  From n = 96: below, one 128-row tile is mostly
+// padding and the FP64 product takes microseconds.  The planes take 20 n^2
+// bytes per bin and operator, so a call works through groups of bins that
+// keep them within RM_PLANE_BYTES.
+constexpr int RM_TC_MIN_N = 96;
+constexpr size_t RM_PLANE_BYTES = size_t(6) << 30;
+
+static bool modes_tc(int n, const ia_config *cfg)
+{
+    return cfg->precision != IA_PREC_MIXED && n >= RM_TC_MIN_N && tc_real_ok(n);
+}
+
+static size_t modes_op_bytes(int n, int b, int F, bool gram)
+{
+    return (gram ? 2 : 1) * tc_planes_real_bytes(n, n, F) + 2 * tc_planes_real_bytes(b, n, F) + 1024;
+}
+
+// bins per group
+static int modes_group(int n, int b, int F, const ia_config *cfg, bool gram)
+{
+    if (!modes_tc(n, cfg)) return F;
+    const size_t one = modes_op_bytes(n, b, 1, gram);
+    const size_t g = RM_PLANE_BYTES / one;
+    const int groups = (int)((F + (g ? g : 1) - 1) / (g ? g : 1));
+    return (F + groups - 1) / groups;
+}
+
 // --------------------------------------------------------------------------
 // Real Householder QR of a tall block (rows x cols, one CTA per matrix):
 // H_j = I - tau v v^T, v(j) = 1, beta = -sign(alpha) ||x|| (LAPACK dlarfg
@@ -916,19 +947,19 @@ __global__ void mode_sign_kernel(int n, int nm, double *__restrict__ X, const do
 size_t radiation_modes_ws_bytes(int n, int F, int nm, const ia_config *cfg, bool gram)
 {
     const size_t b = (size_t)min(n, nm + max(0, cfg->mode_oversample));
+    F = modes_group(n, (int)b, F, cfg, gram);
     const size_t nb = (size_t)n * b * F, bb = b * b * F;
     size_t s = 4 * ws_round(8 * nb) + ws_round(8 * b * F) + ws_round(8 * bb) + 4 * ws_round(16 * bb) +
                ws_round(8 * b * F) + ws_round(8 * b * (size_t)nm * F);
     if (cfg->precision == IA_PREC_MIXED)
         s += ws_round(4 * (size_t)n * n * F) + 3 * ws_round(4 * nb) + ws_round(4 * b * F);
-    (void)gram;
+    if (modes_tc(n, cfg)) s += modes_op_bytes(n, (int)b, F, gram);
     return s + 4096;
 }
 
-// gram: the operator is R R^T (R general, n x n): its eigenpairs are the left
-// singular vectors and the squared singular values of R
-int radiation_modes_batched(ia_context *ctx, int n, int F, const double *R, int nm, const ia_config *cfg,
-                            double *lambda, double *modes, int *info, WsCursor &cur, bool gram)
+// one group of bins
+static int radiation_modes_group(ia_context *ctx, int n, int F, const double *R, int nm, const ia_config *cfg,
+                                 double *lambda, double *modes, int *info, WsCursor &cur, bool gram)
 {
     const int b = min(n, nm + max(0, cfg->mode_oversample));
     const bool mixed = cfg->precision == IA_PREC_MIXED;
@@ -937,8 +968,20 @@ int radiation_modes_batched(ia_context *ctx, int n, int F, const double *R, int 
     double *Y = cur.take<double>(nb * F);
     double *Y2 = cur.take<double>(nb * F);
     double *Tg = cur.take<double>(nb * F);
+    const bool tcp = modes_tc(n, cfg);
+    TcPlanes Pr{}, Pt{};   // slice planes of R and (gram) R^T
     // Yo = op Qi at FP64 accuracy, op = R or R R^T
     auto apply64 = [&](const double *Qi, double *Yo) -> int {
+        if (tcp) {
+            WsCursor cq = cur;   // the vectors' planes: the workspace past the operator's, per product
+            TcPlanes Pq{};
+            int s2 = tc_slice_real(ctx, true, OP_N, Qi, n, nb, b, n, F, Pq, cq);
+            if (!gram) return s2 ? s2 : tc_gemm_real(ctx, Pr, Pq, n, b, 1.0, 0.0, Yo, n, nb, F, info);
+            if (!s2) s2 = tc_gemm_real(ctx, Pt, Pq, n, b, 1.0, 0.0, Tg, n, nb, F, info);
+            cq = cur;
+            if (!s2) s2 = tc_slice_real(ctx, true, OP_N, Tg, n, nb, b, n, F, Pq, cq);
+            return s2 ? s2 : tc_gemm_real(ctx, Pr, Pq, n, b, 1.0, 0.0, Yo, n, nb, F, info);
+        }
         if (!gram) return prod64(ctx, mixed, OP_N, n, b, n, R, n, nn, Qi, n, nb, Yo, n, nb, F);
         int s2 = prod64(ctx, mixed, OP_T, n, b, n, R, n, nn, Qi, n, nb, Tg, n, nb, F);
         return s2 ? s2 : prod64(ctx, mixed, OP_N, n, b, n, R, n, nn, Tg, n, nb, Yo, n, nb, F);
@@ -977,6 +1020,10 @@ int radiation_modes_batched(ia_context *ctx, int n, int F, const double *R, int 
         if ((st = convert(ctx, (size_t)nb * F, Q32, Q))) return st;
         steps64 = max(1, cfg->refine_steps);
     } else {
+        if (tcp) {
+            if ((st = tc_slice_real(ctx, false, OP_N, R, n, nn, n, n, F, Pr, cur))) return st;
+            if (gram && (st = tc_slice_real(ctx, false, OP_T, R, n, nn, n, n, F, Pt, cur))) return st;
+        }
         start_block_kernel<double><<<blocks, 256, 0, ctx->stream>>>(n, b, Q, F);
         IA_LAUNCH_CHECK(ctx);
     }
@@ -986,7 +1033,16 @@ int radiation_modes_batched(ia_context *ctx, int n, int F, const double *R, int 
     }
     // Rayleigh-Ritz: B = Q^T op Q, eigenpairs of B, modes = Q W
     if ((st = apply64(Q, Y2))) return st;
-    if ((st = prod64(ctx, mixed, OP_T, b, b, n, Q, n, nb, Y2, n, nb, B, b, bb, F))) return st;
+    if (tcp) {
+        // (K = n on one tile per bin: 1.4 ms on the FP64 pipe)
+        WsCursor cq = cur;
+        TcPlanes Pq{}, Py{};
+        if ((st = tc_slice_real(ctx, false, OP_T, Q, n, nb, b, n, F, Pq, cq))) return st;
+        if ((st = tc_slice_real(ctx, true, OP_N, Y2, n, nb, b, n, F, Py, cq))) return st;
+        if ((st = tc_gemm_real(ctx, Pq, Py, b, b, 1.0, 0.0, B, b, bb, F, info))) return st;
+    } else if ((st = prod64(ctx, mixed, OP_T, b, b, n, Q, n, nb, Y2, n, nb, B, b, bb, F))) {
+        return st;
+    }
     // eigenpairs of the symmetric (positive semidefinite) B by the two-sided
     // FP64 Jacobi, eigenvectors accumulated from the identity, then ordered by
     // decreasing eigenvalue (was: a one-sided complex Jacobi SVD with a
@@ -1018,6 +1074,23 @@ int radiation_modes_batched(ia_context *ctx, int n, int F, const double *R, int 
         return st;
     mode_sign_kernel<<<F, 256, 0, ctx->stream>>>(n, nm, modes, lambda, info);
     IA_LAUNCH_CHECK(ctx);
+    return IA_OK;
+}
+
+// gram: the operator is R R^T (R general, n x n): its eigenpairs are the left
+// singular vectors and the squared singular values of R
+int radiation_modes_batched(ia_context *ctx, int n, int F, const double *R, int nm, const ia_config *cfg,
+                            double *lambda, double *modes, int *info, WsCursor &cur, bool gram)
+{
+    const int b = min(n, nm + max(0, cfg->mode_oversample));
+    const int fg = modes_group(n, b, F, cfg, gram);
+    for (int f0 = 0; f0 < F; f0 += fg) {
+        WsCursor c = cur;
+        const int st = radiation_modes_group(ctx, n, min(fg, F - f0), R + (size_t)f0 * n * n, nm, cfg,
+                                             lambda + (size_t)f0 * nm, modes + (size_t)f0 * nm * n, info + f0, c,
+                                             gram);
+        if (st) return st;
+    }
     return IA_OK;
 }
 

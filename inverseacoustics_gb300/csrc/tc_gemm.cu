@@ -22,7 +22,13 @@
 // rounding to S digits and the dropped pairs (s + t >= S): at most
 // (4 S + 8) 2^(-6 S) of max|A_row| max|B_col| per product term, 8e-12 at
 // S = 7 and 1.4e-13 at S = 8 (typical errors are far smaller) -- the
-// double-float GEMM's level.
+// double-float GEMM's level.  S = 10 (59-bit integers, 4e-17) serves the FP64
+// path: below an FP64 GEMM's own rounding for every row and column whose
+// entries span less than six bits more than its accumulated products, at 55
+// pair products against a scalar FP64 pipe of 1.1 TFLOP/s.
+//
+// Real operands (double) slice the same way without the complex embedding: K
+// values per row of A and column of B, one real output column per B column.
 //
 // Kernel.  One CTA per 128 output rows x 32 complex output columns of one
 // batch entry; 128 threads.  Warp 0 (one lane) loads, per K step of 32 real
@@ -38,6 +44,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <mutex>
+#include <type_traits>
 #include "ia_common.cuh"
 #include "ia_internal.h"
 #include "tc_ptx.cuh"
@@ -45,15 +52,17 @@
 namespace ia {
 
 constexpr int TC_BM = 128;        // output rows per CTA (TMEM lanes)
-constexpr int TC_BN = 64;         // real output columns per CTA (32 complex)
+// real output columns per CTA (two per complex column): S level accumulators
+// of this width share the 512 TMEM columns
+__host__ __device__ constexpr int tc_bn(int S) { return S <= 8 ? 64 : 48; }
 constexpr int TC_BK = 32;         // real K values per pipeline stage (64 bytes of BF16)
 constexpr int TC_STAGES = 2;
 constexpr int TC_THREADS = 128;
 constexpr uint64_t TC_WAIT_NS = 2000000000ull;
 constexpr uint32_t TC_A_SLICE = TC_BM * TC_BK * 2;   // bytes of one slice's A tile
-constexpr uint32_t TC_B_SLICE = TC_BN * TC_BK * 2;
+__host__ __device__ constexpr uint32_t tc_b_slice(int S) { return tc_bn(S) * TC_BK * 2; }
 
-size_t tc_smem_bytes(int S) { return (size_t)TC_STAGES * S * (TC_A_SLICE + TC_B_SLICE) + 1024; }
+size_t tc_smem_bytes(int S) { return (size_t)TC_STAGES * S * (TC_A_SLICE + tc_b_slice(S)) + 1024; }
 
 // ---------------------------------------------------------------------------
 // slicing
@@ -79,6 +88,24 @@ __device__ __forceinline__ int key_exponent(unsigned long long k, const double2 
 __device__ __forceinline__ int key_exponent(unsigned long long k, const float4 *)
 {
     return k ? (int)((k >> 23) & 0xFF) - 126 : 0;
+}
+
+// The FP64 path's operands may be anything an FP64 GEMM takes: rows below
+// 2^-964 keep the scale 2^-964 (2^q stays a normal number), and a row holding
+// an infinity or a NaN gets TC_EXP_NONFINITE, which makes its output row or
+// column NaN.
+constexpr int TC_EXP_NONFINITE = 1 << 20;
+template <int S>
+__device__ __forceinline__ int fp64_exponent(unsigned long long k)
+{
+    if (k >= 0x7FF0000000000000ull) return TC_EXP_NONFINITE;
+    const int e = key_exponent(k, (const double2 *)nullptr);
+    constexpr int emin = 5 + 6 * (S - 1) - 1023;
+    return e < emin ? emin : e;
+}
+__device__ __forceinline__ double fp64_scale(int e)
+{
+    return e == TC_EXP_NONFINITE ? __longlong_as_double(0x7FF8000000000000ll) : ldexp(1.0, e - 32);
 }
 
 // X = rint(v 2^q) for the real and imaginary parts (q: scale exponent)
@@ -317,9 +344,11 @@ __global__ void __launch_bounds__(SL1_THREADS, 2) tc_slice1_kernel(SliceOp<Src> 
         const unsigned long long ok = __shfl_xor_sync(0xffffffffu, key, o);
         key = ok > key ? ok : key;
     }
-    const int e = key_exponent(key, (const Src *)nullptr);
+    int e = key_exponent(key, (const Src *)nullptr);
+    if constexpr (S == TC_SLICES_FP64) e = fp64_exponent<S>(key);
     const int row = r0 + w;
     if (lane == 0) op.exps[(size_t)f * R + row] = e;
+    if (S == TC_SLICES_FP64 && e == TC_EXP_NONFINITE) e = 0;
     const int q = 5 - e + 6 * (S - 1);
     const int rows = op.role_b ? 2 * R : R;
     const size_t pstride = (size_t)rows * Kp;
@@ -366,22 +395,122 @@ __global__ void __launch_bounds__(SL1_THREADS, 2) tc_slice1_kernel(SliceOp<Src> 
     }
 }
 
+// The single-pass form for a real operand (S = TC_SLICES_FP64): SL1_RB rows of
+// the view per CTA in a shared-memory strip, a warp per row, four digits of
+// each plane (8 bytes) per lane and step.
+__host__ __device__ constexpr int slr_stride(int Kp) { return Kp + 2; }   // even: 16-byte rows
+
+__global__ void __launch_bounds__(SL1_THREADS, 2)
+    tc_slice_real_kernel(const double *__restrict__ Xb, int ld, long long sX, int R, int K, int Kp, int rcontig,
+                         __nv_bfloat16 *__restrict__ planes, int *__restrict__ exps)
+{
+    constexpr int S = TC_SLICES_FP64;
+    extern __shared__ __align__(16) unsigned char slr_smem[];
+    double *strip = reinterpret_cast<double *>(slr_smem);   // SL1_RB x slr_stride(Kp)
+    const int f = blockIdx.y, r0 = blockIdx.x * SL1_RB, t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int ks = slr_stride(Kp), nr = R - r0 < SL1_RB ? R - r0 : SL1_RB;
+    const double *__restrict__ X = Xb + f * sX;
+    [[maybe_unused]] const long long xext = rcontig ? (long long)ld * K : (long long)ld * R;
+    if (rcontig) {
+        const int r = lane & (SL1_RB - 1), kq = lane >> 3;
+        for (int kb = 4 * w; kb < Kp; kb += 4 * (SL1_THREADS / 32) * SL1_UNROLL) {
+            double v[SL1_UNROLL];
+#pragma unroll
+            for (int u = 0; u < SL1_UNROLL; ++u) {
+                const int k = kb + kq + 4 * (SL1_THREADS / 32) * u;
+                v[u] = r < nr && k < K && IA_IDX_OK((r0 + r) + (long long)k * ld, xext)
+                           ? X[(size_t)(r0 + r) + (size_t)k * ld]
+                           : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < SL1_UNROLL; ++u) {
+                const int k = kb + kq + 4 * (SL1_THREADS / 32) * u;
+                if (k < Kp) strip[(size_t)r * ks + k] = v[u];
+            }
+        }
+    } else {
+        const double *xr = X + (size_t)(r0 + w) * ld;
+        for (int kb = lane; kb < Kp; kb += 32 * SL1_UNROLL) {
+            double v[SL1_UNROLL];
+#pragma unroll
+            for (int u = 0; u < SL1_UNROLL; ++u) {
+                const int k = kb + 32 * u;
+                v[u] = w < nr && k < K && IA_IDX_OK((long long)(r0 + w) * ld + k, xext) ? xr[k] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < SL1_UNROLL; ++u) {
+                const int k = kb + 32 * u;
+                if (k < Kp) strip[(size_t)w * ks + k] = v[u];
+            }
+        }
+    }
+    __syncthreads();
+    if (w >= nr) return;
+    const double *srow = strip + (size_t)w * ks;
+    unsigned long long key = 0;
+    for (int k = lane; k < K; k += 32) {
+        const unsigned long long kk = __double_as_longlong(srow[k]) & 0x7FFFFFFFFFFFFFFFull;
+        key = kk > key ? kk : key;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long ok = __shfl_xor_sync(0xffffffffu, key, o);
+        key = ok > key ? ok : key;
+    }
+    int e = fp64_exponent<S>(key);
+    const int row = r0 + w;
+    if (lane == 0) exps[(size_t)f * R + row] = e;
+    if (e == TC_EXP_NONFINITE) e = 0;
+    const int q = 5 - e + 6 * (S - 1);
+    const size_t pstride = (size_t)R * Kp;
+    __nv_bfloat16 *__restrict__ P0 = planes + (size_t)f * S * pstride + (size_t)row * Kp;
+    for (int k = 4 * lane; k < Kp; k += 128) {   // Kp is a multiple of 8
+        long long x[4];
+        to_fixed(make_double2(srow[k], srow[k + 1]), q, x[0], x[1]);
+        to_fixed(make_double2(srow[k + 2], srow[k + 3]), q, x[2], x[3]);
+#pragma unroll
+        for (int s = S - 1; s >= 0; --s) {
+            int d[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (s > 0) {
+                    int r = (int)(x[j] & 63);
+                    if (r > 32) r -= 64;
+                    d[j] = r;
+                    x[j] = (x[j] - r) >> 6;
+                } else {
+                    d[j] = (int)x[j];
+                }
+            }
+            uint2 u;
+            u.x = bf2_bits(bf2(d[0], d[1]));
+            u.y = bf2_bits(bf2(d[2], d[3]));
+            if (IA_IDX_OK((long long)s * pstride + (long long)row * Kp + k + 3, (long long)S * pstride))
+                *reinterpret_cast<uint2 *>(P0 + (size_t)s * pstride + k) = u;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // the tensor-core GEMM on slice planes
 // ---------------------------------------------------------------------------
-template <int S>
+template <int S, bool REAL>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
                    int Kp, const int *__restrict__ ea, const int *__restrict__ eb, double alpha, double beta,
-                   double2 *__restrict__ C, int ldc, long long sC, int *info)
+                   typename std::conditional<REAL, double, double2>::type *__restrict__ C, int ldc, long long sC,
+                   int *info)
 {
+    constexpr int TC_BN = tc_bn(S);
+    constexpr int CPC = REAL ? 1 : 2;   // real columns per output column
+    constexpr uint32_t TC_B_SLICE = tc_b_slice(S);
     static_assert(S * TC_BN <= 512, "the S level accumulators must fit the 512 TMEM columns");
     constexpr uint32_t STAGE = S * (TC_A_SLICE + TC_B_SLICE);
     extern __shared__ unsigned char tc_smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[TC_STAGES], bar_empty[TC_STAGES], bar_done;
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
-    __shared__ double s_colscale[TC_BN / 2];
+    __shared__ double s_colscale[TC_BN / CPC];
     unsigned char *base = reinterpret_cast<unsigned char *>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t base_u = tc::smem_u32(base);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -398,9 +527,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         tc::prefetch_tmap(&tmB);
     }
     if (warp == 2) tc::tmem_alloc(tc::smem_u32(&s_tmem), 512);
-    if (threadIdx.x < TC_BN / 2) {
-        const int n = c0 / 2 + threadIdx.x;
-        s_colscale[threadIdx.x] = n < N ? ldexp(1.0, eb[(size_t)f * N + n]) : 0.0;
+    if (threadIdx.x < TC_BN / CPC) {
+        const int n = c0 / CPC + threadIdx.x;
+        if constexpr (S == TC_SLICES_FP64) s_colscale[threadIdx.x] = n < N ? fp64_scale(eb[(size_t)f * N + n]) : 0.0;
+        else s_colscale[threadIdx.x] = n < N ? ldexp(1.0, eb[(size_t)f * N + n]) : 0.0;
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -466,11 +596,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const bool ok = done && !s_abort;
     if (!ok && threadIdx.x == 0 && info) atomicOr(info + f, IA_INFO_TIMEOUT);
 
-    // epilogue: this thread's row, 16 real columns (8 complex) at a time
+    // epilogue: this thread's row, 16 real columns at a time
     const int row = m0 + warp * 32 + lane;
-    const double rs = row < M ? ldexp(alpha, ea[(size_t)f * M + row] - 10 - 6 * (S - 1)) : 0.0;
-    constexpr double TOP = (double)(1ll << (6 * (S - 1)));
-    double2 *Cf = C + f * sC;
+    double rs = 0.0;
+    if (row < M) {
+        const int er = ea[(size_t)f * M + row];
+        // FP64 path: 2^(er - 32) here, 2^(ec - 32) per column (10 + 54 = 64)
+        if constexpr (S == TC_SLICES_FP64) rs = alpha * fp64_scale(er);
+        else rs = ldexp(alpha, er - 10 - 6 * (S - 1));
+    }
+    auto *Cf = C + f * sC;
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
 #pragma unroll 1
     for (int ch = 0; ch < TC_BN / 16; ++ch) {
@@ -479,28 +614,46 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         for (int L = 0; L < S; ++L) tc::tmem_ld16(lane_base + (uint32_t)(L * TC_BN + ch * 16), v[L]);
         tc::tmem_wait_ld();
         if (!ok || row >= M) continue;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int n = c0 / 2 + ch * 8 + q;
-            if (n >= N) break;
-            double part[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int j = 2 * q + h;
+        // sum_L 64^(S-1-L) lev_L of real column j, rounded once
+        auto combine = [&](int j) -> double {
+            if constexpr (S <= 8) {
+                constexpr double TOP = (double)(1ll << (6 * (S - 1)));
                 long long acc = 0;
 #pragma unroll
                 for (int L = 1; L < S; ++L) acc = acc * 64 + (long long)__float2int_rn(__uint_as_float(v[L][j]));
-                part[h] = fma((double)__float2int_rn(__uint_as_float(v[0][j])), TOP, (double)acc);
+                return fma((double)__float2int_rn(__uint_as_float(v[0][j])), TOP, (double)acc);
+            } else {
+                // two groups of five levels, each an integer below 2^50
+                constexpr int H = 5;
+                long long hi = 0, lo = 0;
+#pragma unroll
+                for (int L = 0; L < S - H; ++L) hi = hi * 64 + (long long)__float2int_rn(__uint_as_float(v[L][j]));
+#pragma unroll
+                for (int L = S - H; L < S; ++L) lo = lo * 64 + (long long)__float2int_rn(__uint_as_float(v[L][j]));
+                return fma((double)hi, (double)(1ll << (6 * H)), (double)lo);
             }
-            const double sc = rs * s_colscale[ch * 8 + q];
-            double2 out = make_double2(part[0] * sc, part[1] * sc);
-            double2 *p = Cf + row + (size_t)n * ldc;
-            if (beta != 0.0) {
-                const double2 old = *p;
-                out.x = fma(beta, old.x, out.x);
-                out.y = fma(beta, old.y, out.y);
+        };
+#pragma unroll
+        for (int q = 0; q < 16 / CPC; ++q) {
+            const int n = c0 / CPC + ch * (16 / CPC) + q;
+            if (n >= N) break;
+            const double cs = s_colscale[ch * (16 / CPC) + q], sc = rs * cs;
+            // one factor at a time on the FP64 path: rs cs may leave the range where the result does not
+            auto scaled = [&](double v) { return S == TC_SLICES_FP64 ? (v * rs) * cs : v * sc; };
+            auto *p = Cf + row + (size_t)n * ldc;
+            if constexpr (REAL) {
+                double out = scaled(combine(q));
+                if (beta != 0.0) out = fma(beta, *p, out);
+                *p = out;
+            } else {
+                double2 out = make_double2(scaled(combine(2 * q)), scaled(combine(2 * q + 1)));
+                if (beta != 0.0) {
+                    const double2 old = *p;
+                    out.x = fma(beta, old.x, out.x);
+                    out.y = fma(beta, old.y, out.y);
+                }
+                *p = out;
             }
-            *p = out;
         }
     }
     tc::tc_fence_before();
@@ -548,15 +701,15 @@ int make_tmap(CUtensorMap *tm, const __nv_bfloat16 *planes, int Kp, int rows, in
     return r == CUDA_SUCCESS ? IA_OK : IA_ERR_CUDA;
 }
 
-template <int S>
+template <int S, bool REAL, class TC>
 int gemm_launch(ia_context *ctx, const CUtensorMap &ta, const CUtensorMap &tb, const TcPlanes &A, const TcPlanes &B,
-                int M, int N, double alpha, double beta, double2 *C, int ldc, long long sC, int batch, int *info)
+                int M, int N, double alpha, double beta, TC *C, int ldc, long long sC, int batch, int *info)
 {
     const size_t smem = tc_smem_bytes(S);
-    IA_CUDA_TRY(cudaFuncSetAttribute(tc_gemm_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((2 * N + TC_BN - 1) / TC_BN, (M + TC_BM - 1) / TC_BM, batch);
-    tc_gemm_kernel<S><<<grid, TC_THREADS, smem, ctx->stream>>>(ta, tb, M, N, A.Kp, A.e, B.e, alpha, beta, C, ldc, sC,
-                                                                info);
+    IA_CUDA_TRY(cudaFuncSetAttribute(tc_gemm_kernel<S, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    dim3 grid(((REAL ? 1 : 2) * N + tc_bn(S) - 1) / tc_bn(S), (M + TC_BM - 1) / TC_BM, batch);
+    tc_gemm_kernel<S, REAL><<<grid, TC_THREADS, smem, ctx->stream>>>(ta, tb, M, N, A.Kp, A.e, B.e, alpha, beta, C,
+                                                                      ldc, sC, info);
     IA_LAUNCH_CHECK(ctx);
     return IA_OK;
 }
@@ -575,10 +728,14 @@ int slice_launch(ia_context *ctx, const SliceOp<Src> &a, const SliceOp<Src> *b, 
         IA_LAUNCH_CHECK(ctx);
         return IA_OK;
     }
-    dim3 grid((rmax + SL_ROWS - 1) / SL_ROWS, batch, b ? 2 : 1);
-    tc_slice_kernel<Src, S><<<grid, 256, 0, ctx->stream>>>(a, b ? *b : a, K, Kp);
-    IA_LAUNCH_CHECK(ctx);
-    return IA_OK;
+    if constexpr (S == TC_SLICES_FP64) {
+        return IA_ERR_TOO_LARGE;   // not reached: K <= 819 fits the strip
+    } else {
+        dim3 grid((rmax + SL_ROWS - 1) / SL_ROWS, batch, b ? 2 : 1);
+        tc_slice_kernel<Src, S><<<grid, 256, 0, ctx->stream>>>(a, b ? *b : a, K, Kp);
+        IA_LAUNCH_CHECK(ctx);
+        return IA_OK;
+    }
 }
 
 // the operand descriptor and plane allocation of one operand
@@ -586,7 +743,8 @@ template <class Src>
 int slice_prepare(bool role_b, Op op, const Src *X, int ld, long long sX, int R, int K, int S, int batch,
                   TcPlanes &out, WsCursor &cur, SliceOp<Src> &d)
 {
-    if (R < 1 || K < 1 || batch < 1 || S < TC_SLICES_MIN || S > TC_SLICES_MAX) return IA_ERR_ARG;
+    if (R < 1 || K < 1 || batch < 1 || ((S < TC_SLICES_MIN || S > TC_SLICES_MAX) && S != TC_SLICES_FP64))
+        return IA_ERR_ARG;
     const int Kp = (2 * K + 7) & ~7;
     if ((long long)S * 1024 * Kp > (1ll << 24)) return IA_ERR_TOO_LARGE;   // level sums would leave FP32's exact range
     const int rows = role_b ? 2 * R : R;
@@ -609,6 +767,10 @@ int slice_dispatch(ia_context *ctx, int S, const SliceOp<Src> &a, const SliceOp<
     switch (S) {
     case 6: return slice_launch<Src, 6>(ctx, a, b, K, Kp, batch);
     case 7: return slice_launch<Src, 7>(ctx, a, b, K, Kp, batch);
+    case TC_SLICES_FP64:
+        if constexpr (std::is_same<Src, double2>::value)
+            return slice_launch<Src, TC_SLICES_FP64>(ctx, a, b, K, Kp, batch);
+        return IA_ERR_ARG;
     default: return slice_launch<Src, 8>(ctx, a, b, K, Kp, batch);
     }
 }
@@ -660,14 +822,59 @@ int tc_gemm(ia_context *ctx, const TcPlanes &A, const TcPlanes &B, int M, int N,
     if (A.S != B.S || A.Kp != B.Kp || A.R != M || B.R != N || A.rows != M || B.rows != 2 * N) return IA_ERR_ARG;
     CUtensorMap ta, tb;
     int st = make_tmap(&ta, A.p, A.Kp, A.rows, A.S, batch, TC_BM);
-    if (!st) st = make_tmap(&tb, B.p, B.Kp, B.rows, B.S, batch, TC_BN);
+    if (!st) st = make_tmap(&tb, B.p, B.Kp, B.rows, B.S, batch, tc_bn(A.S));
     if (st) return st;
     switch (A.S) {
-    case 6: return gemm_launch<6>(ctx, ta, tb, A, B, M, N, alpha, beta, C, ldc, sC, batch, info);
-    case 7: return gemm_launch<7>(ctx, ta, tb, A, B, M, N, alpha, beta, C, ldc, sC, batch, info);
-    case 8: return gemm_launch<8>(ctx, ta, tb, A, B, M, N, alpha, beta, C, ldc, sC, batch, info);
+    case 6: return gemm_launch<6, false>(ctx, ta, tb, A, B, M, N, alpha, beta, C, ldc, sC, batch, info);
+    case 7: return gemm_launch<7, false>(ctx, ta, tb, A, B, M, N, alpha, beta, C, ldc, sC, batch, info);
+    case 8: return gemm_launch<8, false>(ctx, ta, tb, A, B, M, N, alpha, beta, C, ldc, sC, batch, info);
+    case TC_SLICES_FP64:
+        return gemm_launch<TC_SLICES_FP64, false>(ctx, ta, tb, A, B, M, N, alpha, beta, C, ldc, sC, batch, info);
     default: return IA_ERR_ARG;
     }
+}
+
+// real operands: Kp K-values per row, one row per output row (column) in both
+// roles
+size_t tc_planes_real_bytes(int R, int K, int batch)
+{
+    const size_t Kp = (size_t)((K + 7) & ~7);
+    return ws_round(2 * (size_t)batch * TC_SLICES_FP64 * R * Kp) + ws_round(4 * (size_t)batch * R);
+}
+
+int tc_slice_real(ia_context *ctx, bool role_b, Op op, const double *X, int ld, long long sX, int R, int K, int batch,
+                  TcPlanes &out, WsCursor &cur)
+{
+    if (R < 1 || K < 1 || batch < 1) return IA_ERR_ARG;
+    const int Kp = (K + 7) & ~7;
+    if (!tc_real_ok(K)) return IA_ERR_TOO_LARGE;
+    out.R = out.rows = R;
+    out.Kp = Kp;
+    out.S = TC_SLICES_FP64;
+    out.p = cur.take<__nv_bfloat16>((size_t)batch * TC_SLICES_FP64 * R * Kp);
+    out.e = cur.take<int>((size_t)batch * R);
+    if (cur.off > cur.cap) return IA_ERR_ALLOC;
+    const size_t smem = sizeof(double) * SL1_RB * (size_t)slr_stride(Kp);
+    if (smem > 48 * 1024)
+        IA_CUDA_TRY(cudaFuncSetAttribute(tc_slice_real_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // view V(r, k): the A role reads rows of op(A), the B role columns of op(B)
+    const bool rcontig = role_b ? op != OP_N : op == OP_N;
+    tc_slice_real_kernel<<<dim3((R + SL1_RB - 1) / SL1_RB, batch), SL1_THREADS, smem, ctx->stream>>>(
+        X, ld, sX, R, K, Kp, rcontig ? 1 : 0, out.p, out.e);
+    IA_LAUNCH_CHECK(ctx);
+    return IA_OK;
+}
+
+int tc_gemm_real(ia_context *ctx, const TcPlanes &A, const TcPlanes &B, int M, int N, double alpha, double beta,
+                 double *C, int ldc, long long sC, int batch, int *info)
+{
+    if (M <= 0 || N <= 0 || batch <= 0) return IA_OK;
+    if (A.S != TC_SLICES_FP64 || B.S != A.S || A.Kp != B.Kp || A.rows != M || B.rows != N) return IA_ERR_ARG;
+    CUtensorMap ta, tb;
+    int st = make_tmap(&ta, A.p, A.Kp, A.rows, A.S, batch, TC_BM);
+    if (!st) st = make_tmap(&tb, B.p, B.Kp, B.rows, B.S, batch, tc_bn(A.S));
+    if (st) return st;
+    return gemm_launch<TC_SLICES_FP64, true>(ctx, ta, tb, A, B, M, N, alpha, beta, C, ldc, sC, batch, info);
 }
 
 IA_BOUNDS_READER(bounds_read_tc)
