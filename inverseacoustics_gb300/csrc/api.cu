@@ -675,10 +675,18 @@ int ia_ibem_assemble_batch(ia_context *ctx, const ia_mesh *mesh, int l, const do
                      (double2 *)d_Ahs_t, (double2 *)d_Bhs_t, mixed, false, G);
 }
 
-// H^T (m x l per frequency) into Ht, given workspace for A^T, B^T, pivots.
+// slice planes of the FP64 transfer's solver and products
+static size_t transfer_fp64_ws_bytes(int m, int l, int F)
+{
+    return std::max(zlu_ws_bytes(m, l, F), zgemm_tc_ws_bytes(m, l, m, F));
+}
+
+// H^T (m x l per frequency) into Ht, given workspace for A^T, B^T, pivots and
+// scratch for transfer_fp64_ws_bytes.
 static int ibem_transfer_t(ia_context *ctx, const ia_mesh *mesh, int l, const double *d_mics, int F,
                            const double *d_k, const ia_config *cfg, double2 *At, double2 *Bt, int *ipiv,
-                           double2 *Ahs_t, double2 *Ht, int *d_info, cudaEvent_t ev_rows = nullptr)
+                           double2 *Ahs_t, double2 *Ht, int *d_info, const WsCursor &scratch,
+                           cudaEvent_t ev_rows = nullptr)
 {
     const int m = mesh->m;
     int st;
@@ -691,13 +699,12 @@ static int ibem_transfer_t(ia_context *ctx, const ia_mesh *mesh, int l, const do
     NvtxRange r("ia.transfer");
     const long long sMM = (long long)m * m, sML = (long long)m * l;
     // LU of M = A^T; solve M Y = A_hs^T  ->  Y = W^T, W = A_hs A^-1
-    st = zgetrf_batched(ctx, m, At, m, sMM, ipiv, d_info, F);
+    st = zgetrf_ws(ctx, m, At, m, sMM, ipiv, d_info, F, scratch);
     if (st) return st;
-    st = zgetrs_batched(ctx, m, l, At, m, sMM, ipiv, Ahs_t, m, sML, F);
+    st = zgetrs_ws(ctx, m, l, At, m, sMM, ipiv, Ahs_t, m, sML, F, d_info, scratch);
     if (st) return st;
     // H^T = B^T Y - B_hs^T  (in place over B_hs^T)
-    return zgemm_batched(ctx, OP_N, OP_N, m, l, m, make_double2(1.0, 0.0), Bt, m, sMM, Ahs_t, m, sML,
-                         make_double2(-1.0, 0.0), Ht, m, sML, F);
+    return zgemm_tc(ctx, OP_N, OP_N, m, l, m, 1.0, Bt, m, sMM, Ahs_t, m, sML, -1.0, Ht, m, sML, F, d_info, scratch);
 }
 
 // the FP64-level products of the mixed transfer run on the tensor cores
@@ -814,7 +821,7 @@ int ia_ibem_transfer_batch(ia_context *ctx, const ia_mesh *mesh, int l, const do
     const int m = mesh->m;
     const bool mixed = cfg->precision == IA_PREC_MIXED;
     size_t need = ws_round(sizeof(double2) * (size_t)m * m * F) * 2 + ws_round(sizeof(int) * (size_t)m * F) +
-                  ws_round(sizeof(double2) * (size_t)m * l * F) * 2 + (mixed ? transfer_mixed_ws_bytes(mesh, l, F, cfg) : 0);
+                  ws_round(sizeof(double2) * (size_t)m * l * F) * 2 + (mixed ? transfer_mixed_ws_bytes(mesh, l, F, cfg) : transfer_fp64_ws_bytes(m, l, F));
     int st = ws_reserve(ctx, need);
     if (!st) st = clear_info(ctx, d_info, F);
     if (st) return st;
@@ -825,7 +832,7 @@ int ia_ibem_transfer_batch(ia_context *ctx, const ia_mesh *mesh, int l, const do
     double2 *Ahs = cur.take<double2>((size_t)m * l * F);
     double2 *Ht = cur.take<double2>((size_t)m * l * F);
     if (mixed) st = ibem_transfer_t_mixed(ctx, mesh, l, d_mics, F, d_k, cfg, At, Bt, ipiv, Ahs, Ht, d_info, cur);
-    else st = ibem_transfer_t(ctx, mesh, l, d_mics, F, d_k, cfg, At, Bt, ipiv, Ahs, Ht, d_info);
+    else st = ibem_transfer_t(ctx, mesh, l, d_mics, F, d_k, cfg, At, Bt, ipiv, Ahs, Ht, d_info, cur);
     if (st) return st;
     return ztranspose_batched(ctx, m, l, Ht, m, (long long)m * l, (double2 *)d_H, l, (long long)m * l, false, F);
 }
@@ -1062,8 +1069,10 @@ static size_t ibem_solve_ws_bytes(const ia_mesh *mesh, int l, int F, int nrhs, c
     const bool mixed = cfg->precision == IA_PREC_MIXED;
     const int m = mesh->m;
     return ws_round(sizeof(double2) * (size_t)m * m * F) * 2 + ws_round(sizeof(int) * (size_t)m * F) +
-           ws_round(sizeof(double2) * (size_t)m * l * F) * 2 + solve_ws_bytes(l, m, F, nrhs, cfg) +
-           (mixed ? transfer_mixed_ws_bytes(mesh, l, F, cfg, with_table) : 0);
+           ws_round(sizeof(double2) * (size_t)m * l * F) * 2 +
+           (mixed ? solve_ws_bytes(l, m, F, nrhs, cfg) + transfer_mixed_ws_bytes(mesh, l, F, cfg, with_table)
+                  // the transfer's scratch is free again when the solve starts
+                  : std::max(solve_ws_bytes(l, m, F, nrhs, cfg), transfer_fp64_ws_bytes(m, l, F)));
 }
 
 // the whole IBEM pipeline for F bins on ctx->stream; ev_rows (if given) is
@@ -1083,7 +1092,7 @@ static int ibem_solve_part(ia_context *ctx, const ia_mesh *mesh, int l, const do
     if (cfg->precision == IA_PREC_MIXED)
         st = ibem_transfer_t_mixed(ctx, mesh, l, d_mics, F, d_k, cfg, At, Bt, ipiv, Ahs, Ht, info, cur, ev_rows,
                                    shared_geom);
-    else st = ibem_transfer_t(ctx, mesh, l, d_mics, F, d_k, cfg, At, Bt, ipiv, Ahs, Ht, info, ev_rows);
+    else st = ibem_transfer_t(ctx, mesh, l, d_mics, F, d_k, cfg, At, Bt, ipiv, Ahs, Ht, info, cur, ev_rows);
     if (st) return st;
     return solve_core(ctx, l, m, F, Ht, true, nrhs, p, cfg, x, lambda, s, info, cur);
 }
@@ -1382,7 +1391,8 @@ int ia_esm(int m, int l, const double *r_ms, const double *r_lh, ia_complex **m_
     CompatScratch sc{ctx};
     size_t need = ws_round(24 * (size_t)(m + l)) + ws_round(16 * (size_t)m * m) + ws_round(16 * (size_t)m * (m + l)) +
                   ws_round(16 * (size_t)m * (m + l)) + ws_round(4 * (size_t)m) + ws_round(4) + 4096;
-    IA_TRY(sc.alloc(need));
+    const size_t lu = zlu_ws_bytes(m, m + l, 1);
+    IA_TRY(sc.alloc(need + lu));
     double *dr = sc.take<double>(3 * (size_t)m);
     double *dl = sc.take<double>(3 * (size_t)l);
     double2 *DT = sc.take<double2>((size_t)m * m);
@@ -1394,8 +1404,9 @@ int ia_esm(int m, int l, const double *r_ms, const double *r_lh, ia_complex **m_
     IA_CTRY(cudaMemcpyAsync(dl, r_lh, 24 * (size_t)l, cudaMemcpyHostToDevice, ctx->stream));
     IA_CTRY(cudaMemsetAsync(info, 0, 4, ctx->stream));
     IA_TRY(esm_system(ctx, m, l, dr, dl, r_i, k, cfg->c, cfg->rho, DT, RHS));
-    IA_TRY(zgetrf_batched(ctx, m, DT, m, 0, ipiv, info, 1));
-    IA_TRY(zgetrs_batched(ctx, m, m + l, DT, m, 0, ipiv, RHS, m, 0, 1));
+    const WsCursor planes{sc.take<char>(lu), 0, lu};
+    IA_TRY(zgetrf_ws(ctx, m, DT, m, 0, ipiv, info, 1, planes));
+    IA_TRY(zgetrs_ws(ctx, m, m + l, DT, m, 0, ipiv, RHS, m, 0, 1, info, planes));
     // Me = X[:, :m]^T, He = X[:, m:]^T
     IA_TRY(ztranspose_batched(ctx, m, m, RHS, m, 0, OUT, m, 0, false, 1));
     IA_TRY(ztranspose_batched(ctx, m, l, RHS + (size_t)m * m, m, 0, OUT + (size_t)m * m, l, 0, false, 1));

@@ -24,6 +24,7 @@
 // the one-sided Jacobi SVD of G Z (svd.cu).  Each complex column's phase is
 // fixed so that its first component within 1e-6 of the largest magnitude is
 // real and positive.
+#include <algorithm>
 #include "ia_common.cuh"
 #include "ia_internal.h"
 
@@ -350,6 +351,9 @@ size_t bem_modes_ws_bytes(const ia_mesh *mesh, int l, int n_ch, int F, int nm, c
         }
     } else b += ws_round(8 * M * M * FF) + ws_round(8 * nm * FF) + radiation_modes_ws_bytes(mesh->m, F, nm, cfg, true);
     if (cfg->precision == IA_PREC_MIXED) b += ws_round(ibem_geom_bytes(mesh, (int)(MT + L)));   // assembly geometry
+    if (!bem_mixed_solve(cfg, n_ch))   // slice planes of the FP64 solver and products
+        b += std::max({zlu_ws_bytes(mesh->m, mesh->m, F), zgemm_tc_ws_bytes(l, mesh->m, mesh->m, F),
+                       zgemm_tc_ws_bytes(mesh->m > l ? mesh->m : l, nm, mesh->m, F)});
     if (bem_mixed_solve(cfg, n_ch)) {
         b += 2 * ws_round(8 * M * M * FF) + ws_round(16 * M * M * FF);
         if (tc_products_ok(bem_slices(cfg), mesh->m))
@@ -453,7 +457,6 @@ int bem_modes_batched(ia_context *ctx, const ia_mesh *mesh, int l, const double 
     int *ipiv = cur.take<int>((size_t)m * F);
     double *gval = cur.take<double>((size_t)mesh->gnnz);
     double2 *Uc = cplx ? static_cast<double2 *>(Ur) : cur.take<double2>((size_t)m * nm * F);
-    const double2 one = make_double2(1.0, 0.0), mone = make_double2(-1.0, 0.0), zero = make_double2(0.0, 0.0);
     const bool mixed_z = bem_mixed_solve(cfg, n_ch);
     double2 *Z = At;
     if (mixed_z) {
@@ -473,8 +476,8 @@ int bem_modes_batched(ia_context *ctx, const ia_mesh *mesh, int l, const double 
         if ((st = ztranspose_batched(ctx, m, l, Bhs_t, m, ml, H, l, ml, false, F))) return st;
         // Z = A \ B (B's storage, leading dimension mt)
         if (n_ch == 0) {
-            if ((st = zgetrf_batched(ctx, m, A, mt, tm, ipiv, info, F))) return st;
-            if ((st = zgetrs_batched(ctx, m, m, A, mt, tm, ipiv, B, mt, tm, F))) return st;
+            if ((st = zgetrf_ws(ctx, m, A, mt, tm, ipiv, info, F, cur))) return st;
+            if ((st = zgetrs_ws(ctx, m, m, A, mt, tm, ipiv, B, mt, tm, F, info, cur))) return st;
         } else {
             if ((st = zgeqrs_batched(ctx, mt, m, A, mt, tm, m, B, mt, tm, F))) return st;
             if ((st = zbacksolve_upper_batched(ctx, m, m, A, mt, tm, B, mt, tm, F))) return st;
@@ -482,7 +485,7 @@ int bem_modes_batched(ia_context *ctx, const ia_mesh *mesh, int l, const double 
         // compact Z (ld mt -> m) into At's storage
         if ((st = zcopy2d_batched(ctx, m, m, B, mt, tm, Z, m, mm, false, F))) return st;
         // H = A_hs Z - B_hs
-        if ((st = zgemm_batched(ctx, OP_N, OP_N, l, m, m, one, Ahs, l, ml, Z, m, mm, mone, H, l, ml, F))) return st;
+        if ((st = zgemm_tc(ctx, OP_N, OP_N, l, m, m, 1.0, Ahs, l, ml, Z, m, mm, -1.0, H, l, ml, F, info, cur))) return st;
     }
     mass_matrix_kernel<<<(m + 127) / 128, 128, 0, ctx->stream>>>(m, mesh->d_gptr, mesh->d_gidx, mesh->d_adj_ptr,
                                                                   mesh->d_adj, mesh->d_evert, mesh->d_egeo,
@@ -540,9 +543,10 @@ int bem_modes_batched(ia_context *ctx, const ia_mesh *mesh, int l, const double 
         if (Pr) st = dfgemm_batched(ctx, OP_N, OP_N, m, nm, m, 1.0, Z, m, mm, Uc, m, mn, 0.0, Pr, m, mn, F);
         return st;
     }
-    if ((st = zgemm_batched(ctx, OP_N, OP_N, l, nm, m, one, H, l, ml, Uc, m, mn, zero, Hr, l, (long long)l * nm, F)))
+    if ((st = zgemm_tc(ctx, OP_N, OP_N, l, nm, m, 1.0, H, l, ml, Uc, m, mn, 0.0, Hr, l, (long long)l * nm, F, info,
+                       cur)))
         return st;
-    if (Pr) st = zgemm_batched(ctx, OP_N, OP_N, m, nm, m, one, Z, m, mm, Uc, m, mn, zero, Pr, m, mn, F);
+    if (Pr) st = zgemm_tc(ctx, OP_N, OP_N, m, nm, m, 1.0, Z, m, mm, Uc, m, mn, 0.0, Pr, m, mn, F, info, cur);
     return st;
 }
 

@@ -5,6 +5,7 @@
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
+#include <algorithm>
 #include "ia_common.cuh"
 #include "ia_internal.h"
 
@@ -40,9 +41,13 @@ extern "C" int ia_ibem(int m, int l, int n, const double *r_ms, const int *e_n, 
         if (st) break;
         size_t need = ws_round(24 * (size_t)l) + ws_round(24 * (size_t)(n_ch ? n_ch : 1)) + ws_round(8) + 4 * ws_round(16 * (size_t)mt * m) +
                       3 * ws_round(16 * (size_t)l * m) + ws_round(4 * (size_t)m) + ws_round(4) + 8192;
+        // slice planes of the solver and of H's product
+        const size_t pl = std::max(zlu_ws_bytes(m, m, 1), zgemm_tc_ws_bytes(l, m, m, 1));
+        need += pl;
         cudaError_t e = cudaMallocAsync(&scratch, need, stream);
         if (e != cudaSuccess) { st = cuda_status(e); break; }
         WsCursor cur{(char *)scratch, 0, need};
+        const WsCursor planes{cur.take<char>(pl), 0, pl};
         double *dl = cur.take<double>(3 * (size_t)l);
         double *dcp = cur.take<double>(3 * (size_t)(n_ch ? n_ch : 1));
         double *dk = cur.take<double>(1);
@@ -69,17 +74,15 @@ extern "C" int ia_ibem(int m, int l, int n, const double *r_ms, const int *e_n, 
         if ((st = ztranspose_batched(ctx, m, l, Bht, m, 0, H, l, 0, false, 1))) break;
         if ((st = ztranspose_batched(ctx, m, l, Aht, m, 0, Bht, l, 0, false, 1))) break;   // Bht := A_hs
         if (n_ch == 0) {
-            if ((st = zgetrf_batched(ctx, m, A, mt, 0, ipiv, info, 1))) break;
-            if ((st = zgetrs_batched(ctx, m, m, A, mt, 0, ipiv, B, mt, 0, 1))) break;
+            if ((st = zgetrf_ws(ctx, m, A, mt, 0, ipiv, info, 1, planes))) break;
+            if ((st = zgetrs_ws(ctx, m, m, A, mt, 0, ipiv, B, mt, 0, 1, info, planes))) break;
         } else {
             // least squares: Q^H [A | B], then R Z = (Q^H B)(1:m, :)
             if ((st = zgeqrs_batched(ctx, mt, m, A, mt, 0, m, B, mt, 0, 1))) break;
             if ((st = zbacksolve_upper_batched(ctx, m, m, A, mt, 0, B, mt, 0, 1))) break;
         }
         // H = A_hs Z - B_hs
-        if ((st = zgemm_batched(ctx, OP_N, OP_N, l, m, m, make_double2(1.0, 0.0), Bht, l, 0, B, mt, 0,
-                                make_double2(-1.0, 0.0), H, l, 0, 1)))
-            break;
+        if ((st = zgemm_tc(ctx, OP_N, OP_N, l, m, m, 1.0, Bht, l, 0, B, mt, 0, -1.0, H, l, 0, 1, info, planes))) break;
         // compact Z (ld mt -> m) into A's storage
         if ((st = zcopy2d_batched(ctx, m, m, B, mt, 0, A, m, 0, false, 1))) break;
         if ((e = cudaMemcpyAsync(&hinfo, info, 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) { st = cuda_status(e); break; }

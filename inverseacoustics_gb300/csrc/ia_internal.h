@@ -156,6 +156,20 @@ inline int zcopy2d_batched(ia_context *ctx, int rows, int cols, const double2 *i
 {
     return copy2d_batched<double2, double2>(ctx, rows, cols, in, ldi, si, out, ldo, so, conj, batch);
 }
+// FP64 path on the tensor cores (zlu.cu).  Products: alpha op(A) op(B) + beta C
+// on 10 BF16 slices per operand, planes in scratch (at least
+// zgemm_tc_ws_bytes; smaller products may share it).  LU and solves as
+// zgetrf_batched / zgetrs_batched, scratch of zlu_ws_bytes.
+size_t zgemm_tc_ws_bytes(int M, int N, int K, int batch);
+int zgemm_tc(ia_context *ctx, Op opa, Op opb, int M, int N, int K, double alpha, const double2 *A, int lda,
+             long long sA, const double2 *B, int ldb, long long sB, double beta, double2 *C, int ldc, long long sC,
+             int batch, int *info, WsCursor scratch);
+size_t zlu_ws_bytes(int n, int nrhs, int batch);
+int zgetrf_ws(ia_context *ctx, int n, double2 *A, int lda, long long sA, int *ipiv, int *info, int batch,
+              WsCursor scratch);
+int zgetrs_ws(ia_context *ctx, int n, int nrhs, const double2 *LU, int lda, long long sA, const int *ipiv, double2 *B,
+              int ldb, long long sB, int batch, int *info, WsCursor scratch);
+
 // Householder QR of A (rows x cols, rows >= cols) applied to [A | B] in place:
 // on exit the upper triangle of A is R and B holds Q^H B.
 int zgeqrs_batched(ia_context *ctx, int rows, int cols, double2 *A, int lda, long long sA, int nrhs, double2 *B,
