@@ -30,13 +30,13 @@ namespace cg = cooperative_groups;
 // panels and diagonal blocks at the same tensor-core time (a rank-64 update's
 // tile costs ~10 us of MMAs and ~6 us of set-up and epilogue).
 constexpr int ZLU_NB = 64;
-// A few small matrices (more than one panel): panels of 32 columns and rank-32
-// FP64 GEMMs (staged panels, dense.cu).  The panels' latency sets the time and
-// the FP64 tiles find idle SMs, so the two forms are level (transfer of 8 bins:
-// n = 92 1.07 ms against 1.08 with rank-64 slice products, n = 162 1 bin 1.42
-// and 1.41 ms); with more bins the slice products win (n = 162, 64 bins: 8.8
-// against 9.3 ms), and a single panel (n <= 64) is better whole.
-constexpr int ZLU_SMALL_N = 192, ZLU_SMALL_BATCH = 8;
+// Small matrices of more than one panel: panels of 32 columns and rank-32 FP64
+// GEMMs (staged panels, dense.cu).  For a few bins the panels' latency sets the
+// time and the two forms are level (transfer of 8 bins: n = 92 1.07 ms against
+// 1.08 with rank-64 slice products; n = 162, 1 bin 1.42 and 1.41 ms); at 64 bins
+// the slices would gain 6 % (n = 162), but the choice must not depend on the
+// batch: a bin's results are bitwise those it has alone or in another split.
+constexpr int ZLU_SMALL_N = 192;
 constexpr int ZP_THREADS = 256;
 constexpr int ZP_MAX_CS = 8;
 constexpr size_t ZP_SMEM_MAX = 200 * 1024;
@@ -462,7 +462,7 @@ int zgetrf_ws(ia_context *ctx, int n, double2 *A, int lda, long long sA, int *ip
     if (!zlu_ok(ctx, n)) return zgetrf_batched(ctx, n, A, lda, sA, ipiv, info, batch);
     IA_CUDA_TRY(cudaFuncSetAttribute(zlu_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZP_SMEM_MAX));
     int st;
-    const bool small = n > ZLU_NB && n <= ZLU_SMALL_N && batch <= ZLU_SMALL_BATCH;
+    const bool small = n > ZLU_NB && n <= ZLU_SMALL_N;
     const int NB = small ? ZLU_NB / 2 : ZLU_NB;
     for (int k0 = 0; k0 < n; k0 += NB) {
         const int nb = n - k0 < NB ? n - k0 : NB, kend = k0 + nb, rest = n - kend;
