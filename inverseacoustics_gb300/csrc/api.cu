@@ -699,8 +699,14 @@ static int ibem_transfer_t(ia_context *ctx, const ia_mesh *mesh, int l, const do
     NvtxRange r("ia.transfer");
     const long long sMM = (long long)m * m, sML = (long long)m * l;
     // LU of M = A^T; solve M Y = A_hs^T  ->  Y = W^T, W = A_hs A^-1
-    st = zgetrf_ws(ctx, m, At, m, sMM, ipiv, d_info, F, scratch);
+    st = zgetrf_ws(ctx, m, At, m, sMM, ipiv, d_info, F, scratch, ctx->plain_fp64 != 0);
     if (st) return st;
+    if (ctx->plain_fp64) {
+        st = zgetrs_batched(ctx, m, l, At, m, sMM, ipiv, Ahs_t, m, sML, F);
+        if (st) return st;
+        return zgemm_batched(ctx, OP_N, OP_N, m, l, m, make_double2(1.0, 0.0), Bt, m, sMM, Ahs_t, m, sML,
+                             make_double2(-1.0, 0.0), Ht, m, sML, F);
+    }
     st = zgetrs_ws(ctx, m, l, At, m, sMM, ipiv, Ahs_t, m, sML, F, d_info, scratch);
     if (st) return st;
     // H^T = B^T Y - B_hs^T  (in place over B_hs^T)
@@ -1025,6 +1031,7 @@ static int fp64_fallback(ia_context *ctx, const ia_config *cfg, int F, int *d_in
     }
     if (!st && !fp64.empty()) {
         const ia_config rc = fp64_config(cfg);
+        const PlainFp64 plain(ctx, true);
         st = redo_bins(ctx, fp64, d_info, ins, outs, redo, &rc);
     }
     if (!st) ctx->last_fallback = (int)(retry.size() + fp64.size());
@@ -1121,6 +1128,7 @@ int ia_ibem_solve_batch(ia_context *ctx, const ia_mesh *mesh, int l, const doubl
         parts = cfg->pipeline_parts;
         if (parts < 1 || parts > IA_SPLIT_PARTS || F % parts || (parts > 1 && (F / parts) % 4)) return IA_ERR_ARG;
     }
+    const PlainFp64 plain(ctx, cfg->precision != IA_PREC_MIXED);
     const int Fp = F / parts;
     const size_t need = ibem_solve_ws_bytes(mesh, l, Fp, nrhs, cfg, parts == 1);
     const size_t gshared = parts > 1 && cfg->precision == IA_PREC_MIXED ? ibem_geom_bytes(mesh, m + l) : 0;

@@ -508,6 +508,12 @@ __global__ void __launch_bounds__(128) trsm_block_kernel(int nbk, const T *Tm, i
         if (r < nbk) X[r + (size_t)col * ldx] = x[r];
 }
 
+// threads per CTA of the block solves: in FP64 a warp holds its SM's FP64 pipe
+// for the whole solve (~18 us), so the columns spread over as many SMs as
+// there are warps (74 -> 20 us at 642 columns); in FP32 four warps share a CTA
+template <class T>
+constexpr int trsm_threads() { return sizeof(T) == sizeof(double2) ? 32 : 128; }
+
 template <class T>
 int getrf_batched(ia_context *ctx, int n, T *A, int lda, long long sA, int *ipiv, int *info, int batch)
 {
@@ -535,8 +541,8 @@ int getrf_batched(ia_context *ctx, int n, T *A, int lda, long long sA, int *ipiv
         }
         int rest = n - kend;
         if (rest <= 0) break;
-        dim3 g((rest + 127) / 128, batch);
-        trsm_block_kernel<T, false><<<g, 128, 0, ctx->stream>>>(nb, A + k0 + (size_t)k0 * lda, lda, sA,
+        dim3 g((rest + trsm_threads<T>() - 1) / trsm_threads<T>(), batch);
+        trsm_block_kernel<T, false><<<g, trsm_threads<T>(), 0, ctx->stream>>>(nb, A + k0 + (size_t)k0 * lda, lda, sA,
                                                                  A + k0 + (size_t)kend * lda, lda, sA, rest);
         IA_LAUNCH_CHECK(ctx);
         int r = gemm_batched<T>(ctx, OP_N, OP_N, rest, rest, nb, mone, A + kend + (size_t)k0 * lda, lda, sA,
@@ -570,13 +576,13 @@ int backsolve_upper_batched(ia_context *ctx, int n, int nrhs, const T *LU, int l
                             long long sB, int batch)
 {
     const T one = ctraits<T>::make(1, 0), mone = ctraits<T>::make(-1, 0);
-    dim3 g((nrhs + 127) / 128, batch);
+    dim3 g((nrhs + trsm_threads<T>() - 1) / trsm_threads<T>(), batch);
     int nblk = (n + LU_NB - 1) / LU_NB;
     for (int bi = nblk - 1; bi >= 0; --bi) {
         int k0 = bi * LU_NB;
         int kend = k0 + LU_NB < n ? k0 + LU_NB : n;
         int nb = kend - k0;
-        trsm_block_kernel<T, true><<<g, 128, 0, ctx->stream>>>(nb, LU + k0 + (size_t)k0 * lda, lda, sA, B + k0, ldb,
+        trsm_block_kernel<T, true><<<g, trsm_threads<T>(), 0, ctx->stream>>>(nb, LU + k0 + (size_t)k0 * lda, lda, sA, B + k0, ldb,
                                                                 sB, nrhs);
         IA_LAUNCH_CHECK(ctx);
         if (k0 > 0) {
@@ -789,14 +795,14 @@ int getrs_batched(ia_context *ctx, int n, int nrhs, const T *LU, int lda, long l
         }
     }
     const T one = ctraits<T>::make(1, 0), mone = ctraits<T>::make(-1, 0);
-    dim3 g((nrhs + 127) / 128, batch);
-    apply_pivots_kernel<T><<<g, 128, 0, ctx->stream>>>(n, nrhs, ipiv, B, ldb, sB);
+    apply_pivots_kernel<T><<<dim3((nrhs + 127) / 128, batch), 128, 0, ctx->stream>>>(n, nrhs, ipiv, B, ldb, sB);
     IA_LAUNCH_CHECK(ctx);
+    dim3 g((nrhs + trsm_threads<T>() - 1) / trsm_threads<T>(), batch);
     // forward: L Y = B
     for (int k0 = 0; k0 < n; k0 += LU_NB) {
         int kend = k0 + LU_NB < n ? k0 + LU_NB : n;
         int nb = kend - k0;
-        trsm_block_kernel<T, false><<<g, 128, 0, ctx->stream>>>(nb, LU + k0 + (size_t)k0 * lda, lda, sA, B + k0, ldb,
+        trsm_block_kernel<T, false><<<g, trsm_threads<T>(), 0, ctx->stream>>>(nb, LU + k0 + (size_t)k0 * lda, lda, sA, B + k0, ldb,
                                                                  sB, nrhs);
         IA_LAUNCH_CHECK(ctx);
         if (kend < n) {

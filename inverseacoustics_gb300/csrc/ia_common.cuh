@@ -113,6 +113,23 @@ __device__ __forceinline__ double2 zdiv(double2 a, double2 b)
     return make_double2((a.x * b.x + a.y * b.y) * s, (a.y * b.x - a.x * b.y) * s);
 }
 
+// |b|^2 with the contraction spelled out: which of the two products is rounded
+// alone is otherwise the compiler's choice, kernel by kernel.  The QR and LU
+// kernels that reproduce another kernel's factors bit for bit need its choice.
+__device__ __forceinline__ double zabs2_x(double2 b) { return fma(b.x, b.x, b.y * b.y); }
+__device__ __forceinline__ double zabs2_y(double2 b) { return fma(b.y, b.y, b.x * b.x); }
+// 1 / b with that choice
+__device__ __forceinline__ double2 zrcp_x(double2 b)
+{
+    const double s = 1.0 / zabs2_x(b);
+    return make_double2(b.x * s, -b.y * s);
+}
+__device__ __forceinline__ double2 zrcp_y(double2 b)
+{
+    const double s = 1.0 / zabs2_y(b);
+    return make_double2(b.x * s, -b.y * s);
+}
+
 __device__ __forceinline__ double warp_sum(double v)
 {
 #pragma unroll

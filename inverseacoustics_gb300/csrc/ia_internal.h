@@ -23,6 +23,7 @@ struct ia_context {
     int last_fallback;     // bins the last batched solve recomputed in FP64 (mixed_fallback)
     int tail_part;         // the last part of a staggered pipeline is running (its chain ends the pass:
                            // latency-bound stages may take more SMs per bin)
+    int plain_fp64;        // the FP64 solve in progress keeps the plain operation order (PlainFp64)
     int *dcount;           // small device counters (the GPU-wide Jacobi's per-bin flags), lazily allocated
     size_t dcount_n;
     // streams and events of the staggered IBEM pipeline (one stream per part;
@@ -34,6 +35,25 @@ struct ia_context {
 
 namespace ia {
 int ensure_side_stream(ia_context *ctx);
+
+// Scope of an FP64 solve that keeps the plain operation order (FP64 GEMM
+// updates and products, Jacobi from the pivoted R): the IBEM inversion and the
+// FP64 solution of a mixed call's flagged bins.  In a bin whose GCV minimum
+// sits at the bottom of its grid (0.6 % of the sphere's bins at 30 dB:
+// lambda ~ 1e-10 s_1) the solution carries the operator's and the
+// decomposition's rounding times s_1 / lambda, so only the same operations
+// give the same digits there.
+struct PlainFp64 {
+    ia_context *ctx;
+    int prev;
+    PlainFp64(ia_context *c, bool on) : ctx(c), prev(c->plain_fp64)
+    {
+        if (on) c->plain_fp64 = 1;
+    }
+    ~PlainFp64() { ctx->plain_fp64 = prev; }
+    PlainFp64(const PlainFp64 &) = delete;
+    PlainFp64 &operator=(const PlainFp64 &) = delete;
+};
 }
 
 // threads per CTA of the IBEM assembly kernel; mesh colours are balanced to it
@@ -165,11 +185,18 @@ int zgemm_tc(ia_context *ctx, Op opa, Op opb, int M, int N, int K, double alpha,
              long long sA, const double2 *B, int ldb, long long sB, double beta, double2 *C, int ldc, long long sC,
              int batch, int *info, WsCursor scratch);
 size_t zlu_ws_bytes(int n, int nrhs, int batch);
+// plain: rank-32 FP64 updates at every n, bitwise zgetrf_batched's factors
 int zgetrf_ws(ia_context *ctx, int n, double2 *A, int lda, long long sA, int *ipiv, int *info, int batch,
-              WsCursor scratch);
+              WsCursor scratch, bool plain = false);
 int zgetrs_ws(ia_context *ctx, int n, int nrhs, const double2 *LU, int lda, long long sA, const int *ipiv, double2 *B,
               int ldb, long long sB, int batch, int *info, WsCursor scratch);
 
+// FP64 Householder QR over a cluster per matrix (zqr.cu), where zqr_ok: with
+// column pivoting (columns unmoved: R(i, k) at A(i, perm[k])), or LAPACK's
+// zgeqrf layout
+bool zqr_ok(int rows, int cols);
+int zqr_pivoted_batched(ia_context *ctx, int rows, int cols, double2 *A, int lda, long long sA, int *perm, int batch);
+int zqr_plain_batched(ia_context *ctx, int rows, int cols, double2 *A, int lda, long long sA, double2 *tau, int batch);
 // Householder QR of A (rows x cols, rows >= cols) applied to [A | B] in place:
 // on exit the upper triangle of A is R and B holds Q^H B.
 int zgeqrs_batched(ia_context *ctx, int rows, int cols, double2 *A, int lda, long long sA, int nrhs, double2 *B,

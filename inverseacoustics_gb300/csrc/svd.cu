@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(sizeof(T) <= 8 ? 1024 : 512)
 // The same iteration over a cluster of CS CTAs per bin (no accumulator).
 // FP32: for latency, in small batches and the last part of a staggered
 // pipeline, whose chain ends the pass.  FP64 (bound by the FP64 pipe of its
-// SM): whenever the batch leaves SMs idle, CS = 2 or 4 CTAs per bin.  CTA q owns the pair slots
+// SM): whenever the batch leaves SMs idle, 2 to 8 CTAs per bin.  CTA q owns the pair slots
 // [q P, (q + 1) P) of the circle ordering (P = N2 / 2 / JC_CS).  From one
 // round to the next the ordering moves every "upper" column (slot k holds
 // columns (r + k) and (r - k) mod (N2 - 1), column N2 - 1 fixed in slot 0)
@@ -373,14 +373,14 @@ __global__ void __launch_bounds__(sizeof(T) <= 8 ? 1024 : 512)
 // reductions, rotation and stopping rule; the sweep's rotation count and
 // largest coupling are combined over the cluster), so the factors are
 // bitwise the same.
-template <class T, int JC_CS, int KPL = 8>
+template <class T, int KPL = 8>
 __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
     jacobi_cluster_kernel(int M, int Mdot, int N, T *Yg, long long sY, int max_sweeps, typename ctraits<T>::R tol,
                           int *info)
 {
     typedef typename ctraits<T>::R R;
     cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
+    const int rank = (int)cluster.block_rank(), JC_CS = (int)cluster.num_blocks();
     const int f = blockIdx.x / JC_CS;
     const int N2 = N + (N & 1), NR = N2 - 1, P = N2 / 2 / JC_CS, RING = P + 1, k0 = rank * P;
     extern __shared__ __align__(16) unsigned char jc_raw[];
@@ -743,38 +743,52 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
         // needed: their alternative is a one-CTA kernel on global memory.
         const int np = (N + (N & 1)) / 2;
         int cs = 0, kpl = 8;
+        cudaLaunchConfig_t lc = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        lc.attrs = at;
+        lc.numAttrs = 1;
+        lc.stream = ctx->stream;
+        auto configure = [&](int c) {
+            const int P = np / c;
+            lc.gridDim = dim3((unsigned)(c * batch));
+            lc.blockDim = dim3((unsigned)(32 * ((P + 1) / 2)));
+            lc.dynamicSmemBytes = sizeof(T) * ((size_t)2 * (P + 1) * M + M);
+            at[0].val.clusterDim.x = c;
+        };
+        auto kern = jacobi_cluster_kernel<T, 8>;
         if (!V && M <= 128 && N <= 128) {
             if (sizeof(T) == 8) {
                 if (np % 4 == 0 && np / 4 >= 2 && (16 * batch <= ctx->sm_count || ctx->tail_part)) cs = 4;
             } else {
-                for (int c : {4, 2})
-                    if (!cs && np % c == 0 && np / c >= 2 && c * batch <= ctx->sm_count) cs = c;
+                // the largest cluster that divides the pairs and whose clusters
+                // all run at once (a cluster stays inside one GPC)
+                for (int c : {8, 6, 5, 4, 3, 2}) {
+                    if (np % c || np / c < 2 || c * batch > ctx->sm_count) continue;
+                    configure(c);
+                    if (lc.dynamicSmemBytes > 48 * 1024)
+                        IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)lc.dynamicSmemBytes));
+                    int fit = 0;
+                    IA_CUDA_TRY(cudaOccupancyMaxActiveClusters(&fit, kern, &lc));
+                    if (fit >= batch) {
+                        cs = c;
+                        break;
+                    }
+                }
             }
         } else if (!V && M <= 272 && N <= 272 && M > 128 && np % 8 == 0 && np / 8 >= 2) {
             cs = 8;
             kpl = M <= 192 ? 12 : 17;
         }
         if (cs) {
-            const int P = np / cs;
-            const size_t csm = sizeof(T) * ((size_t)2 * (P + 1) * M + M);
-            const int nwc = (P + 1) / 2;
-            cudaLaunchConfig_t lc = {};
-            lc.gridDim = dim3((unsigned)(cs * batch));
-            lc.blockDim = dim3((unsigned)(32 * nwc));
-            lc.dynamicSmemBytes = csm;
-            lc.stream = ctx->stream;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = cs;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            lc.attrs = at;
-            lc.numAttrs = 1;
-            auto kern = kpl == 17   ? jacobi_cluster_kernel<T, 8, 17>
-                        : kpl == 12 ? jacobi_cluster_kernel<T, 8, 12>
-                        : (cs == 4 ? jacobi_cluster_kernel<T, 4> : jacobi_cluster_kernel<T, 2>);
-            if (csm > 48 * 1024)
-                IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
+            configure(cs);
+            kern = kpl == 17 ? jacobi_cluster_kernel<T, 17> : kpl == 12 ? jacobi_cluster_kernel<T, 12> : kern;
+            if (lc.dynamicSmemBytes > 48 * 1024)
+                IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)lc.dynamicSmemBytes));
             IA_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, M, Mdot, N, Y, sY, max_sweeps, tol, info));
             IA_LAUNCH_CHECK(ctx);
             return IA_OK;

@@ -538,6 +538,8 @@ int zgeqrs_batched(ia_context *ctx, int rows, int cols, double2 *A, int lda, lon
 template <class T>
 int qr_batched(ia_context *ctx, int rows, int cols, T *A, int lda, long long sA, T *tau, int batch)
 {
+    if constexpr (std::is_same<T, double2>::value)
+        if (zqr_ok(rows, cols)) return zqr_plain_batched(ctx, rows, cols, A, lda, sA, tau, batch);
     return qr_launch<T>(ctx, rows, cols, A, lda, sA, tau, 0, nullptr, 0, 0, batch);
 }
 template int qr_batched<float2>(ia_context *, int, int, float2 *, int, long long, float2 *, int);
@@ -631,8 +633,9 @@ __global__ void eig_backproject_kernel(int m, int n, int N, const double2 *H, in
 
 // Raug ((N + nrhs) x N) of the pivoted-QR solve: R^H (R: upper triangle of
 // Y P = Q R) over the rows conj(v_r)^T, v_r = R P^T b_r, so that the
-// one-sided Jacobi's column rotations J carry J^H v_r along.
-__global__ void build_rh_aug_kernel(int N, int Mrows, int nrhs, const double2 *Y, const int *perm,
+// one-sided Jacobi's column rotations J carry J^H v_r along.  R's column k
+// stands in Y's column perm[k] (unmoved) or k.
+__global__ void build_rh_aug_kernel(int N, int Mrows, int nrhs, const double2 *Y, const int *perm, int unmoved,
                                     const double2 *B, double2 *Rg)
 {
     const int f = blockIdx.y;
@@ -647,7 +650,7 @@ __global__ void build_rh_aug_kernel(int N, int Mrows, int nrhs, const double2 *Y
         const int i = (int)(e % N), j = (int)(e / N);     // R^H(i, j) = conj(R(j, i)), R upper
         double2 v = make_double2(0.0, 0.0);
         if (j <= i) {
-            const double2 r = Y[j + (size_t)i * Mrows];
+            const double2 r = Y[j + (size_t)(unmoved ? perm[i] : i) * Mrows];
             v = make_double2(r.x, -r.y);
         }
         Rg[i + (size_t)j * ld] = v;
@@ -658,7 +661,7 @@ __global__ void build_rh_aug_kernel(int N, int Mrows, int nrhs, const double2 *Y
         const int i = (int)(e % N), r = (int)(e / N);
         const double2 *br = b + (size_t)r * N;
         double2 acc = make_double2(0.0, 0.0);
-        for (int j = i; j < N; ++j) zfma(acc, Y[i + (size_t)j * Mrows], br[perm[j]]);
+        for (int j = i; j < N; ++j) zfma(acc, Y[i + (size_t)(unmoved ? perm[j] : j) * Mrows], br[perm[j]]);
         Rg[N + r + (size_t)i * ld] = make_double2(acc.x, -acc.y);
     }
 }
@@ -744,13 +747,15 @@ int wide_solve_batched(ia_context *ctx, int m, int n, int batch, const double2 *
     if (transposed) st = zcopy2d_batched(ctx, n, m, A, n, sA, Y, Mr, (long long)Mr * N, true, batch);
     else st = ztranspose_batched(ctx, m, n, A, m, sA, Y, Mr, (long long)Mr * N, true, batch);
     if (st) return st;
-    if ((st = qr_launch<double2>(ctx, Mr, N, Y, Mr, (long long)Mr * N, tau, 0, nullptr, 0, 0, batch, perm)))
-        return st;
+    const bool unmoved = zqr_ok(Mr, N);
+    st = unmoved ? zqr_pivoted_batched(ctx, Mr, N, Y, Mr, (long long)Mr * N, perm, batch)
+                 : qr_launch<double2>(ctx, Mr, N, Y, Mr, (long long)Mr * N, tau, 0, nullptr, 0, 0, batch, perm);
+    if (st) return st;
     {
         long long total = (long long)N * N;
         int blocks = (int)((total + 255) / 256);
         if (blocks > 512) blocks = 512;
-        build_rh_aug_kernel<<<dim3(blocks, batch), 256, 0, ctx->stream>>>(N, Mr, nrhs, Y, perm, b, Rg);
+        build_rh_aug_kernel<<<dim3(blocks, batch), 256, 0, ctx->stream>>>(N, Mr, nrhs, Y, perm, unmoved ? 1 : 0, b, Rg);
         IA_LAUNCH_CHECK(ctx);
     }
     st = jacobi_rows_batched<double2>(ctx, N + nrhs, N, N, Rg, nullptr, batch, cfg->svd_max_sweeps, info);

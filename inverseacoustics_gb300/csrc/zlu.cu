@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(ZP_THREADS) zlu_panel_kernel(int n, double2 *A
                 if (rank == own_j) P[(size_t)tid * rpc + (j - r0)] = pv;
             }
             prow[tid] = pv;
-            if (tid == j && (pv.x != 0.0 || pv.y != 0.0)) s_inv = zdiv(make_double2(1.0, 0.0), pv);   // one division
+            if (tid == j && (pv.x != 0.0 || pv.y != 0.0)) s_inv = zrcp_x(pv);   // one division
         }
         __syncthreads();
         // multipliers of the rows below j
@@ -457,12 +457,12 @@ size_t zlu_ws_bytes(int n, int nrhs, int batch)
 }
 
 int zgetrf_ws(ia_context *ctx, int n, double2 *A, int lda, long long sA, int *ipiv, int *info, int batch,
-              WsCursor scratch)
+              WsCursor scratch, bool plain)
 {
     if (!zlu_ok(ctx, n)) return zgetrf_batched(ctx, n, A, lda, sA, ipiv, info, batch);
     IA_CUDA_TRY(cudaFuncSetAttribute(zlu_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZP_SMEM_MAX));
     int st;
-    const bool small = n > ZLU_NB && n <= ZLU_SMALL_N;
+    const bool small = plain || (n > ZLU_NB && n <= ZLU_SMALL_N);
     const int NB = small ? ZLU_NB / 2 : ZLU_NB;
     for (int k0 = 0; k0 < n; k0 += NB) {
         const int nb = n - k0 < NB ? n - k0 : NB, kend = k0 + nb, rest = n - kend;
