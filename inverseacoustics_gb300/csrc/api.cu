@@ -1041,7 +1041,7 @@ static int fp64_fallback(ia_context *ctx, const ia_config *cfg, int F, int *d_in
 static size_t solve_ws_bytes(int m, int n, int F, int nrhs, const ia_config *cfg)
 {
     if (use_mixed_wide(m, n, cfg)) return wide_solve_mixed_ws_bytes(m, n, nrhs, F);
-    if (m <= n) return wide_solve_ws_bytes(m, n, nrhs, F);
+    if (m <= n) return wide_solve_ws_bytes(m, n, nrhs, F) + wide_start_ws_bytes(m, F);
     const int p = m < n ? m : n;
     const int M = m >= n ? m : n;
     return ws_round(sizeof(double2) * (size_t)M * p * F) + ws_round(sizeof(double2) * (size_t)p * p * F) +

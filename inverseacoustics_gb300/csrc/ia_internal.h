@@ -1,5 +1,6 @@
 // Internal declarations shared by the libia.so translation units.
 #pragma once
+#include <math.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
@@ -259,7 +260,20 @@ int tc_gemm(ia_context *ctx, const TcPlanes &A, const TcPlanes &B, int M, int N,
 int jacobi_svd_batched(ia_context *ctx, int M, int N, double2 *Y, double2 *V, int batch, int max_sweeps, int *info);
 // Jacobi on Y (M x N) with only the first Mdot rows in the dot products
 template <class T>
-int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int batch, int max_sweeps, int *info);
+int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int batch, int max_sweeps, int *info,
+                        const int *skip = nullptr);
+// the FP64 test: a pair rotates while |y_i^H y_j| > tol |y_i||y_j|
+inline double jacobi_tol_fp64(int rows) { return sqrt((double)rows) * 2.220446049250313e-16; }
+int jacobi_start_batched(ia_context *ctx, int N, float2 *Y, int batch, int max_sweeps);
+int jacobi_flagged_batched(ia_context *ctx, int N, double2 *Y, int batch, const int *skip, const unsigned char *flags);
+// start of the FP64 Jacobi (jstart.cu): M = R K (N x N, R with leading dimension
+// ldr and stride ldr N), K unitary to FP64 rounding, M's columns nearly
+// orthogonal, done[f] set where every pair passes the FP64 test already; scratch
+// of jacobi_precondition_ws_bytes
+bool jacobi_precondition_ok(int N);
+size_t jacobi_precondition_ws_bytes(int N, int batch);
+int jacobi_precondition_batched(ia_context *ctx, int N, const double2 *R, int ldr, double2 *M, int *done, int batch,
+                                int *info, WsCursor cur);
 // sigma, normalised sorted outputs: Uy (M x N) <- Y/sigma, Vs (N x N) <- V, both column-permuted to
 // descending sigma.  Either output may be null.
 int svd_finalize_batched(ia_context *ctx, int M, int N, const double2 *Y, const double2 *V, double *s,
@@ -285,6 +299,9 @@ int gcv_beta_batched(ia_context *ctx, int m, int p, int batch, const double *s, 
 // of A^H when n > m, one-sided Jacobi on R with U^H b carried as extra rows,
 // GCV / Tikhonov, x = Q [U_R (phi .* beta); 0].
 size_t wide_solve_ws_bytes(int m, int n, int nrhs, int batch);
+// what the FP64 solve uses on top of that for a preconditioned Jacobi, where
+// the caller's scratch has it
+size_t wide_start_ws_bytes(int m, int batch);
 int wide_solve_batched(ia_context *ctx, int m, int n, int batch, const double2 *A, bool transposed, int nrhs,
                        const double2 *b, const ia_config *cfg, double2 *x, double *lambda, double *s_out, int *info,
                        WsCursor &cur);

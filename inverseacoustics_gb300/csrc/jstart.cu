@@ -1,0 +1,313 @@
+// Start of the FP64 one-sided Jacobi iteration (wide_solve.cu): M = R K with K
+// unitary and the columns of M nearly orthogonal.
+//
+// On R (here the lower triangular factor R^H of the pivoted QR) the FP64 Jacobi
+// takes 8 to 11 sweeps, nearly all pairs rotating in all but the last
+// two or three, on the FP64 pipe (two FMA per clock and SM; 20 FMA per row of a
+// rotated pair, 8 of a tested one).  Here the rotations are found in FP32 and
+// the FP64 work is products on the tensor cores (10 BF16 slices, zgemm_tc):
+//   1. FP32 Jacobi of R scaled by a power of two, rotations accumulated in J;
+//   2. J's polar factor in FP64: with D = I - J^H J (|D|_F ~ 2e-4 in FP32),
+//      J <- J + J (D / 2 + 3 D^2 / 8 + D^2 (5 D / 16 + 35 D^2 / 128)), unitary to
+//      |D|^5 (cf. Higham, Functions of Matrices, ch. 8);  M = R J: couplings
+//      |m_i^H m_j| / |m_i||m_j| ~ 1e-5;
+//   3. twice: G = M^H M, T_ij = G_ij / (G_jj - G_ii) anti-Hermitian, the
+//      first-order rotation that removes G_ij, with the large entries (near-equal
+//      norms) left out; M <- M K, K = (I + T)(I - T^2)^(-1/2), the polar factor of
+//      I + T, by its series: to T^11 in the first step (|T| <= 0.05), to T^4 in
+//      the second (|T| <= 6e-4).  Each step squares the couplings;
+//   4. what is left -- near-equal singular values, columns at the rounding level
+//      of the largest -- in FP64 sweeps over the pairs that G = M^H M shows above
+//      the Jacobi's test, G anew for each: a sweep costs its rotations and a
+//      barrier per round, not a dot product per pair.
+// The FP64 Jacobi then runs the bins that still fail its test (none, as a rule)
+// as before; a bin whose J is not usable starts from R itself.
+// K is unitary to FP64 rounding, so the decomposition is normwise backward
+// stable; a small column of M carries that rounding of the large ones, so
+// U^H b is formed from U = M / sigma instead of being carried along.
+// (Mixed-precision Jacobi SVD: Gao, Ma, Shao 2022; Hermitian refinement: Ogita
+// and Aishima 2018.)
+#include "ia_common.cuh"
+#include "ia_internal.h"
+
+namespace ia {
+
+// Sizes that take the start.  Solves of N x 4 N operators whose singular values
+// fall to the rounding level (the start's worst case: the tail's pairs still
+// rotate), GB300, without and with it: N = 48, 1 bin 3.33 / 3.46 ms, 150 bins
+// 7.95 / 9.04 ms; 64: 5.07 / 4.85 and 16.2 / 15.7 ms, 512 bins 62.1 / 49.9 ms;
+// 120: 17.9 / 15.0, 92 / 77 and 355 / 261 ms; 256: 104 / 87, 985 / 807 and
+// 3438 / 2822 ms.  The upper end is the FP32 iteration's 2 N = 512 rows.
+// Single-precision-resolved operators gain more: 64 microphones, one bin, the
+// whole ESM solve 4.6 -> 2.28 ms; 160 x 160 by 256 bins 170 -> 83 ms; 256 x 256
+// by 512 order-15 HELS bins 410 -> 130 ms.
+constexpr int JS_MIN_N = 64, JS_MAX_N = 256;
+constexpr int JS_FP32_SWEEPS = 12;
+constexpr double JS_MAX_D = 1e-3;      // largest |J^H J - I|_F: 63/256 |D|^5 = 2.5e-16
+constexpr double JS_MAX_T1 = 0.05;     // largest |T|_F of the first step: 231/1024 |T|^12 = 6e-17
+constexpr double JS_MAX_T2 = 6e-4;     // of the second: 3/8 |T|^5 = 3e-17
+// flagged sweeps: where a tested pair is cheap (few rows) the Jacobi itself
+// finishes as fast
+constexpr int JS_FLAG_SWEEPS = 4, JS_FLAG_SWEEPS_SMALL = 2, JS_SMALL_N = 128;
+constexpr int JS_THREADS = 512;
+
+bool jacobi_precondition_ok(int N) { return N >= JS_MIN_N && N <= JS_MAX_N && tc_fp64_ok(N); }
+
+// 2^-e with |R(0, 0)| < 2^e (the pivoted R's largest entry); 1 for a zero or
+// non-finite R(0, 0)
+__device__ __forceinline__ double js_scale(const double2 *R)
+{
+    const double a = fmax(fabs(R[0].x), fabs(R[0].y));
+    const int e = (int)((__double_as_longlong(a) >> 52) & 0x7FF);
+    return e > 0 && e < 0x7FF ? ldexp(1.0, 1022 - e) : 1.0;
+}
+
+// Y (2 N x N FP32) = R's first N rows, scaled, over the identity
+__global__ void js_init_kernel(int ld, int N, const double2 *__restrict__ R, float2 *__restrict__ Y)
+{
+    const int f = blockIdx.y;
+    R += (size_t)f * ld * N;
+    Y += (size_t)f * 2 * N * N;
+    const double sc = js_scale(R);
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N * N; e += gridDim.x * blockDim.x) {
+        const int c = e / N, r = e - c * N;
+        const double2 v = R[r + (size_t)c * ld];
+        Y[r + (size_t)c * 2 * N] = make_float2((float)(v.x * sc), (float)(v.y * sc));
+        Y[N + r + (size_t)c * 2 * N] = make_float2(r == c ? 1.f : 0.f, 0.f);
+    }
+}
+
+// J (N x N FP64) = the accumulated rotations
+__global__ void js_rotations_kernel(int N, const float2 *__restrict__ Y, double2 *__restrict__ J)
+{
+    const int f = blockIdx.y;
+    Y += (size_t)f * 2 * N * N;
+    J += (size_t)f * N * N;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N * N; e += gridDim.x * blockDim.x) {
+        const int c = e / N, r = e - c * N;
+        const float2 v = Y[N + r + (size_t)c * 2 * N];
+        J[e] = make_double2((double)v.x, (double)v.y);
+    }
+}
+
+__device__ __forceinline__ double js_block_sum(double v, double *red)
+{
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    for (int w = 0; w < JS_THREADS / 32; ++w) t += red[w];
+    __syncthreads();
+    return t;
+}
+
+// E = J^H J -> D = I - E; a bin whose |D| is too large (or not a number) gets
+// J = I, D = 0.  One CTA per bin.
+__global__ void __launch_bounds__(JS_THREADS) js_defect_kernel(int N, double2 *E, double2 *J)
+{
+    __shared__ double red[JS_THREADS / 32];
+    const int f = blockIdx.x;
+    E += (size_t)f * N * N;
+    J += (size_t)f * N * N;
+    double s = 0.0;
+    for (int e = threadIdx.x; e < N * N; e += JS_THREADS) {
+        const int c = e / N, r = e - c * N;
+        double2 d = E[e];
+        d = make_double2((r == c ? 1.0 : 0.0) - d.x, -d.y);
+        E[e] = d;
+        s += zabs2(d);
+    }
+    s = js_block_sum(s, red);
+    if (s <= JS_MAX_D * JS_MAX_D) return;
+    for (int e = threadIdx.x; e < N * N; e += JS_THREADS) {
+        const int c = e / N, r = e - c * N;
+        E[e] = make_double2(0.0, 0.0);
+        J[e] = make_double2(r == c ? 1.0 : 0.0, 0.0);
+    }
+}
+
+// Z = a X + b Y
+__global__ void js_combine_kernel(size_t count, double a, const double2 *__restrict__ X, double b, const double2 *Y,
+                                  double2 *Z)
+{
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < count; e += (size_t)gridDim.x * blockDim.x)
+        Z[e] = make_double2(fma(a, X[e].x, b * Y[e].x), fma(a, X[e].y, b * Y[e].y));
+}
+
+// 1 / x to ~20 bits (T only has to be accurate to the couplings it leaves)
+__device__ __forceinline__ double js_rcp(double x)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    return r;
+}
+
+// G = M^H M -> T in place: T_ij = G_ij / (G_jj - G_ii) where |T_ij| <= theta, the
+// largest of 5e-2, 1e-2 .. 1e-7 that keeps |T|_F <= limit, else 0.  Exactly
+// anti-Hermitian: each pair is computed once.  One CTA per bin.
+constexpr int JS_NT = 7;
+__host__ __device__ constexpr float js_theta2(int q)
+{
+    return q == 0 ? 2.5e-3f : q == 1 ? 1e-4f : q == 2 ? 1e-6f : q == 3 ? 1e-8f : q == 4 ? 1e-10f : q == 5 ? 1e-12f : 1e-14f;
+}
+
+__global__ void __launch_bounds__(JS_THREADS) js_rotation_kernel(int N, double limit, double2 *G)
+{
+    extern __shared__ double js_g[];   // N: diag(G)
+    __shared__ double red[JS_THREADS / 32];
+    const int f = blockIdx.x;
+    G += (size_t)f * N * N;
+    for (int i = threadIdx.x; i < N; i += JS_THREADS) js_g[i] = G[i + (size_t)i * N].x;
+    __syncthreads();
+    double s[JS_NT];
+#pragma unroll
+    for (int q = 0; q < JS_NT; ++q) s[q] = 0.0;
+    for (int e = threadIdx.x; e < N * N; e += JS_THREADS) {
+        const int j = e / N, i = e - j * N;
+        if (i >= j) continue;
+        const double2 g = G[e];
+        const double q = js_rcp(js_g[j] - js_g[i]);
+        const double2 t = make_double2(g.x * q, g.y * q);
+        const double d = zabs2(t);
+        const float m = (float)d;
+        // a zero gap, a NaN and an infinity fail every comparison
+        if (m <= js_theta2(0)) {
+            G[e] = t;
+#pragma unroll
+            for (int k = 0; k < JS_NT; ++k)
+                if (m <= js_theta2(k)) s[k] += d;
+        } else {
+            G[e] = make_double2(0.0, 0.0);
+        }
+    }
+    float keep = -1.f;   // largest |T_ij|^2 kept
+#pragma unroll
+    for (int q = 0; q < JS_NT; ++q) {
+        const double t = 2.0 * js_block_sum(s[q], red);
+        if (keep < 0.f && t <= limit * limit) keep = js_theta2(q);
+    }
+    for (int e = threadIdx.x; e < N * N; e += JS_THREADS) {
+        const int j = e / N, i = e - j * N;
+        if (i > j) continue;
+        if (i == j) {
+            G[e] = make_double2(0.0, 0.0);
+            continue;
+        }
+        double2 t = G[e];
+        if (!((float)zabs2(t) <= keep)) t = make_double2(0.0, 0.0);
+        G[e] = t;
+        G[j + (size_t)i * N] = make_double2(-t.x, t.y);
+    }
+}
+
+// The FP64 Jacobi's test on every pair, from G = M^H M: flags[i + j N] (i < j) for
+// a pair to rotate, done[f] when there is none.  One CTA per bin.
+__global__ void __launch_bounds__(JS_THREADS) js_flags_kernel(int N, double tol, const double2 *G,
+                                                              unsigned char *flags, int *done)
+{
+    extern __shared__ double js_g[];   // N: column norms
+    const int f = blockIdx.x;
+    G += (size_t)f * N * N;
+    flags += (size_t)f * N * N;
+    for (int i = threadIdx.x; i < N; i += JS_THREADS) js_g[i] = sqrt(G[i + (size_t)i * N].x);
+    __syncthreads();
+    int any = 0;
+    for (int e = threadIdx.x; e < N * N; e += JS_THREADS) {
+        const int j = e / N, i = e - j * N;
+        const double b = tol * js_g[i] * js_g[j];
+        const bool rot = i < j && zabs2(G[e]) > b * b;
+        flags[e] = rot ? 1 : 0;
+        any |= rot ? 1 : 0;
+    }
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0) done[f] = !any;
+}
+
+size_t jacobi_precondition_ws_bytes(int N, int batch)
+{
+    const size_t nn = (size_t)N * N * batch;
+    return 5 * ws_round(16 * nn) + ws_round(nn) + zgemm_tc_ws_bytes(N, N, N, batch) + 2048;
+}
+
+int jacobi_precondition_batched(ia_context *ctx, int N, const double2 *R, int ldr, double2 *M, int *done, int batch,
+                                int *info, WsCursor cur)
+{
+    const long long nn = (long long)N * N;
+    const size_t count = (size_t)nn * batch;
+    float2 *Y = cur.take<float2>(2 * count);
+    double2 *J = cur.take<double2>(count), *D = cur.take<double2>(count), *Q = cur.take<double2>(count),
+            *P = cur.take<double2>(count);
+    unsigned char *flags = cur.take<unsigned char>(count);
+    if (cur.off > cur.cap) return IA_ERR_ALLOC;
+    int st;
+    int blocks = (int)((nn + 255) / 256);
+    if (blocks > 64) blocks = 64;
+    const dim3 grid(blocks, batch);
+    const size_t want = (count + 255) / 256, cap = (size_t)ctx->sm_count * 8;
+    const int flat = (int)(want < cap ? want : cap);
+    // C = op(A) B + beta C, N x N
+    auto prod = [&](Op opa, const double2 *A, int lda, const double2 *B, double beta, double2 *C) {
+        return zgemm_tc(ctx, opa, OP_N, N, N, N, 1.0, A, lda, (long long)lda * N, B, N, nn, beta, C, N, nn, batch, info,
+                        cur);
+    };
+    auto combine = [&](double a, const double2 *X, double b, const double2 *Z, double2 *W) -> int {
+        js_combine_kernel<<<flat, 256, 0, ctx->stream>>>(count, a, X, b, Z, W);
+        IA_LAUNCH_CHECK(ctx);
+        return IA_OK;
+    };
+    js_init_kernel<<<grid, 256, 0, ctx->stream>>>(ldr, N, R, Y);
+    IA_LAUNCH_CHECK(ctx);
+    if ((st = jacobi_start_batched(ctx, N, Y, batch, JS_FP32_SWEEPS))) return st;
+    js_rotations_kernel<<<grid, 256, 0, ctx->stream>>>(N, Y, J);
+    IA_LAUNCH_CHECK(ctx);
+    // J to its polar factor (M holds the product's second operand), M = R J
+    if ((st = prod(OP_C, J, N, J, 0.0, D))) return st;
+    js_defect_kernel<<<batch, JS_THREADS, 0, ctx->stream>>>(N, D, J);
+    IA_LAUNCH_CHECK(ctx);
+    if ((st = prod(OP_N, D, N, D, 0.0, Q))) return st;
+    if ((st = combine(0.5, D, 0.375, Q, P))) return st;
+    if ((st = combine(0.3125, D, 35.0 / 128.0, Q, M))) return st;
+    if ((st = prod(OP_N, Q, N, M, 1.0, P))) return st;
+    if ((st = prod(OP_N, J, N, P, 1.0, J))) return st;
+    if ((st = prod(OP_N, R, ldr, J, 0.0, M))) return st;
+    const size_t nsm = sizeof(double) * (size_t)N;
+    // first step: p = (I - T^2)^(-1/2) - I to (T^2)^5, P = T + p + T p
+    if ((st = prod(OP_C, M, N, M, 0.0, D))) return st;
+    js_rotation_kernel<<<batch, JS_THREADS, nsm, ctx->stream>>>(N, JS_MAX_T1, D);
+    IA_LAUNCH_CHECK(ctx);
+    {
+        // D = T, Q = T^2, J = T^4, P = T^6, then P = 5/16 Q + 35/128 J + 63/256 P
+        double2 *T = D, *S = reinterpret_cast<double2 *>(Y);   // (Y's 2 N^2 FP32 pairs: N^2 FP64 ones)
+        if ((st = prod(OP_N, T, N, T, 0.0, Q))) return st;
+        if ((st = prod(OP_N, Q, N, Q, 0.0, J))) return st;
+        if ((st = prod(OP_N, Q, N, J, 0.0, P))) return st;
+        if ((st = combine(35.0 / 128.0, J, 63.0 / 256.0, P, P))) return st;
+        if ((st = combine(5.0 / 16.0, Q, 1.0, P, P))) return st;
+        if ((st = combine(0.5, Q, 0.375, J, S))) return st;
+        if ((st = prod(OP_N, J, N, P, 1.0, S))) return st;      // p
+        if ((st = combine(1.0, T, 1.0, S, P))) return st;
+        if ((st = prod(OP_N, T, N, S, 1.0, P))) return st;
+        if ((st = prod(OP_N, M, N, P, 1.0, M))) return st;
+    }
+    // second step: P = T + T^2 / 2 + T^2 (T / 2 + 3 T^2 / 8)
+    if ((st = prod(OP_C, M, N, M, 0.0, D))) return st;
+    js_rotation_kernel<<<batch, JS_THREADS, nsm, ctx->stream>>>(N, JS_MAX_T2, D);
+    IA_LAUNCH_CHECK(ctx);
+    if ((st = prod(OP_N, D, N, D, 0.0, Q))) return st;
+    if ((st = combine(0.5, D, 0.375, Q, J))) return st;
+    if ((st = combine(1.0, D, 0.5, Q, P))) return st;
+    if ((st = prod(OP_N, Q, N, J, 1.0, P))) return st;
+    if ((st = prod(OP_N, M, N, P, 1.0, M))) return st;
+    // sweeps over the pairs above the test
+    const int sweeps = N > JS_SMALL_N ? JS_FLAG_SWEEPS : JS_FLAG_SWEEPS_SMALL;
+    for (int it = 0;; ++it) {
+        if ((st = prod(OP_C, M, N, M, 0.0, D))) return st;
+        js_flags_kernel<<<batch, JS_THREADS, nsm, ctx->stream>>>(N, jacobi_tol_fp64(N), D, flags, done);
+        IA_LAUNCH_CHECK(ctx);
+        if (it == sweeps) break;
+        if ((st = jacobi_flagged_batched(ctx, N, M, batch, done, flags))) return st;
+    }
+    return IA_OK;
+}
+
+}  // namespace ia

@@ -59,6 +59,28 @@ __device__ __forceinline__ bool jacobi_rotation(R a, R b, T g, R tol, R &c, T &s
     return true;
 }
 
+// jacobi_rotation for a start whose columns span more than FP32's squares can
+// (norms down to 1e-17 of the largest): the modulus of g from scaled parts, so
+// that the rotation is unitary whatever g's size, and no rotation with a column
+// whose squared norm nears the underflow limit (an iteration in FP64 follows)
+__device__ __forceinline__ bool jacobi_rotation_start(float a, float b, float2 g, float tol, float &c, float2 &sp,
+                                                      float &rel)
+{
+    const float m = fmaxf(fabsf(g.x), fabsf(g.y));
+    if (!(fminf(a, b) > 1e-33f) || !(m > 0.f)) return false;
+    const float x = g.x / m, y = g.y / m, h = sqrtf(x * x + y * y), gm = m * h;
+    const float sab = sqrtf(a) * sqrtf(b);
+    if (!(gm > tol * sab)) return false;
+    rel = gm / sab;
+    const float zeta = (b - a) / (2 * gm);
+    const float t = fabsf(zeta) > 1e18f ? 0.5f / zeta
+                                         : (zeta >= 0 ? 1.f : -1.f) / (fabsf(zeta) + sqrtf(1 + zeta * zeta));
+    c = 1 / sqrtf(1 + t * t);
+    const float s = t * c;
+    sp = make_float2(s * (x / h), s * (y / h));
+    return true;
+}
+
 template <class T>
 __device__ __forceinline__ void rotate_pair(T &u, T &v, typename ctraits<T>::R c, T sp)
 {
@@ -73,11 +95,13 @@ __device__ __forceinline__ void rotate_pair(T &u, T &v, typename ctraits<T>::R c
 template <class T, int KPL>
 __global__ void __launch_bounds__(SVD_MAX_WARPS * 32) jacobi_kernel(int M, int Mdot, int N, T *Y, long long sY, T *V,
                                                                       long long sV, int max_sweeps,
-                                                                      typename ctraits<T>::R tol, int *info)
+                                                                      typename ctraits<T>::R tol, int *info,
+                                                                      const int *skip)
 {
     typedef typename ctraits<T>::R R;
     __shared__ int s_rot;
     const int f = blockIdx.x;
+    if (skip && skip[f]) return;
     Y += f * sY;
     if (V) V += f * sV;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -271,7 +295,7 @@ __device__ __forceinline__ typename ctraits<T>::R half_sum(typename ctraits<T>::
 template <class T>
 __global__ void __launch_bounds__(sizeof(T) <= 8 ? 1024 : 512)
     jacobi_half_kernel(int M, int Mdot, int N, T *Yg, long long sY, int max_sweeps, typename ctraits<T>::R tol,
-                       int *info)
+                       int *info, const int *skip)
 {
     typedef typename ctraits<T>::R R;
     constexpr int KPL = 8;
@@ -280,6 +304,7 @@ __global__ void __launch_bounds__(sizeof(T) <= 8 ? 1024 : 512)
     __shared__ int s_rot;
     __shared__ unsigned s_maxrel;   // largest |y_i^H y_j| / (|y_i||y_j|) rotated in the sweep (float bits)
     const int f = blockIdx.x;
+    if (skip && skip[f]) return;
     Yg += f * sY;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int half = lane >> 4, hl = lane & 15;
@@ -373,16 +398,27 @@ __global__ void __launch_bounds__(sizeof(T) <= 8 ? 1024 : 512)
 // reductions, rotation and stopping rule; the sweep's rotation count and
 // largest coupling are combined over the cluster), so the factors are
 // bitwise the same.
-template <class T, int KPL = 8>
+//
+// MODE: JC_PLAIN; JC_START, the FP32 start of an FP64 iteration; JC_FLAGGED, one
+// FP64 sweep over the pairs (i, j), i < j, whose byte flags[i + j N] is set
+// (the others were tested elsewhere): unflagged pairs cost nothing but the
+// round's barrier.  CSC: the cluster size when fixed (0: read at run time).
+// Bins with skip[f] set are left alone.
+enum { JC_PLAIN = 0, JC_START = 1, JC_FLAGGED = 2 };
+
+template <class T, int KPL = 8, int MODE = JC_PLAIN, int CSC = 0>
 __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
-    jacobi_cluster_kernel(int M, int Mdot, int N, T *Yg, long long sY, int max_sweeps, typename ctraits<T>::R tol,
-                          int *info)
+    jacobi_cluster_kernel(int M, int Mdot, int N, int N2, T *Yg, long long sY, int max_sweeps,
+                          typename ctraits<T>::R tol, int *info, const int *skip, const unsigned char *flags)
 {
+    constexpr bool START = MODE == JC_START;
     typedef typename ctraits<T>::R R;
     cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank(), JC_CS = (int)cluster.num_blocks();
+    const int rank = (int)cluster.block_rank(), JC_CS = CSC ? CSC : (int)cluster.num_blocks();
     const int f = blockIdx.x / JC_CS;
-    const int N2 = N + (N & 1), NR = N2 - 1, P = N2 / 2 / JC_CS, RING = P + 1, k0 = rank * P;
+    if (skip && skip[f]) return;   // the whole cluster
+    // N2 >= N slots, a multiple of 2 JC_CS; columns past N are zero and never rotate
+    const int NR = N2 - 1, P = N2 / 2 / JC_CS, RING = P + 1, k0 = rank * P;
     extern __shared__ __align__(16) unsigned char jc_raw[];
     T *up = reinterpret_cast<T *>(jc_raw);   // RING x M: upper columns, entry (slot + t) mod RING
     T *lo = up + (size_t)RING * M;           // RING x M: lower columns, entry (slot - t) mod RING
@@ -413,6 +449,20 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
         s_rot[0] = s_rot[1] = 0;
         s_rel[0] = s_rel[1] = 0u;
     }
+    // JC_FLAGGED: this CTA's flagged slots per round, a bit each
+    const int MW = (P + 31) / 32;
+    unsigned *fmask = reinterpret_cast<unsigned *>(fixc + M);   // NR x MW
+    if constexpr (MODE == JC_FLAGGED) {
+        flags += (size_t)f * N * N;
+        for (int e = threadIdx.x; e < NR * MW; e += blockDim.x) fmask[e] = 0u;
+        __syncthreads();
+        for (int e = threadIdx.x; e < NR * P; e += blockDim.x) {
+            const int rr = e / P, s = e - rr * P;
+            const int cu = col_up(k0 + s, rr), cl = col_lo(k0 + s, rr);
+            const int i = cu < cl ? cu : cl, j = cu < cl ? cl : cu;
+            if (j < N && flags[i + (size_t)j * N]) atomicOr(&fmask[rr * MW + s / 32], 1u << (s & 31));
+        }
+    }
     cluster.sync();
     int r = 0, t = 0, par = 0, sweep = 0;   // round mod NR, round mod RING
     for (; sweep < max_sweeps; ++sweep) {
@@ -422,6 +472,8 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
             const int tn = t + 1 == RING ? 0 : t + 1;
             for (int s = hw; s < P; s += 2 * nw) {
                 const int k = k0 + s;
+                const bool flagged = MODE != JC_FLAGGED || (fmask[r * MW + s / 32] >> (s & 31) & 1u);
+                if (MODE == JC_FLAGGED && !flagged && s != 0 && s != P - 1) continue;
                 const int cu = col_up(k, r), cl = col_lo(k, r);
                 int eu = s + t;
                 if (eu >= RING) eu -= RING;
@@ -438,7 +490,7 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
                     ui[q] = rr < M ? yi[rr] : zero;
                     uj[q] = rr < M ? yj[rr] : zero;
                 }
-                if (j < N) {
+                if (j < N && flagged) {
                     R a = 0, b = 0, c;
                     T g = zero, sp;
 #pragma unroll
@@ -454,7 +506,10 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
                     g.x = half_sum<T>(g.x, mask);
                     g.y = half_sum<T>(g.y, mask);
                     R rel = 0;
-                    if (jacobi_rotation(a, b, g, tol, c, sp, sizeof(R) == 4 ? &rel : nullptr)) {
+                    bool rotate;
+                    if constexpr (START) rotate = jacobi_rotation_start(a, b, g, tol, c, sp, rel);
+                    else rotate = jacobi_rotation(a, b, g, tol, c, sp, sizeof(R) == 4 ? &rel : nullptr);
+                    if (rotate) {
                         relmax = fmaxf(relmax, (float)rel);
 #pragma unroll
                         for (int q = 0; q < KPL; ++q) {
@@ -710,7 +765,8 @@ static int jacobi_wide(ia_context *ctx, int M, int Mdot, int N, T *Y, long long 
 }
 
 template <class T>
-int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int batch, int max_sweeps, int *info)
+int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int batch, int max_sweeps, int *info,
+                        const int *skip)
 {
     typedef typename ctraits<T>::R R;
     if (V) {
@@ -726,8 +782,7 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
     // the rounding noise of FP32 dot products.  A looser start (64x) cut the
     // FP32 sweeps but left more coupled pairs for the FP64 Jacobi on X^H E X
     // and made the whole solve slower.
-    const double eps = sizeof(R) == 8 ? 2.220446049250313e-16 : 8.0 * 1.1920928955078125e-07;
-    const R tol = (R)(sqrt((double)Mdot) * eps);
+    const R tol = sizeof(R) == 8 ? (R)jacobi_tol_fp64(Mdot) : (R)(sqrt((double)Mdot) * (8.0 * 1.1920928955078125e-07));
     const long long sY = (long long)M * N, sV = (long long)N * N;
     const size_t smem = sizeof(T) * (size_t)M * N;
     // without accumulator: a half-warp per pair (FP32: every pair of a round at
@@ -737,7 +792,7 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
     {
         // over a cluster per bin: FP32 for batches that leave most of the GPU
         // idle and for the last part of a staggered pipeline (4x the SMs for
-        // ~0.7x the time per bin); FP64 whenever 2 or 4 CTAs per bin fit on
+        // ~0.7x the time per bin); FP64 whenever 2 to 8 CTAs per bin fit on
         // the SMs (the FP64 pipe of more SMs per bin).  Systems of 129-272 rows
         // (12 or 17 rows per lane) take 8-CTA clusters in as many waves as
         // needed: their alternative is a one-CTA kernel on global memory.
@@ -758,7 +813,7 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
             lc.dynamicSmemBytes = sizeof(T) * ((size_t)2 * (P + 1) * M + M);
             at[0].val.clusterDim.x = c;
         };
-        auto kern = jacobi_cluster_kernel<T, 8>;
+        auto kern = sizeof(T) == 8 ? jacobi_cluster_kernel<T, 8, JC_PLAIN, 4> : jacobi_cluster_kernel<T, 8>;
         if (!V && M <= 128 && N <= 128) {
             if (sizeof(T) == 8) {
                 if (np % 4 == 0 && np / 4 >= 2 && (16 * batch <= ctx->sm_count || ctx->tail_part)) cs = 4;
@@ -789,7 +844,8 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
             if (lc.dynamicSmemBytes > 48 * 1024)
                 IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)lc.dynamicSmemBytes));
-            IA_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, M, Mdot, N, Y, sY, max_sweeps, tol, info));
+            IA_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, M, Mdot, N, N + (N & 1), Y, sY, max_sweeps, tol, info, skip,
+                                           (const unsigned char *)nullptr));
             IA_LAUNCH_CHECK(ctx);
             return IA_OK;
         }
@@ -802,7 +858,7 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
         if (nws < 1) nws = 1;
         IA_CUDA_TRY(cudaFuncSetAttribute(jacobi_half_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)half_smem_max));
-        jacobi_half_kernel<T><<<batch, nws * 32, smem, ctx->stream>>>(M, Mdot, N, Y, sY, max_sweeps, tol, info);
+        jacobi_half_kernel<T><<<batch, nws * 32, smem, ctx->stream>>>(M, Mdot, N, Y, sY, max_sweeps, tol, info, skip);
     } else if (M <= 128 && N <= 128 && smem <= 200 * 1024) {
         const int wmax = sizeof(T) <= 8 ? 2 * SVD_MAX_WARPS : SVD_MAX_WARPS;
         int nws = (N + 1) / 2 < wmax ? (N + 1) / 2 : wmax;
@@ -812,9 +868,9 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
         jacobi_smem_kernel<T, 4><<<batch, nws * 32, smem, ctx->stream>>>(M, Mdot, N, Y, sY, V, sV, max_sweeps, tol,
                                                                          info);
     } else if (M <= 128)
-        jacobi_kernel<T, 4><<<batch, nw * 32, 0, ctx->stream>>>(M, Mdot, N, Y, sY, V, sV, max_sweeps, tol, info);
+        jacobi_kernel<T, 4><<<batch, nw * 32, 0, ctx->stream>>>(M, Mdot, N, Y, sY, V, sV, max_sweeps, tol, info, skip);
     else if (M <= 256)
-        jacobi_kernel<T, 8><<<batch, nw * 32, 0, ctx->stream>>>(M, Mdot, N, Y, sY, V, sV, max_sweeps, tol, info);
+        jacobi_kernel<T, 8><<<batch, nw * 32, 0, ctx->stream>>>(M, Mdot, N, Y, sY, V, sV, max_sweeps, tol, info, skip);
     else {
         // large systems, few of them (one CTA per bin would leave most SMs
         // idle): over the whole GPU, round by round, where the host may
@@ -825,13 +881,68 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
         IA_CUDA_TRY(cudaStreamIsCapturing(ctx->stream, &cs));
         if (cs == cudaStreamCaptureStatusNone && !ctx->capturing && 2 * batch <= ctx->sm_count)
             return jacobi_wide<T>(ctx, M, Mdot, N, Y, sY, V, sV, batch, max_sweeps, tol, info);
-        jacobi_kernel<T, 0><<<batch, nw * 32, 0, ctx->stream>>>(M, Mdot, N, Y, sY, V, sV, max_sweeps, tol, info);
+        jacobi_kernel<T, 0><<<batch, nw * 32, 0, ctx->stream>>>(M, Mdot, N, Y, sY, V, sV, max_sweeps, tol, info, skip);
     }
     IA_LAUNCH_CHECK(ctx);
     return IA_OK;
 }
-template int jacobi_rows_batched<double2>(ia_context *, int, int, int, double2 *, double2 *, int, int, int *);
-template int jacobi_rows_batched<float2>(ia_context *, int, int, int, float2 *, float2 *, int, int, int *);
+template int jacobi_rows_batched<double2>(ia_context *, int, int, int, double2 *, double2 *, int, int, int *,
+                                          const int *);
+template int jacobi_rows_batched<float2>(ia_context *, int, int, int, float2 *, float2 *, int, int, int *,
+                                         const int *);
+
+template <class T, int MODE>
+static int jc_launch(ia_context *ctx, int M, int Mdot, int N, T *Y, int batch, int max_sweeps,
+                     typename ctraits<T>::R tol, const int *skip, const unsigned char *flags)
+{
+    // clusters of 8 whatever the batch (a round is latency-bound), N padded to
+    // whole slots
+    constexpr int cs = 8;
+    const int N2 = (N + 15) / 16 * 16, P = N2 / 2 / cs;
+    if (P < 2 || M > (sizeof(T) == sizeof(float2) ? 512 : 272)) return IA_ERR_ARG;
+    cudaLaunchConfig_t lc = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    lc.stream = ctx->stream;
+    constexpr bool F32 = sizeof(T) == sizeof(float2);
+    auto kern = jacobi_cluster_kernel<T, 8, MODE>;
+    if (M > 128) kern = F32 ? (M <= 256 ? jacobi_cluster_kernel<T, F32 ? 16 : 12, MODE>
+                                        : jacobi_cluster_kernel<T, F32 ? 32 : 17, MODE>)
+                            : (M <= 192 ? jacobi_cluster_kernel<T, F32 ? 16 : 12, MODE>
+                                        : jacobi_cluster_kernel<T, F32 ? 32 : 17, MODE>);
+    lc.gridDim = dim3((unsigned)(cs * batch));
+    lc.blockDim = dim3((unsigned)(32 * ((P + 1) / 2)));
+    lc.dynamicSmemBytes = sizeof(T) * ((size_t)2 * (P + 1) * M + M) +
+                          (MODE == JC_FLAGGED ? sizeof(unsigned) * (size_t)N2 * ((P + 31) / 32) : 0);
+    at[0].val.clusterDim.x = cs;
+    if (lc.dynamicSmemBytes > 48 * 1024)
+        IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lc.dynamicSmemBytes));
+    IA_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, M, Mdot, N, N2, Y, (long long)M * N, max_sweeps, tol, (int *)nullptr,
+                                   skip, flags));
+    IA_LAUNCH_CHECK(ctx);
+    return IA_OK;
+}
+
+// FP32 one-sided Jacobi of batch N x N matrices with the rotations accumulated:
+// Y (2 N x N) holds the matrix over the identity on entry, which the rotations
+// turn into J (only the first N rows enter the dot products).  A start for an
+// FP64 iteration: the sweep cap is not an error, and columns whose products
+// underflow stay as they are.
+int jacobi_start_batched(ia_context *ctx, int N, float2 *Y, int batch, int max_sweeps)
+{
+    const float tol = (float)(sqrt((double)N) * 8.0 * 1.1920928955078125e-07);
+    return jc_launch<float2, JC_START>(ctx, 2 * N, N, N, Y, batch, max_sweeps, tol, nullptr, nullptr);
+}
+
+// one FP64 sweep of Y (N x N) over the flagged pairs
+int jacobi_flagged_batched(ia_context *ctx, int N, double2 *Y, int batch, const int *skip, const unsigned char *flags)
+{
+    return jc_launch<double2, JC_FLAGGED>(ctx, N, N, N, Y, batch, 1, jacobi_tol_fp64(N), skip, flags);
+}
 
 int jacobi_svd_batched(ia_context *ctx, int M, int N, double2 *Y, double2 *V, int batch, int max_sweeps, int *info)
 {

@@ -669,14 +669,14 @@ __global__ void build_rh_aug_kernel(int N, int Mrows, int nrhs, const double2 *Y
 // After the Jacobi on Raug: sigma_i = |column i of R^H J| (sorted, S), the
 // rank of each column (RANK), beta = Sigma^-1 J^H v (sorted, BETA) and the
 // left singular vectors U = P W, W = (R^H J) Sigma^-1, in the columns' own
-// order (X, N x N).
-__global__ void finalize_dv_kernel(int N, int nrhs, const double2 *Rg, const int *perm, double *S, double2 *BETA,
-                                   double2 *X, int *RANK, int *info)
+// order (X, N x N).  Rg has leading dimension ld; with B (batch x nrhs x N)
+// nothing is carried and beta = U^H b is formed here.
+__global__ void finalize_dv_kernel(int N, int ld, int nrhs, const double2 *Rg, const int *perm, const double2 *B,
+                                   double *S, double2 *BETA, double2 *X, int *RANK, int *info)
 {
     extern __shared__ double sm_dv[];
     double *sig = sm_dv;
     const int f = blockIdx.x;
-    const int ld = N + nrhs;
     Rg += (size_t)f * ld * N;
     perm += (size_t)f * N;
     X += (size_t)f * N * N;
@@ -699,7 +699,7 @@ __global__ void finalize_dv_kernel(int N, int nrhs, const double2 *Rg, const int
         S[(size_t)f * N + rk] = sj;
         if (info && (!(sj == sj) || isinf(sj))) atomicOr(&info[f], IA_INFO_NONFINITE);
         const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
-        for (int r = 0; r < nrhs; ++r) {
+        for (int r = 0; r < nrhs && !B; ++r) {
             const double2 v = Rg[N + r + (size_t)j * ld];
             BETA[((size_t)f * nrhs + r) * N + rk] = make_double2(v.x * inv, -v.y * inv);
         }
@@ -708,6 +708,18 @@ __global__ void finalize_dv_kernel(int N, int nrhs, const double2 *Rg, const int
         const double inv = sig[j] > 0.0 ? 1.0 / sig[j] : 0.0;
         for (int r = lane; r < N; r += 32) X[perm[r] + (size_t)j * N] = zscale(Rg[r + (size_t)j * ld], inv);
     }
+    if (!B) return;
+    __syncthreads();   // RANK
+    for (int j = wid; j < N; j += nw) {
+        const double inv = sig[j] > 0.0 ? 1.0 / sig[j] : 0.0;
+        for (int rr = 0; rr < nrhs; ++rr) {
+            const double2 *b = B + ((size_t)f * nrhs + rr) * N;
+            double2 acc = make_double2(0.0, 0.0);
+            for (int r = lane; r < N; r += 32) zcfma(acc, Rg[r + (size_t)j * ld], b[perm[r]]);
+            acc = warp_sum2(acc);
+            if (lane == 0) BETA[((size_t)f * nrhs + rr) * N + RANK[(size_t)f * N + j]] = zscale(acc, inv);
+        }
+    }
 }
 
 size_t wide_solve_ws_bytes(int m, int n, int nrhs, int batch)
@@ -715,6 +727,13 @@ size_t wide_solve_ws_bytes(int m, int n, int nrhs, int batch)
     const size_t F = batch, N = m, M = n, R = nrhs;
     return ws_round(16 * M * N * F) + ws_round(16 * N * F) + ws_round(16 * (N + R) * N * F) + ws_round(8 * N * F) +
            ws_round(16 * R * N * F) * 2 + ws_round(16 * N * N * F) + 2 * ws_round(4 * N * F) + 2048;
+}
+
+size_t wide_start_ws_bytes(int m, int batch)
+{
+    if (!jacobi_precondition_ok(m)) return 0;
+    return ws_round(16 * (size_t)m * m * batch) + ws_round(4 * (size_t)batch) + jacobi_precondition_ws_bytes(m, batch) +
+           512;
 }
 
 // FP64 wide solve (Drmac-Veselic preconditioned one-sided Jacobi):
@@ -758,10 +777,22 @@ int wide_solve_batched(ia_context *ctx, int m, int n, int batch, const double2 *
         build_rh_aug_kernel<<<dim3(blocks, batch), 256, 0, ctx->stream>>>(N, Mr, nrhs, Y, perm, unmoved ? 1 : 0, b, Rg);
         IA_LAUNCH_CHECK(ctx);
     }
-    st = jacobi_rows_batched<double2>(ctx, N + nrhs, N, N, Rg, nullptr, batch, cfg->svd_max_sweeps, info);
+    // the Jacobi starts from R^H K (jstart.cu), which as a rule passes its test
+    const size_t extra = wide_start_ws_bytes(m, batch);
+    const bool started = !ctx->plain_fp64 && extra && cur.off + extra <= cur.cap;
+    int *done = nullptr;
+    if (started) {
+        double2 *M = cur.take<double2>((size_t)N * N * batch);
+        done = cur.take<int>((size_t)batch);
+        if ((st = jacobi_precondition_batched(ctx, N, Rg, N + nrhs, M, done, batch, info, cur))) return st;
+        Rg = M;
+    }
+    const int rows = started ? N : N + nrhs;
+    st = jacobi_rows_batched<double2>(ctx, rows, N, N, Rg, nullptr, batch, cfg->svd_max_sweeps, info, done);
     if (st) return st;
-    finalize_dv_kernel<<<batch, 256, (size_t)N * sizeof(double), ctx->stream>>>(N, nrhs, Rg, perm, s, beta, X, rank,
-                                                                                 info);
+    finalize_dv_kernel<<<batch, 256, (size_t)N * sizeof(double), ctx->stream>>>(N, rows, nrhs, Rg, perm,
+                                                                                 started ? b : nullptr, s, beta, X,
+                                                                                 rank, info);
     IA_LAUNCH_CHECK(ctx);
     st = gcv_beta_batched(ctx, m, N, batch, s, nrhs, beta, nullptr, cfg, z, lambda);
     if (st) return st;
