@@ -264,8 +264,12 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
                         const int *skip = nullptr);
 // the FP64 test: a pair rotates while |y_i^H y_j| > tol |y_i||y_j|
 inline double jacobi_tol_fp64(int rows) { return sqrt((double)rows) * 2.220446049250313e-16; }
-int jacobi_start_batched(ia_context *ctx, int N, float2 *Y, int batch, int max_sweeps);
-int jacobi_flagged_batched(ia_context *ctx, int N, double2 *Y, int batch, const int *skip, const unsigned char *flags);
+size_t jacobi_start_ws_bytes(int N, int max_sweeps, int batch);
+int jacobi_start_batched(ia_context *ctx, int N, float2 *Y, float2 *J, int batch, int max_sweeps, WsCursor cur);
+// column slots of the start's and the flagged sweeps' pair ordering: N padded to
+// clusters of 8
+inline int jacobi_slots(int N) { return (N + 15) / 16 * 16; }
+int jacobi_flagged_batched(ia_context *ctx, int N, double2 *Y, int batch, int *done, const unsigned char *flags);
 // start of the FP64 Jacobi (jstart.cu): M = R K (N x N, R with leading dimension
 // ldr and stride ldr N), K unitary to FP64 rounding, M's columns nearly
 // orthogonal, done[f] set where every pair passes the FP64 test already; scratch

@@ -6,22 +6,29 @@
 // two or three, on the FP64 pipe (two FMA per clock and SM; 20 FMA per row of a
 // rotated pair, 8 of a tested one).  Here the rotations are found in FP32 and
 // the FP64 work is products on the tensor cores (10 BF16 slices, zgemm_tc):
-//   1. FP32 Jacobi of R scaled by a power of two, rotations accumulated in J;
+//   1. FP32 Jacobi of R scaled by a power of two; the rotations are recorded and
+//      then applied to J;
 //   2. J's polar factor in FP64: with D = I - J^H J (|D|_F ~ 2e-4 in FP32),
 //      J <- J + J (D / 2 + 3 D^2 / 8 + D^2 (5 D / 16 + 35 D^2 / 128)), unitary to
 //      |D|^5 (cf. Higham, Functions of Matrices, ch. 8);  M = R J: couplings
 //      |m_i^H m_j| / |m_i||m_j| ~ 1e-5;
-//   3. twice: G = M^H M, T_ij = G_ij / (G_jj - G_ii) anti-Hermitian, the
+//   3. three times: G = M^H M, T_ij = G_ij / (G_jj - G_ii) anti-Hermitian, the
 //      first-order rotation that removes G_ij, with the large entries (near-equal
 //      norms) left out; M <- M K, K = (I + T)(I - T^2)^(-1/2), the polar factor of
 //      I + T, by its series: to T^11 in the first step (|T| <= 0.05), to T^4 in
-//      the second (|T| <= 6e-4).  Each step squares the couplings;
+//      the second (|T| <= 6e-4), to T^2 in the third (|T| <= 5e-6).  Each step
+//      squares the couplings; the third clears the smallest columns, whose
+//      products the large ones hide before the first.  A step runs
+//      on M D^-1 and D T D^-1, D the column norms: a slice product's error is
+//      relative to the largest entries of a row and a column, which would leave
+//      columns far below the largest with the large ones' rounding (order-15 HELS:
+//      22,000 of 32,640 pairs left to rotate);
 //   4. what is left -- near-equal singular values, columns at the rounding level
 //      of the largest -- in FP64 sweeps over the pairs that G = M^H M shows above
 //      the Jacobi's test, G anew for each: a sweep costs its rotations and a
 //      barrier per round, not a dot product per pair.
-// The FP64 Jacobi then runs the bins that still fail its test (none, as a rule)
-// as before; a bin whose J is not usable starts from R itself.
+// A bin is done when none of its pairs is above the test; the FP64 Jacobi runs
+// those that are not (none, as a rule) as before; a bin whose J is not usable starts from R itself.
 // K is unitary to FP64 rounding, so the decomposition is normwise backward
 // stable; a small column of M carries that rounding of the large ones, so
 // U^H b is formed from U = M / sigma instead of being carried along.
@@ -37,18 +44,20 @@ namespace ia {
 // rotate), GB300, without and with it: N = 48, 1 bin 3.33 / 3.46 ms, 150 bins
 // 7.95 / 9.04 ms; 64: 5.07 / 4.85 and 16.2 / 15.7 ms, 512 bins 62.1 / 49.9 ms;
 // 120: 17.9 / 15.0, 92 / 77 and 355 / 261 ms; 256: 104 / 87, 985 / 807 and
-// 3438 / 2822 ms.  The upper end is the FP32 iteration's 2 N = 512 rows.
-// Single-precision-resolved operators gain more: 64 microphones, one bin, the
-// whole ESM solve 4.6 -> 2.28 ms; 160 x 160 by 256 bins 170 -> 83 ms; 256 x 256
-// by 512 order-15 HELS bins 410 -> 130 ms.
+// 3438 / 2822 ms.  The upper end is the recorded rotations' 128 slots.
+// (measured with the rotations still carried along: the figures below are
+// today's).  Operators above that level gain more: 64 microphones, one bin, the
+// whole ESM solve 4.7 -> 2.5 ms; 192 microphones, 48 bins 170 -> 61 ms; 64 order-15
+// HELS bins (256 x 256) 401 -> 54 to 63 ms, the more the more bins need the FP64
+// Jacobi's last sweep.
 constexpr int JS_MIN_N = 64, JS_MAX_N = 256;
 constexpr int JS_FP32_SWEEPS = 12;
 constexpr double JS_MAX_D = 1e-3;      // largest |J^H J - I|_F: 63/256 |D|^5 = 2.5e-16
-constexpr double JS_MAX_T1 = 0.05;     // largest |T|_F of the first step: 231/1024 |T|^12 = 6e-17
-constexpr double JS_MAX_T2 = 6e-4;     // of the second: 3/8 |T|^5 = 3e-17
-// flagged sweeps: where a tested pair is cheap (few rows) the Jacobi itself
-// finishes as fast
-constexpr int JS_FLAG_SWEEPS = 4, JS_FLAG_SWEEPS_SMALL = 2, JS_SMALL_N = 128;
+constexpr float JS_MAX_T1 = 0.05f;     // largest |T|_F of the first step: 231/1024 |T|^12 = 6e-17
+constexpr float JS_MAX_T2 = 6e-4f;     // of the second: 3/8 |T|^5 = 3e-17
+constexpr float JS_MAX_T3 = 5e-6f;     // of the third: |T|^3 / 2 = 6e-17
+// flagged sweeps: they rotate a few pairs at the rounding level
+constexpr int JS_FLAG_SWEEPS = 2;
 constexpr int JS_THREADS = 512;
 
 bool jacobi_precondition_ok(int N) { return N >= JS_MIN_N && N <= JS_MAX_N && tc_fp64_ok(N); }
@@ -62,32 +71,24 @@ __device__ __forceinline__ double js_scale(const double2 *R)
     return e > 0 && e < 0x7FF ? ldexp(1.0, 1022 - e) : 1.0;
 }
 
-// Y (2 N x N FP32) = R's first N rows, scaled, over the identity
+// Y (N x N FP32) = R's first N rows, scaled
 __global__ void js_init_kernel(int ld, int N, const double2 *__restrict__ R, float2 *__restrict__ Y)
 {
     const int f = blockIdx.y;
     R += (size_t)f * ld * N;
-    Y += (size_t)f * 2 * N * N;
+    Y += (size_t)f * N * N;
     const double sc = js_scale(R);
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N * N; e += gridDim.x * blockDim.x) {
         const int c = e / N, r = e - c * N;
         const double2 v = R[r + (size_t)c * ld];
-        Y[r + (size_t)c * 2 * N] = make_float2((float)(v.x * sc), (float)(v.y * sc));
-        Y[N + r + (size_t)c * 2 * N] = make_float2(r == c ? 1.f : 0.f, 0.f);
+        Y[e] = make_float2((float)(v.x * sc), (float)(v.y * sc));
     }
 }
 
-// J (N x N FP64) = the accumulated rotations
-__global__ void js_rotations_kernel(int N, const float2 *__restrict__ Y, double2 *__restrict__ J)
+__global__ void js_widen_kernel(size_t count, const float2 *__restrict__ X, double2 *__restrict__ J)
 {
-    const int f = blockIdx.y;
-    Y += (size_t)f * 2 * N * N;
-    J += (size_t)f * N * N;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N * N; e += gridDim.x * blockDim.x) {
-        const int c = e / N, r = e - c * N;
-        const float2 v = Y[N + r + (size_t)c * 2 * N];
-        J[e] = make_double2((double)v.x, (double)v.y);
-    }
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < count; e += (size_t)gridDim.x * blockDim.x)
+        J[e] = make_double2((double)X[e].x, (double)X[e].y);
 }
 
 __device__ __forceinline__ double js_block_sum(double v, double *red)
@@ -142,40 +143,84 @@ __device__ __forceinline__ double js_rcp(double x)
     return r;
 }
 
-// G = M^H M -> T in place: T_ij = G_ij / (G_jj - G_ii) where |T_ij| <= theta, the
-// largest of 5e-2, 1e-2 .. 1e-7 that keeps |T|_F <= limit, else 0.  Exactly
-// anti-Hermitian: each pair is computed once.  One CTA per bin.
+// Columns scaled by powers of two to a largest component in [1, 2): X <- X D^-1,
+// E (+)= the exponents of D.  A warp per column.
+__global__ void js_normalize_kernel(int N, int first, double2 *__restrict__ X, int *__restrict__ E)
+{
+    const int f = blockIdx.y, lane = threadIdx.x & 31, j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (j >= N) return;
+    X += ((size_t)f * N + j) * N;
+    int e = 0;   // biased exponent of the largest component
+    for (int i = lane; i < N; i += 32) {
+        const double2 v = X[i];
+        const int ex = (int)((__double_as_longlong(v.x) >> 52) & 0x7FF), ey = (int)((__double_as_longlong(v.y) >> 52) & 0x7FF);
+        e = max(e, max(ex, ey));
+    }
+    for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    e = e == 0 || e == 0x7FF ? 0 : min(max(e - 1023, -1000), 1000);   // zero and non-finite columns stay
+    const double sc = ldexp(1.0, -e);
+    for (int i = lane; i < N; i += 32) X[i] = zscale(X[i], sc);
+    if (lane == 0) E[(size_t)f * N + j] = (first ? 0 : E[(size_t)f * N + j]) + e;
+}
+
+// X <- X D
+__global__ void js_unscale_kernel(int N, double2 *__restrict__ X, const int *__restrict__ E)
+{
+    const int f = blockIdx.y, lane = threadIdx.x & 31, j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (j >= N) return;
+    X += ((size_t)f * N + j) * N;
+    const double sc = ldexp(1.0, E[(size_t)f * N + j]);
+    for (int i = lane; i < N; i += 32) X[i] = zscale(X[i], sc);
+}
+
+// G = (M D^-1)^H (M D^-1) -> D T D^-1 in place: T_ij = (D G D)_ij / ((D G D)_jj -
+// (D G D)_ii) where |T_ij| <= theta, the largest of 5e-2, 1e-2 .. 1e-7 that keeps
+// |T|_F <= limit, else 0.  T is exactly anti-Hermitian: each pair is computed
+// once.  One CTA per bin.
 constexpr int JS_NT = 7;
 __host__ __device__ constexpr float js_theta2(int q)
 {
     return q == 0 ? 2.5e-3f : q == 1 ? 1e-4f : q == 2 ? 1e-6f : q == 3 ? 1e-8f : q == 4 ? 1e-10f : q == 5 ? 1e-12f : 1e-14f;
 }
 
-__global__ void __launch_bounds__(JS_THREADS) js_rotation_kernel(int N, double limit, double2 *G)
+__global__ void __launch_bounds__(JS_THREADS) js_rotation_kernel(int N, float limit, const int *E, double2 *G)
 {
-    extern __shared__ double js_g[];   // N: diag(G)
-    __shared__ double red[JS_THREADS / 32];
+    extern __shared__ double js_g[];   // N: diag(D G D); N: d; N: 1 / d, relative to the largest d
+    double *w = js_g + N, *wi = w + N;
+    __shared__ float red[JS_NT][JS_THREADS / 32];
+    __shared__ int s_emax;
     const int f = blockIdx.x;
     G += (size_t)f * N * N;
-    for (int i = threadIdx.x; i < N; i += JS_THREADS) js_g[i] = G[i + (size_t)i * N].x;
+    E += (size_t)f * N;
+    if (threadIdx.x == 0) s_emax = -4000;
     __syncthreads();
-    double s[JS_NT];
+    for (int i = threadIdx.x; i < N; i += JS_THREADS) atomicMax(&s_emax, E[i]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < N; i += JS_THREADS) {
+        w[i] = ldexp(1.0, E[i] - s_emax);
+        wi[i] = ldexp(1.0, s_emax - E[i]);
+        js_g[i] = G[i + (size_t)i * N].x * w[i] * w[i];
+    }
+    __syncthreads();
+    // |T_ij|^2 and its sums in FP32: they only choose theta (below 1e-19 they
+    // underflow, and count as nothing)
+    auto size2 = [](double2 t) { const float x = (float)t.x, y = (float)t.y; return x * x + y * y; };
+    float s[JS_NT];
 #pragma unroll
-    for (int q = 0; q < JS_NT; ++q) s[q] = 0.0;
+    for (int q = 0; q < JS_NT; ++q) s[q] = 0.f;
     for (int e = threadIdx.x; e < N * N; e += JS_THREADS) {
         const int j = e / N, i = e - j * N;
         if (i >= j) continue;
         const double2 g = G[e];
-        const double q = js_rcp(js_g[j] - js_g[i]);
+        const double q = js_rcp(js_g[j] - js_g[i]) * w[i] * w[j];
         const double2 t = make_double2(g.x * q, g.y * q);
-        const double d = zabs2(t);
-        const float m = (float)d;
+        const float m = size2(t);
         // a zero gap, a NaN and an infinity fail every comparison
         if (m <= js_theta2(0)) {
             G[e] = t;
 #pragma unroll
             for (int k = 0; k < JS_NT; ++k)
-                if (m <= js_theta2(k)) s[k] += d;
+                if (m <= js_theta2(k)) s[k] += m;
         } else {
             G[e] = make_double2(0.0, 0.0);
         }
@@ -183,8 +228,16 @@ __global__ void __launch_bounds__(JS_THREADS) js_rotation_kernel(int N, double l
     float keep = -1.f;   // largest |T_ij|^2 kept
 #pragma unroll
     for (int q = 0; q < JS_NT; ++q) {
-        const double t = 2.0 * js_block_sum(s[q], red);
-        if (keep < 0.f && t <= limit * limit) keep = js_theta2(q);
+        float v = s[q];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < JS_NT; ++q) {
+        float t = 0.f;
+        for (int v = 0; v < JS_THREADS / 32; ++v) t += red[q][v];
+        if (keep < 0.f && 2.f * t <= limit * limit) keep = js_theta2(q);
     }
     for (int e = threadIdx.x; e < N * N; e += JS_THREADS) {
         const int j = e / N, i = e - j * N;
@@ -194,9 +247,10 @@ __global__ void __launch_bounds__(JS_THREADS) js_rotation_kernel(int N, double l
             continue;
         }
         double2 t = G[e];
-        if (!((float)zabs2(t) <= keep)) t = make_double2(0.0, 0.0);
-        G[e] = t;
-        G[j + (size_t)i * N] = make_double2(-t.x, t.y);
+        if (!(size2(t) <= keep)) t = make_double2(0.0, 0.0);
+        const double u = w[i] * wi[j], v = w[j] * wi[i];
+        G[e] = zscale(t, u);
+        G[j + (size_t)i * N] = make_double2(-t.x * v, t.y * v);
     }
 }
 
@@ -226,7 +280,8 @@ __global__ void __launch_bounds__(JS_THREADS) js_flags_kernel(int N, double tol,
 size_t jacobi_precondition_ws_bytes(int N, int batch)
 {
     const size_t nn = (size_t)N * N * batch;
-    return 5 * ws_round(16 * nn) + ws_round(nn) + zgemm_tc_ws_bytes(N, N, N, batch) + 2048;
+    const size_t prod = zgemm_tc_ws_bytes(N, N, N, batch), start = jacobi_start_ws_bytes(N, JS_FP32_SWEEPS, batch);
+    return 5 * ws_round(16 * nn) + ws_round(nn) + ws_round(4 * (size_t)N * batch) + (prod > start ? prod : start) + 2048;
 }
 
 int jacobi_precondition_batched(ia_context *ctx, int N, const double2 *R, int ldr, double2 *M, int *done, int batch,
@@ -238,11 +293,12 @@ int jacobi_precondition_batched(ia_context *ctx, int N, const double2 *R, int ld
     double2 *J = cur.take<double2>(count), *D = cur.take<double2>(count), *Q = cur.take<double2>(count),
             *P = cur.take<double2>(count);
     unsigned char *flags = cur.take<unsigned char>(count);
+    int *E = cur.take<int>((size_t)N * batch);
     if (cur.off > cur.cap) return IA_ERR_ALLOC;
     int st;
     int blocks = (int)((nn + 255) / 256);
     if (blocks > 64) blocks = 64;
-    const dim3 grid(blocks, batch);
+    const dim3 grid(blocks, batch), cols((N + 7) / 8, batch);
     const size_t want = (count + 255) / 256, cap = (size_t)ctx->sm_count * 8;
     const int flat = (int)(want < cap ? want : cap);
     // C = op(A) B + beta C, N x N
@@ -257,8 +313,8 @@ int jacobi_precondition_batched(ia_context *ctx, int N, const double2 *R, int ld
     };
     js_init_kernel<<<grid, 256, 0, ctx->stream>>>(ldr, N, R, Y);
     IA_LAUNCH_CHECK(ctx);
-    if ((st = jacobi_start_batched(ctx, N, Y, batch, JS_FP32_SWEEPS))) return st;
-    js_rotations_kernel<<<grid, 256, 0, ctx->stream>>>(N, Y, J);
+    if ((st = jacobi_start_batched(ctx, N, Y, Y + count, batch, JS_FP32_SWEEPS, cur))) return st;
+    js_widen_kernel<<<flat, 256, 0, ctx->stream>>>(count, Y + count, J);
     IA_LAUNCH_CHECK(ctx);
     // J to its polar factor (M holds the product's second operand), M = R J
     if ((st = prod(OP_C, J, N, J, 0.0, D))) return st;
@@ -271,13 +327,20 @@ int jacobi_precondition_batched(ia_context *ctx, int N, const double2 *R, int ld
     if ((st = prod(OP_N, J, N, P, 1.0, J))) return st;
     if ((st = prod(OP_N, R, ldr, J, 0.0, M))) return st;
     const size_t nsm = sizeof(double) * (size_t)N;
+    // T of M, on M with its columns scaled
+    auto rotation = [&](float limit, int first) -> int {
+        js_normalize_kernel<<<cols, 256, 0, ctx->stream>>>(N, first, M, E);
+        IA_LAUNCH_CHECK(ctx);
+        if ((st = prod(OP_C, M, N, M, 0.0, D))) return st;
+        js_rotation_kernel<<<batch, JS_THREADS, 3 * nsm, ctx->stream>>>(N, limit, E, D);
+        IA_LAUNCH_CHECK(ctx);
+        return IA_OK;
+    };
     // first step: p = (I - T^2)^(-1/2) - I to (T^2)^5, P = T + p + T p
-    if ((st = prod(OP_C, M, N, M, 0.0, D))) return st;
-    js_rotation_kernel<<<batch, JS_THREADS, nsm, ctx->stream>>>(N, JS_MAX_T1, D);
-    IA_LAUNCH_CHECK(ctx);
+    if ((st = rotation(JS_MAX_T1, 1))) return st;
     {
         // D = T, Q = T^2, J = T^4, P = T^6, then P = 5/16 Q + 35/128 J + 63/256 P
-        double2 *T = D, *S = reinterpret_cast<double2 *>(Y);   // (Y's 2 N^2 FP32 pairs: N^2 FP64 ones)
+        double2 *T = D, *S = reinterpret_cast<double2 *>(Y);   // (Y and J in FP32: N^2 FP64 pairs)
         if ((st = prod(OP_N, T, N, T, 0.0, Q))) return st;
         if ((st = prod(OP_N, Q, N, Q, 0.0, J))) return st;
         if ((st = prod(OP_N, Q, N, J, 0.0, P))) return st;
@@ -290,21 +353,24 @@ int jacobi_precondition_batched(ia_context *ctx, int N, const double2 *R, int ld
         if ((st = prod(OP_N, M, N, P, 1.0, M))) return st;
     }
     // second step: P = T + T^2 / 2 + T^2 (T / 2 + 3 T^2 / 8)
-    if ((st = prod(OP_C, M, N, M, 0.0, D))) return st;
-    js_rotation_kernel<<<batch, JS_THREADS, nsm, ctx->stream>>>(N, JS_MAX_T2, D);
-    IA_LAUNCH_CHECK(ctx);
+    if ((st = rotation(JS_MAX_T2, 0))) return st;
     if ((st = prod(OP_N, D, N, D, 0.0, Q))) return st;
     if ((st = combine(0.5, D, 0.375, Q, J))) return st;
     if ((st = combine(1.0, D, 0.5, Q, P))) return st;
     if ((st = prod(OP_N, Q, N, J, 1.0, P))) return st;
     if ((st = prod(OP_N, M, N, P, 1.0, M))) return st;
+    // third step: P = T + T^2 / 2
+    if ((st = rotation(JS_MAX_T3, 0))) return st;
+    if ((st = prod(OP_N, D, N, D, 0.0, Q))) return st;
+    if ((st = combine(1.0, D, 0.5, Q, P))) return st;
+    if ((st = prod(OP_N, M, N, P, 1.0, M))) return st;
+    js_unscale_kernel<<<cols, 256, 0, ctx->stream>>>(N, M, E);
+    IA_LAUNCH_CHECK(ctx);
     // sweeps over the pairs above the test
-    const int sweeps = N > JS_SMALL_N ? JS_FLAG_SWEEPS : JS_FLAG_SWEEPS_SMALL;
-    for (int it = 0;; ++it) {
+    for (int it = 0; it < JS_FLAG_SWEEPS; ++it) {
         if ((st = prod(OP_C, M, N, M, 0.0, D))) return st;
         js_flags_kernel<<<batch, JS_THREADS, nsm, ctx->stream>>>(N, jacobi_tol_fp64(N), D, flags, done);
         IA_LAUNCH_CHECK(ctx);
-        if (it == sweeps) break;
         if ((st = jacobi_flagged_batched(ctx, N, M, batch, done, flags))) return st;
     }
     return IA_OK;

@@ -15,6 +15,7 @@
 // along (the pipeline keeps conj(b)^T there, so U^H b falls out of the
 // rotations without forming U).
 #include <cooperative_groups.h>
+#include <algorithm>
 #include "ia_common.cuh"
 #include "ia_internal.h"
 
@@ -78,6 +79,42 @@ __device__ __forceinline__ bool jacobi_rotation_start(float a, float b, float2 g
     c = 1 / sqrtf(1 + t * t);
     const float s = t * c;
     sp = make_float2(s * (x / h), s * (y / h));
+    return true;
+}
+
+// jacobi_rotation for the flagged sweeps: the same test and rotation, with c to
+// FP64 rounding and c, s on the unit circle to it, and the angle to ~2^-40, by
+// Newton steps from the 20-bit reciprocal and reciprocal square root.  A pair of
+// a sparse sweep waits on this chain: ~30 dependent FP64 instructions instead of
+// ~200 (eight IEEE divisions and square roots in a row, 8 us).  a, b and g are
+// scaled by a power of two, which leaves the squares of squares in range.
+__device__ __forceinline__ bool jacobi_rotation_flagged(double a, double b, double2 g, double tol, double &c, double2 &sp)
+{
+    const double m = fmax(a, b);
+    const int e = (int)((__double_as_longlong(m) >> 52) & 0x7FF);
+    if (e < 64 || e >= 0x7FF) return false;   // |y| < 1e-144: zero, or not a number
+    const double sc = __longlong_as_double((long long)(2046 - e) << 52);
+    a *= sc;
+    b *= sc;
+    g.x *= sc;
+    g.y *= sc;
+    const double x = fma(g.x, g.x, g.y * g.y);
+    if (!(x > tol * tol * a * b) || x == 0.0) return false;
+    // t = tau |g|, tau = sign(d) 2 / (|d| + sqrt(d^2 + 4 |g|^2)), d = b - a
+    const double d = b - a, y = fma(d, d, 4.0 * x);
+    double r, q;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
+    r = r * fma(-0.5 * y * r, r, 1.5);
+    const double den = fma(y, r, fabs(d));
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(q) : "d"(den));
+    q = q * fma(-den, q, 2.0);
+    const double tau = copysign(2.0 * q, d);
+    const double w = fma(tau * tau, x, 1.0);
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(w));
+    r = r * fma(-0.5 * w * r, r, 1.5);
+    c = fma(0.5 * r, fma(-w * r, r, 1.0), r);
+    const double s = c * tau;
+    sp = make_double2(s * g.x, s * g.y);
     return true;
 }
 
@@ -399,17 +436,19 @@ __global__ void __launch_bounds__(sizeof(T) <= 8 ? 1024 : 512)
 // largest coupling are combined over the cluster), so the factors are
 // bitwise the same.
 //
-// MODE: JC_PLAIN; JC_START, the FP32 start of an FP64 iteration; JC_FLAGGED, one
-// FP64 sweep over the pairs (i, j), i < j, whose byte flags[i + j N] is set
+// MODE: JC_PLAIN; JC_START, the FP32 start of an FP64 iteration, each pair's
+// rotation written to rec[sweep][round][slot] (c, s, rotated or not) and the
+// number of recorded sweeps to sweeps[f]; JC_FLAGGED, one FP64 sweep over the pairs (i, j), i < j, whose byte flags[i + j N] is set
 // (the others were tested elsewhere): unflagged pairs cost nothing but the
 // round's barrier.  CSC: the cluster size when fixed (0: read at run time).
 // Bins with skip[f] set are left alone.
 enum { JC_PLAIN = 0, JC_START = 1, JC_FLAGGED = 2 };
 
 template <class T, int KPL = 8, int MODE = JC_PLAIN, int CSC = 0>
-__global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
+__global__ void __launch_bounds__(KPL <= 8 ? 512 : KPL <= 16 ? 256 : 288)
     jacobi_cluster_kernel(int M, int Mdot, int N, int N2, T *Yg, long long sY, int max_sweeps,
-                          typename ctraits<T>::R tol, int *info, const int *skip, const unsigned char *flags)
+                          typename ctraits<T>::R tol, int *info, const int *skip, const unsigned char *flags,
+                          float4 *rec, int *sweeps)
 {
     constexpr bool START = MODE == JC_START;
     typedef typename ctraits<T>::R R;
@@ -425,10 +464,21 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
     T *fixc = lo + (size_t)RING * M;         // M: column N2 - 1 (CTA 0)
     __shared__ int s_rot[2];
     __shared__ unsigned s_rel[2];
+    // FP64: norms and products of the CTA's pairs, then their rotations (c = 0: none)
+    constexpr bool FP64 = sizeof(R) == 8;
+    __shared__ double2 s_ab[FP64 ? 32 : 1], s_g[FP64 ? 32 : 1];
     Yg += f * sY;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int half = lane >> 4, hl = lane & 15, hw = 2 * wid + half;
+    // lanes per pair: a half-warp; a warp over the few pairs of a flagged sweep,
+    // whose FP64 pipe waits on one pair's chain
+    constexpr int LN = MODE == JC_FLAGGED ? 32 : 16;
+    const int half = LN == 32 ? 0 : lane >> 4, hl = lane & (LN - 1), hw = LN == 32 ? wid : 2 * wid + half;
+    const int nhw = LN == 32 ? nw : 2 * nw;
     const unsigned mask = half ? 0xffff0000u : 0x0000ffffu;
+    auto pair_sum = [&](R v) -> R {
+        if constexpr (LN == 32) return warp_sum(v);
+        else return half_sum<T>(v, mask);
+    };
     const T zero = ctraits<T>::make(0, 0);
     // columns of slot k at round r (k0 = 0 .. NP - 1)
     auto col_up = [&](int k, int r) { int c = r + k; return c >= NR ? c - NR : c; };
@@ -465,15 +515,23 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
     }
     cluster.sync();
     int r = 0, t = 0, par = 0, sweep = 0;   // round mod NR, round mod RING
+    int nrec = 0;                           // sweeps with rotations
     for (; sweep < max_sweeps; ++sweep) {
         int rot_local = 0;
         float relmax = 0.f;
         for (int round = 0; round < NR; ++round) {
             const int tn = t + 1 == RING ? 0 : t + 1;
-            for (int s = hw; s < P; s += 2 * nw) {
+            // FP64: a slot per half-warp (warp)
+            bool live = true;   // some pair of this CTA is tested in this round
+            if constexpr (MODE == JC_FLAGGED) {
+                live = false;
+                for (int w = 0; w < MW; ++w) live |= fmask[r * MW + w] != 0u;
+            }
+            for (int s = hw; FP64 ? s == hw : s < P; s += nhw) {
                 const int k = k0 + s;
-                const bool flagged = MODE != JC_FLAGGED || (fmask[r * MW + s / 32] >> (s & 31) & 1u);
-                if (MODE == JC_FLAGGED && !flagged && s != 0 && s != P - 1) continue;
+                const bool flagged = s < P && (MODE != JC_FLAGGED || (fmask[r * MW + s / 32] >> (s & 31) & 1u));
+                // a flagged sweep's other slots stay, but for the edges that move on
+                const bool work = s < P && (flagged || s == 0 || s == P - 1);
                 const int cu = col_up(k, r), cl = col_lo(k, r);
                 int eu = s + t;
                 if (eu >= RING) eu -= RING;
@@ -484,44 +542,85 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
                 T *yi = uf ? pu : pl, *yj = uf ? pl : pu;
                 const int j = uf ? cl : cu;
                 T ui[KPL], uj[KPL];
-#pragma unroll
-                for (int q = 0; q < KPL; ++q) {
-                    const int rr = hl + 16 * q;
-                    ui[q] = rr < M ? yi[rr] : zero;
-                    uj[q] = rr < M ? yj[rr] : zero;
-                }
-                if (j < N && flagged) {
-                    R a = 0, b = 0, c;
-                    T g = zero, sp;
+                if (work) {
 #pragma unroll
                     for (int q = 0; q < KPL; ++q) {
-                        if (hl + 16 * q < Mdot) {
+                        const int rr = hl + LN * q;
+                        ui[q] = rr < M ? yi[rr] : zero;
+                        uj[q] = rr < M ? yj[rr] : zero;
+                    }
+                }
+                bool rotate = false;
+                R c = 1;
+                T sp = zero;
+                const bool test = j < N && flagged;
+                if (test) {
+                    R a = 0, b = 0;
+                    T g = zero;
+#pragma unroll
+                    for (int q = 0; q < KPL; ++q) {
+                        if (hl + LN * q < Mdot) {
                             a += zabs2(ui[q]);
                             b += zabs2(uj[q]);
                             zcfma(g, ui[q], uj[q]);
                         }
                     }
-                    a = half_sum<T>(a, mask);
-                    b = half_sum<T>(b, mask);
-                    g.x = half_sum<T>(g.x, mask);
-                    g.y = half_sum<T>(g.y, mask);
-                    R rel = 0;
-                    bool rotate;
-                    if constexpr (START) rotate = jacobi_rotation_start(a, b, g, tol, c, sp, rel);
-                    else rotate = jacobi_rotation(a, b, g, tol, c, sp, sizeof(R) == 4 ? &rel : nullptr);
-                    if (rotate) {
-                        relmax = fmaxf(relmax, (float)rel);
-#pragma unroll
-                        for (int q = 0; q < KPL; ++q) {
-                            const int rr = hl + 16 * q;
-                            if (rr < M) {
-                                rotate_pair(ui[q], uj[q], c, sp);
-                                yi[rr] = ui[q];
-                                yj[rr] = uj[q];
-                            }
+                    a = pair_sum(a);
+                    b = pair_sum(b);
+                    g.x = pair_sum(g.x);
+                    g.y = pair_sum(g.y);
+                    if constexpr (FP64) {
+                        if (hl == 0) {
+                            s_ab[s] = make_double2(a, b);
+                            s_g[s] = make_double2(g.x, g.y);
                         }
-                        rot_local++;
+                    } else {
+                        R rel = 0;
+                        if constexpr (START) rotate = jacobi_rotation_start(a, b, g, tol, c, sp, rel);
+                        else rotate = jacobi_rotation(a, b, g, tol, c, sp, &rel);
+                        if (rotate) relmax = fmaxf(relmax, (float)rel);
                     }
+                }
+                if constexpr (FP64) {
+                    // the CTA's rotations at once, a lane each: the ~100 FP64
+                    // instructions of one cost the SM's pipe the same for a warp
+                    if (live) {
+                        if (s < P && hl == 0 && !test) s_ab[s].x = -1.0;
+                        __syncthreads();
+                        if (wid == 0 && lane < P && !(s_ab[lane].x < 0.0)) {
+                            R c2;
+                            T sp2;
+                            const R a2 = s_ab[lane].x, b2 = s_ab[lane].y;
+                            const T g2 = ctraits<T>::make(s_g[lane].x, s_g[lane].y);
+                            bool rot;
+                            if constexpr (MODE == JC_FLAGGED) rot = jacobi_rotation_flagged(a2, b2, g2, tol, c2, sp2);
+                            else rot = jacobi_rotation(a2, b2, g2, tol, c2, sp2);
+                            s_ab[lane].x = rot ? c2 : 0.0;
+                            if (rot) s_g[lane] = make_double2(sp2.x, sp2.y);
+                        }
+                        __syncthreads();
+                        if (test) {
+                            c = (R)s_ab[s].x;
+                            rotate = c != 0;
+                            sp = ctraits<T>::make(s_g[s].x, s_g[s].y);
+                        }
+                    }
+                }
+                if (rotate) {
+#pragma unroll
+                    for (int q = 0; q < KPL; ++q) {
+                        const int rr = hl + LN * q;
+                        if (rr < M) {
+                            rotate_pair(ui[q], uj[q], c, sp);
+                            yi[rr] = ui[q];
+                            yj[rr] = uj[q];
+                        }
+                    }
+                    rot_local++;
+                }
+                if constexpr (START) {
+                    if (hl == 0)
+                        rec[(((size_t)f * max_sweeps + sweep) * NR + round) * (N2 / 2) + k] = make_float4(c, sp.x, sp.y, rotate ? 1.f : 0.f);
                 }
                 // the columns that leave this CTA's rings for the next round
                 const T *vu = uf ? ui : uj, *vl = uf ? uj : ui;   // registers of the upper / lower column
@@ -538,7 +637,7 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
                     }
 #pragma unroll
                     for (int q = 0; q < KPL; ++q)
-                        if (hl + 16 * q < M) dst[hl + 16 * q] = vu[q];
+                        if (hl + LN * q < M) dst[hl + LN * q] = vu[q];
                 }
                 if (s == P - 1) {
                     T *dst;
@@ -553,7 +652,7 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
                     }
 #pragma unroll
                     for (int q = 0; q < KPL; ++q)
-                        if (hl + 16 * q < M) dst[hl + 16 * q] = vl[q];
+                        if (hl + LN * q < M) dst[hl + LN * q] = vl[q];
                 }
             }
             cluster.sync();
@@ -578,6 +677,7 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
         }
         par ^= 1;
         if (total == 0) break;
+        ++nrec;
         if (sizeof(R) == 4 && __uint_as_float(mr) < 0.5f * sqrtf((float)tol)) break;
     }
     cluster.sync();   // every CTA has read the others' counters
@@ -595,7 +695,96 @@ __global__ void __launch_bounds__(KPL <= 8 ? 512 : 256)
             if (cl < N && IA_IDX_OK((long long)cl * M + i, yext)) Yg[(size_t)cl * M + i] = pl[i];
         }
     }
-    if (rank == 0 && threadIdx.x == 0 && sweep >= max_sweeps && info) atomicOr(&info[f], IA_INFO_NOCONV);
+    if (rank == 0 && threadIdx.x == 0) {
+        if (START) sweeps[f] = nrec;
+        else if (MODE == JC_FLAGGED) {
+            if (nrec == 0) sweeps[f] = 1;   // no pair, flagged or not, above the test
+        } else if (sweep >= max_sweeps && info) atomicOr(&info[f], IA_INFO_NOCONV);
+    }
+}
+
+// J (N x N) = the product of the recorded rotations.  A row of J only meets
+// itself: a warp carries JA_ROWS rows in shared memory through all the sweeps,
+// lanes over the pairs, with no barrier but its own; reading and writing the rows
+// (32 bytes per rotated pair and row) bounds it at many bins; at few, a round's
+// latency, so the records are read eight loads ahead.  Carried through the Jacobi as
+// further rows of its columns instead, J doubled the shared memory and the time
+// of every round there (order-15 HELS, 64 bins: 43.9 ms, against 13.1 and 4.4 ms).
+constexpr int JA_WARPS = 8, JA_ROWS = 4, JA_MAX_CHUNKS = 4;
+
+template <int CHUNKS>   // of 32 pairs
+__global__ void __launch_bounds__(32 * JA_WARPS) jacobi_apply_kernel(int N, int N2, int max_sweeps,
+                                                                     const float4 *__restrict__ rec,
+                                                                     const int *__restrict__ sweeps,
+                                                                     float2 *__restrict__ J)
+{
+    extern __shared__ float2 ja_rows[];   // JA_WARPS JA_ROWS x N2
+    constexpr int ROWS = JA_WARPS * JA_ROWS;
+    const int f = blockIdx.y, r0 = blockIdx.x * ROWS;
+    const int NR = N2 - 1, NP = N2 / 2, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    J += (size_t)f * N * N;
+    rec += (size_t)f * max_sweeps * NR * NP;
+    const int total = sweeps[f] * NR;
+    for (int e = threadIdx.x; e < ROWS * N2; e += blockDim.x) {
+        const int c = e % N2, r = e / N2;
+        ja_rows[e] = make_float2(r0 + r == c ? 1.f : 0.f, 0.f);
+    }
+    __syncthreads();
+    float2 *row = ja_rows + (size_t)wid * JA_ROWS * N2;
+    constexpr int AHEAD = 8 / CHUNKS;
+    float4 nx[AHEAD][CHUNKS];
+    auto fetch = [&](float4 *q, int g) {
+        if (g < total) {
+#pragma unroll
+            for (int h = 0; h < CHUNKS; ++h)
+                if (lane + 32 * h < NP) q[h] = rec[(size_t)g * NP + lane + 32 * h];
+        }
+    };
+#pragma unroll
+    for (int a = 0; a < AHEAD; ++a) fetch(nx[a], a);
+    int r = 0;   // round of the sweep
+    for (int g0 = 0; g0 < total; g0 += AHEAD) {
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a) {
+            if (g0 + a >= total) break;
+            float4 q[CHUNKS];
+#pragma unroll
+            for (int h = 0; h < CHUNKS; ++h) q[h] = nx[a][h];
+            fetch(nx[a], g0 + a + AHEAD);
+#pragma unroll
+            for (int h = 0; h < CHUNKS; ++h) {
+                const int k = lane + 32 * h;
+                if (k < NP && q[h].w != 0.f) {
+                    // slot k's columns in round r (jacobi_cluster_kernel), both below N
+                    int cu = r + k, cl = r - k;
+                    if (cu >= NR) cu -= NR;
+                    if (cl < 0) cl += NR;
+                    if (k == 0) cl = N2 - 1;
+                    const int i = cu < cl ? cu : cl, j = cu < cl ? cl : cu;
+                    const float2 sp = make_float2(q[h].y, q[h].z);
+                    float2 u[JA_ROWS], v[JA_ROWS];
+#pragma unroll
+                    for (int w = 0; w < JA_ROWS; ++w) {
+                        u[w] = row[w * N2 + i];
+                        v[w] = row[w * N2 + j];
+                    }
+#pragma unroll
+                    for (int w = 0; w < JA_ROWS; ++w) {
+                        rotate_pair(u[w], v[w], q[h].x, sp);
+                        row[w * N2 + i] = u[w];
+                        row[w * N2 + j] = v[w];
+                    }
+                }
+            }
+            __syncwarp();
+            r = r + 1 == NR ? 0 : r + 1;
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < ROWS * N; e += blockDim.x) {
+        const int c = e / ROWS, r = e - c * ROWS;
+        if (r0 + r < N) J[r0 + r + (size_t)c * N] = ja_rows[r * N2 + c];
+    }
 }
 
 template <class T>
@@ -845,7 +1034,7 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
                 IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)lc.dynamicSmemBytes));
             IA_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, M, Mdot, N, N + (N & 1), Y, sY, max_sweeps, tol, info, skip,
-                                           (const unsigned char *)nullptr));
+                                           (const unsigned char *)nullptr, (float4 *)nullptr, (int *)nullptr));
             IA_LAUNCH_CHECK(ctx);
             return IA_OK;
         }
@@ -892,14 +1081,18 @@ template int jacobi_rows_batched<float2>(ia_context *, int, int, int, float2 *, 
                                          const int *);
 
 template <class T, int MODE>
-static int jc_launch(ia_context *ctx, int M, int Mdot, int N, T *Y, int batch, int max_sweeps,
-                     typename ctraits<T>::R tol, const int *skip, const unsigned char *flags)
+static int jc_launch(ia_context *ctx, int N, T *Y, int batch, int max_sweeps, typename ctraits<T>::R tol,
+                     const int *skip, const unsigned char *flags, float4 *rec, int *sweeps)
 {
-    // clusters of 8 whatever the batch (a round is latency-bound), N padded to
-    // whole slots
-    constexpr int cs = 8;
-    const int N2 = (N + 15) / 16 * 16, P = N2 / 2 / cs;
-    if (P < 2 || M > (sizeof(T) == sizeof(float2) ? 512 : 272)) return IA_ERR_ARG;
+    // N padded to whole slots of clusters of 8 whatever the batch: a round is
+    // latency-bound.  FP32: of 4 where a CTA's share is small or the clusters
+    // would queue for the SMs (64 columns, 1 bin 0.61 against 0.63 ms, 150 bins
+    // 0.96 against 1.47; 160 columns, 48 bins 5.97 against 6.97; but 96 columns, 1
+    // bin 1.04 against 0.92, 180 columns, 20 bins 4.36 against 3.07)
+    const int N2 = jacobi_slots(N);
+    const int cs = sizeof(T) == sizeof(float2) && N <= 192 && (N <= 64 || 8 * batch > 2 * ctx->sm_count) ? 4 : 8;
+    const int P = N2 / 2 / cs;
+    if (P < 2 || N > 256) return IA_ERR_ARG;
     cudaLaunchConfig_t lc = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -908,40 +1101,77 @@ static int jc_launch(ia_context *ctx, int M, int Mdot, int N, T *Y, int batch, i
     lc.attrs = at;
     lc.numAttrs = 1;
     lc.stream = ctx->stream;
-    constexpr bool F32 = sizeof(T) == sizeof(float2);
-    auto kern = jacobi_cluster_kernel<T, 8, MODE>;
-    if (M > 128) kern = F32 ? (M <= 256 ? jacobi_cluster_kernel<T, F32 ? 16 : 12, MODE>
-                                        : jacobi_cluster_kernel<T, F32 ? 32 : 17, MODE>)
-                            : (M <= 192 ? jacobi_cluster_kernel<T, F32 ? 16 : 12, MODE>
-                                        : jacobi_cluster_kernel<T, F32 ? 32 : 17, MODE>);
+    constexpr int H = MODE == JC_FLAGGED ? 2 : 1;   // lanes per pair: 16 H
+    auto kern = N <= 128   ? jacobi_cluster_kernel<T, 8 / H, MODE>
+                : N <= 192 ? jacobi_cluster_kernel<T, 12 / H, MODE>
+                           : jacobi_cluster_kernel<T, 16 / H, MODE>;
     lc.gridDim = dim3((unsigned)(cs * batch));
-    lc.blockDim = dim3((unsigned)(32 * ((P + 1) / 2)));
-    lc.dynamicSmemBytes = sizeof(T) * ((size_t)2 * (P + 1) * M + M) +
+    // FP64: a warp per slot; FP32: half-warps, several slots each past 8 warps
+    const int nw = H == 2 ? P : std::min((P + 1) / 2, N <= 128 ? 16 : 8);
+    lc.blockDim = dim3((unsigned)(32 * nw));
+    lc.dynamicSmemBytes = sizeof(T) * ((size_t)2 * (P + 1) * N + N) +
                           (MODE == JC_FLAGGED ? sizeof(unsigned) * (size_t)N2 * ((P + 31) / 32) : 0);
     at[0].val.clusterDim.x = cs;
     if (lc.dynamicSmemBytes > 48 * 1024)
         IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lc.dynamicSmemBytes));
-    IA_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, M, Mdot, N, N2, Y, (long long)M * N, max_sweeps, tol, (int *)nullptr,
-                                   skip, flags));
+    IA_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, N, N, N, N2, Y, (long long)N * N, max_sweeps, tol, (int *)nullptr, skip,
+                                   flags, rec, sweeps));
     IA_LAUNCH_CHECK(ctx);
     return IA_OK;
 }
 
-// FP32 one-sided Jacobi of batch N x N matrices with the rotations accumulated:
-// Y (2 N x N) holds the matrix over the identity on entry, which the rotations
-// turn into J (only the first N rows enter the dot products).  A start for an
-// FP64 iteration: the sweep cap is not an error, and columns whose products
-// underflow stay as they are.
-int jacobi_start_batched(ia_context *ctx, int N, float2 *Y, int batch, int max_sweeps)
+// recorded rotations of one bin; held for at most JA_REC_BYTES of bins at once
+static size_t jacobi_record_bytes(int N, int max_sweeps)
 {
-    const float tol = (float)(sqrt((double)N) * 8.0 * 1.1920928955078125e-07);
-    return jc_launch<float2, JC_START>(ctx, 2 * N, N, N, Y, batch, max_sweeps, tol, nullptr, nullptr);
+    const size_t N2 = jacobi_slots(N);
+    return sizeof(float4) * (size_t)max_sweeps * (N2 - 1) * (N2 / 2);
+}
+constexpr size_t JA_REC_BYTES = size_t(2) << 30;
+
+size_t jacobi_start_ws_bytes(int N, int max_sweeps, int batch)
+{
+    const size_t one = jacobi_record_bytes(N, max_sweeps), all = one * batch;
+    return (all < JA_REC_BYTES ? all : JA_REC_BYTES > one ? JA_REC_BYTES : one) + ws_round(sizeof(int) * (size_t)batch) +
+           512;
 }
 
-// one FP64 sweep of Y (N x N) over the flagged pairs
-int jacobi_flagged_batched(ia_context *ctx, int N, double2 *Y, int batch, const int *skip, const unsigned char *flags)
+// FP32 one-sided Jacobi of batch N x N matrices Y, J (N x N) the product of the
+// rotations.  A start for an FP64 iteration: the sweep cap is not an error, and
+// columns whose products underflow stay as they are.  The rotations are recorded
+// and then applied to J, in groups of as many bins as the scratch holds.
+int jacobi_start_batched(ia_context *ctx, int N, float2 *Y, float2 *J, int batch, int max_sweeps, WsCursor cur)
 {
-    return jc_launch<double2, JC_FLAGGED>(ctx, N, N, N, Y, batch, 1, jacobi_tol_fp64(N), skip, flags);
+    const float tol = (float)(sqrt((double)N) * 8.0 * 1.1920928955078125e-07);
+    const int N2 = jacobi_slots(N), rows = JA_WARPS * JA_ROWS;
+    if (N2 / 2 > 32 * JA_MAX_CHUNKS) return IA_ERR_ARG;
+    int *sweeps = cur.take<int>((size_t)batch);
+    const size_t one = jacobi_record_bytes(N, max_sweeps), room = cur.cap > cur.off + 256 ? cur.cap - cur.off - 256 : 0;
+    if (room < one) return IA_ERR_ALLOC;
+    const int fit = room / one < (size_t)batch ? (int)(room / one) : batch;
+    float4 *rec = cur.take<float4>(one / sizeof(float4) * fit);
+    const size_t smem = sizeof(float2) * (size_t)rows * N2;
+    auto apply = N2 <= 64    ? jacobi_apply_kernel<1>
+                 : N2 <= 128 ? jacobi_apply_kernel<2>
+                             : jacobi_apply_kernel<JA_MAX_CHUNKS>;
+    IA_CUDA_TRY(cudaFuncSetAttribute(apply, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (int f0 = 0; f0 < batch; f0 += fit) {
+        const int nf = batch - f0 < fit ? batch - f0 : fit;
+        const size_t o = (size_t)f0 * N * N;
+        const int st = jc_launch<float2, JC_START>(ctx, N, Y + o, nf, max_sweeps, tol, nullptr, nullptr, rec,
+                                                   sweeps + f0);
+        if (st) return st;
+        apply<<<dim3((N + rows - 1) / rows, nf), 32 * JA_WARPS, smem, ctx->stream>>>(
+            N, N2, max_sweeps, rec, sweeps + f0, J + o);
+        IA_LAUNCH_CHECK(ctx);
+    }
+    return IA_OK;
+}
+
+// one FP64 sweep of Y (N x N) over the flagged pairs of the bins that are not
+// done; done where none of them rotates
+int jacobi_flagged_batched(ia_context *ctx, int N, double2 *Y, int batch, int *done, const unsigned char *flags)
+{
+    return jc_launch<double2, JC_FLAGGED>(ctx, N, Y, batch, 1, jacobi_tol_fp64(N), done, flags, nullptr, done);
 }
 
 int jacobi_svd_batched(ia_context *ctx, int M, int N, double2 *Y, double2 *V, int batch, int max_sweeps, int *info)
