@@ -108,12 +108,26 @@ __device__ __forceinline__ double fp64_scale(int e)
     return e == TC_EXP_NONFINITE ? __longlong_as_double(0x7FF8000000000000ll) : ldexp(1.0, e - 32);
 }
 
-// X = rint(v 2^q) for the real and imaginary parts (q: scale exponent)
+// X = rint(v 2^q) (to nearest, ties to even) for the real and imaginary parts (q:
+// scale exponent; |X| < 2^62), in integers: an FP64 instruction costs a warp 64
+// cycles of its SM sub-partition on GB300, an integer one 2
+__device__ __forceinline__ long long to_fixed(double v, int q)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const int ex = (int)(b >> 52) & 0x7FF;
+    unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | ((unsigned long long)(ex != 0) << 52);
+    const int sh = (ex ? ex : 1) - 1075 + q;
+    if (sh >= 0) m <<= sh < 10 ? sh : 10;
+    else {
+        const int r = -sh < 55 ? -sh : 55;   // m < 2^53: 0 at 55
+        m = (m + ((1ull << (r - 1)) - 1) + ((m >> r) & 1)) >> r;
+    }
+    return (long long)b < 0 ? -(long long)m : (long long)m;
+}
 __device__ __forceinline__ void to_fixed(const double2 &v, int q, long long &xr, long long &xi)
 {
-    const double sc = __longlong_as_double((long long)(q + 1023) << 52);
-    xr = __double2ll_rn(v.x * sc);
-    xi = __double2ll_rn(v.y * sc);
+    xr = to_fixed(v.x, q);
+    xi = to_fixed(v.y, q);
 }
 __device__ __forceinline__ void to_fixed(const float4 &v, int q, long long &xr, long long &xi)
 {
@@ -157,6 +171,33 @@ __device__ __forceinline__ void digits64(long long X, int (&d)[S])
 __device__ __forceinline__ __nv_bfloat162 bf2(int a, int b)
 {
     return __floats2bfloat162_rn((float)a, (float)b);
+}
+
+// The digits of digits64 as bit fields: X + sum_{i < S - 1} 31 64^i has the plain
+// base-64 digits d + 31 below the top one.  A pair of digits becomes BF16 without a
+// conversion: in [128, 256) BF16 is integers, so the field is OR-ed into 192 and
+// 192 + 31 subtracted.
+template <int S>
+__host__ __device__ constexpr long long digit_bias()
+{
+    long long b = 0;
+    for (int i = 0; i < S - 1; ++i) b = b * 64 + 31;
+    return b;
+}
+template <int S>
+__device__ __forceinline__ unsigned digit_pair(long long x, long long y, int s)
+{
+    unsigned u;
+    if (s > 0) {
+        const int sh = 6 * (S - 1 - s);
+        u = ((unsigned)(x >> sh) & 63u) | (((unsigned)(y >> sh) & 63u) << 16) | 0x43404340u;
+    } else {   // the top digit, -32 .. 32
+        const int a = (int)(x >> (6 * (S - 1))) + 31, b = (int)(y >> (6 * (S - 1))) + 31;
+        u = ((unsigned)(0x4340 + a) & 0xFFFFu) | ((unsigned)(0x4340 + b) << 16);
+    }
+    const __nv_bfloat162 off = __floats2bfloat162_rn(223.f, 223.f);
+    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&u), off);
+    return *reinterpret_cast<const unsigned *>(&v);
 }
 
 // One CTA per 32 rows of the operand view V (R x K, element (r, k)); V is
@@ -262,6 +303,9 @@ __global__ void __launch_bounds__(256) tc_slice_kernel(SliceOp<Src> op0, SliceOp
     }
 }
 
+// (Digits as bit fields, in place of conversions: 256 x 256 operands of 64 bins
+// 200 -> 120 us.)
+//
 // Single-pass form: SL1_RB rows of the view per CTA, their K values read from
 // global memory once into a shared-memory strip; warp w then takes row w: the
 // row maximum from the strip, then the digits of two complex values per lane
@@ -272,11 +316,6 @@ __global__ void __launch_bounds__(256) tc_slice_kernel(SliceOp<Src> op0, SliceOp
 constexpr int SL1_RB = 8, SL1_THREADS = 256, SL1_UNROLL = 4;
 
 __host__ __device__ constexpr int sl1_stride(int Kh) { return Kh + 1; }   // odd in 16-byte units: no bank conflicts
-
-__device__ __forceinline__ unsigned bf2_bits(__nv_bfloat162 v)
-{
-    return (unsigned)__bfloat16_as_ushort(v.x) | ((unsigned)__bfloat16_as_ushort(v.y) << 16);
-}
 
 template <class Src, int S>
 __global__ void __launch_bounds__(SL1_THREADS, 2) tc_slice1_kernel(SliceOp<Src> op0, SliceOp<Src> op1, int K, int Kp)
@@ -358,36 +397,22 @@ __global__ void __launch_bounds__(SL1_THREADS, 2) tc_slice1_kernel(SliceOp<Src> 
         long long x[4];
         to_fixed(srow[k], q, x[0], x[1]);
         to_fixed(srow[k + 1], q, x[2], x[3]);
-        // digits least significant first (digits64's order), each plane
-        // written as soon as its four digits exist
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[j] += digit_bias<S>();
 #pragma unroll
         for (int s = S - 1; s >= 0; --s) {
-            int d[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (s > 0) {
-                    int r = (int)(x[j] & 63);
-                    if (r > 32) r -= 64;
-                    d[j] = r;
-                    x[j] = (x[j] - r) >> 6;
-                } else {
-                    d[j] = (int)x[j];
-                }
-            }
+            uint2 u;
+            u.x = digit_pair<S>(x[0], x[1], s);
+            u.y = digit_pair<S>(x[2], x[3], s);
             __nv_bfloat16 *P = planes + (size_t)s * pstride + 2 * (size_t)k;
             const long long pext = (long long)S * pstride;   // this entry's planes
             if (!op.role_b) {
-                uint2 u;
-                u.x = bf2_bits(bf2(d[0], d[1]));
-                u.y = bf2_bits(bf2(d[2], d[3]));
                 if (IA_IDX_OK((long long)s * pstride + (long long)row * Kp + 2 * k + 3, pext))
                     *reinterpret_cast<uint2 *>(P + (size_t)row * Kp) = u;
             } else if (IA_IDX_OK((long long)s * pstride + (long long)(2 * row + 1) * Kp + 2 * k + 3, pext)) {
-                uint2 u0, u1;
-                u0.x = bf2_bits(bf2(d[0], -d[1]));
-                u0.y = bf2_bits(bf2(d[2], -d[3]));
-                u1.x = bf2_bits(bf2(d[1], d[0]));
-                u1.y = bf2_bits(bf2(d[3], d[2]));
+                // (re, -im) and (im, re)
+                const uint2 u0 = make_uint2(u.x ^ 0x80000000u, u.y ^ 0x80000000u);
+                const uint2 u1 = make_uint2(__funnelshift_l(u.x, u.x, 16), __funnelshift_l(u.y, u.y, 16));
                 *reinterpret_cast<uint2 *>(P + (size_t)(2 * row) * Kp) = u0;
                 *reinterpret_cast<uint2 *>(P + (size_t)(2 * row + 1) * Kp) = u1;
             }
@@ -469,22 +494,12 @@ __global__ void __launch_bounds__(SL1_THREADS, 2)
         to_fixed(make_double2(srow[k], srow[k + 1]), q, x[0], x[1]);
         to_fixed(make_double2(srow[k + 2], srow[k + 3]), q, x[2], x[3]);
 #pragma unroll
-        for (int s = S - 1; s >= 0; --s) {
-            int d[4];
+        for (int j = 0; j < 4; ++j) x[j] += digit_bias<S>();
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (s > 0) {
-                    int r = (int)(x[j] & 63);
-                    if (r > 32) r -= 64;
-                    d[j] = r;
-                    x[j] = (x[j] - r) >> 6;
-                } else {
-                    d[j] = (int)x[j];
-                }
-            }
+        for (int s = S - 1; s >= 0; --s) {
             uint2 u;
-            u.x = bf2_bits(bf2(d[0], d[1]));
-            u.y = bf2_bits(bf2(d[2], d[3]));
+            u.x = digit_pair<S>(x[0], x[1], s);
+            u.y = digit_pair<S>(x[2], x[3], s);
             if (IA_IDX_OK((long long)s * pstride + (long long)row * Kp + k + 3, (long long)S * pstride))
                 *reinterpret_cast<uint2 *>(P0 + (size_t)s * pstride + k) = u;
         }
@@ -494,6 +509,25 @@ __global__ void __launch_bounds__(SL1_THREADS, 2)
 // ---------------------------------------------------------------------------
 // the tensor-core GEMM on slice planes
 // ---------------------------------------------------------------------------
+// hi 2^30 + lo rounded once (|hi|, |lo| < 2^51): the integers become FP64 as the
+// low bits of 1.5 2^52, three FP64 instructions
+__device__ __forceinline__ double tc_round(long long hi, long long lo)
+{
+    constexpr long long MAGIC = 0x4338000000000000ll;   // 1.5 2^52
+    const double m = __longlong_as_double(MAGIC);
+    return fma(__longlong_as_double(MAGIC + hi) - m, 1073741824.0, __longlong_as_double(MAGIC + lo) - m);
+}
+// +-v 2^sc of an integer v, |v| < 2^81, by its exponent (a zero stays one):
+// TC_SAFE(sc) keeps the result a normal number
+__device__ __forceinline__ double tc_scale(double v, int sc, unsigned flip)
+{
+    int h = __double2hiint(v);
+    const int l = __double2loint(v);
+    h = (h & 0x7FFFFFFF) | l ? (h + (sc << 20)) ^ (int)flip : 0;
+    return __hiloint2double(h, l);
+}
+__device__ __forceinline__ bool tc_safe(int sc) { return sc > -1000 && sc < 900; }
+
 template <int S, bool REAL>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
@@ -510,7 +544,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     __shared__ __align__(8) uint64_t bar_full[TC_STAGES], bar_empty[TC_STAGES], bar_done;
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
-    __shared__ double s_colscale[TC_BN / CPC];
+    __shared__ double s_colscale[TC_BN / CPC];   // S <= 8
+    __shared__ int s_colexp[TC_BN / CPC];        // FP64 path
     unsigned char *base = reinterpret_cast<unsigned char *>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t base_u = tc::smem_u32(base);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -529,7 +564,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     if (warp == 2) tc::tmem_alloc(tc::smem_u32(&s_tmem), 512);
     if (threadIdx.x < TC_BN / CPC) {
         const int n = c0 / CPC + threadIdx.x;
-        if constexpr (S == TC_SLICES_FP64) s_colscale[threadIdx.x] = n < N ? fp64_scale(eb[(size_t)f * N + n]) : 0.0;
+        if constexpr (S == TC_SLICES_FP64) s_colexp[threadIdx.x] = n < N ? eb[(size_t)f * N + n] : 0;
         else s_colscale[threadIdx.x] = n < N ? ldexp(1.0, eb[(size_t)f * N + n]) : 0.0;
     }
     tc::tc_fence_before();
@@ -599,63 +634,82 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     // epilogue: this thread's row, 16 real columns at a time
     const int row = m0 + warp * 32 + lane;
     double rs = 0.0;
+    int er = 0;
     if (row < M) {
-        const int er = ea[(size_t)f * M + row];
-        // FP64 path: 2^(er - 32) here, 2^(ec - 32) per column (10 + 54 = 64)
-        if constexpr (S == TC_SLICES_FP64) rs = alpha * fp64_scale(er);
-        else rs = ldexp(alpha, er - 10 - 6 * (S - 1));
+        er = ea[(size_t)f * M + row];
+        if constexpr (S != TC_SLICES_FP64) rs = ldexp(alpha, er - 10 - 6 * (S - 1));
     }
+    const double amag = fabs(alpha);
     auto *Cf = C + f * sC;
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
+    // FP64 path: 2^(er + ec - 64) (10 + 54 = 64) goes into the exponents where no
+    // entry of the tile can leave the normal range, else by two multiplications:
+    // FP64 instructions, 64 cycles of a sub-partition each, bound the epilogue
+    // (with two conversions and the multiplications everywhere, rank-64 updates of
+    // a 642 x 642 matrix took 10 % longer; rounding in 128-bit integers was slower
+    // than either).
+    bool fast = true;
+    if constexpr (S == TC_SLICES_FP64) {
+        for (int q = 0; q < TC_BN / CPC; ++q) fast &= tc_safe(er + s_colexp[q] - 64);
+        fast = __syncthreads_and(fast) && amag == 1.0;
+    }
+    auto epilogue = [&](auto FAST) {
 #pragma unroll 1
-    for (int ch = 0; ch < TC_BN / 16; ++ch) {
-        uint32_t v[S][16];
+        for (int ch = 0; ch < TC_BN / 16; ++ch) {
+            uint32_t v[S][16];
 #pragma unroll
-        for (int L = 0; L < S; ++L) tc::tmem_ld16(lane_base + (uint32_t)(L * TC_BN + ch * 16), v[L]);
-        tc::tmem_wait_ld();
-        if (!ok || row >= M) continue;
-        // sum_L 64^(S-1-L) lev_L of real column j, rounded once
-        auto combine = [&](int j) -> double {
-            if constexpr (S <= 8) {
-                constexpr double TOP = (double)(1ll << (6 * (S - 1)));
-                long long acc = 0;
+            for (int L = 0; L < S; ++L) tc::tmem_ld16(lane_base + (uint32_t)(L * TC_BN + ch * 16), v[L]);
+            tc::tmem_wait_ld();
+            if (!ok || row >= M) continue;
+            // sum_L 64^(S-1-L) lev_L of real column j, scaled; FP64 path: rounded once
+            auto combine = [&](int j, int cq) -> double {
+                if constexpr (S <= 8) {
+                    constexpr double TOP = (double)(1ll << (6 * (S - 1)));
+                    long long acc = 0;
 #pragma unroll
-                for (int L = 1; L < S; ++L) acc = acc * 64 + (long long)__float2int_rn(__uint_as_float(v[L][j]));
-                return fma((double)__float2int_rn(__uint_as_float(v[0][j])), TOP, (double)acc);
-            } else {
-                // two groups of five levels, each an integer below 2^50
-                constexpr int H = 5;
-                long long hi = 0, lo = 0;
+                    for (int L = 1; L < S; ++L) acc = acc * 64 + (long long)__float2int_rn(__uint_as_float(v[L][j]));
+                    return fma((double)__float2int_rn(__uint_as_float(v[0][j])), TOP, (double)acc) *
+                           (rs * s_colscale[cq]);
+                } else {
+                    // two groups of five levels, each an integer below 2^50
+                    constexpr int H = 5;
+                    long long hi = 0, lo = 0;
 #pragma unroll
-                for (int L = 0; L < S - H; ++L) hi = hi * 64 + (long long)__float2int_rn(__uint_as_float(v[L][j]));
+                    for (int L = 0; L < S - H; ++L)
+                        hi = hi * 64 + (long long)__float2int_rn(__uint_as_float(v[L][j]));
 #pragma unroll
-                for (int L = S - H; L < S; ++L) lo = lo * 64 + (long long)__float2int_rn(__uint_as_float(v[L][j]));
-                return fma((double)hi, (double)(1ll << (6 * H)), (double)lo);
-            }
-        };
-#pragma unroll
-        for (int q = 0; q < 16 / CPC; ++q) {
-            const int n = c0 / CPC + ch * (16 / CPC) + q;
-            if (n >= N) break;
-            const double cs = s_colscale[ch * (16 / CPC) + q], sc = rs * cs;
-            // one factor at a time on the FP64 path: rs cs may leave the range where the result does not
-            auto scaled = [&](double v) { return S == TC_SLICES_FP64 ? (v * rs) * cs : v * sc; };
-            auto *p = Cf + row + (size_t)n * ldc;
-            if constexpr (REAL) {
-                double out = scaled(combine(q));
-                if (beta != 0.0) out = fma(beta, *p, out);
-                *p = out;
-            } else {
-                double2 out = make_double2(scaled(combine(2 * q)), scaled(combine(2 * q + 1)));
-                if (beta != 0.0) {
-                    const double2 old = *p;
-                    out.x = fma(beta, old.x, out.x);
-                    out.y = fma(beta, old.y, out.y);
+                    for (int L = S - H; L < S; ++L)
+                        lo = lo * 64 + (long long)__float2int_rn(__uint_as_float(v[L][j]));
+                    const double u = tc_round(hi, lo);
+                    const int ec = s_colexp[cq];
+                    if constexpr (decltype(FAST)::value) return tc_scale(u, er + ec - 64, alpha < 0.0 ? 0x80000000u : 0u);
+                    else return (u * (alpha * fp64_scale(er))) * fp64_scale(ec);
                 }
-                *p = out;
+            };
+#pragma unroll
+            for (int q = 0; q < 16 / CPC; ++q) {
+                const int n = c0 / CPC + ch * (16 / CPC) + q;
+                if (n >= N) break;
+                const int cq = ch * (16 / CPC) + q;
+                auto *p = Cf + row + (size_t)n * ldc;
+                if constexpr (REAL) {
+                    double out = combine(q, cq);
+                    if (beta != 0.0) out = fma(beta, *p, out);
+                    *p = out;
+                } else {
+                    double2 out = make_double2(combine(2 * q, cq), combine(2 * q + 1, cq));
+                    if (beta != 0.0) {
+                        const double2 old = *p;
+                        out.x = fma(beta, old.x, out.x);
+                        out.y = fma(beta, old.y, out.y);
+                    }
+                    *p = out;
+                }
             }
         }
-    }
+    };
+    if (fast) epilogue(std::true_type{});
+    else epilogue(std::false_type{});
     tc::tc_fence_before();
     __syncthreads();
     if (warp == 2) tc::tmem_dealloc(tmem, 512);
