@@ -665,14 +665,14 @@ int ia_ibem_assemble_batch(ia_context *ctx, const ia_mesh *mesh, int l, const do
     const bool mixed = cfg->precision == IA_PREC_MIXED;
     // the double-float assembly's geometry table lives in the workspace
     float2 *G = nullptr;
-    const size_t gbytes = mixed ? ibem_geom_bytes(mesh, mesh->m + n_ch + l) : 0;
+    const size_t gbytes = mixed ? ibem_geom_own_bytes(mesh, mesh->m + n_ch + l, F) : 0;
     if (gbytes) {
         const int st = ws_reserve(ctx, gbytes);
         if (st) return st;
         G = reinterpret_cast<float2 *>(ctx->ws);
     }
     return ibem_rows(ctx, mesh, l, d_mics, n_ch, d_cp, F, d_k, cfg->c, cfg->rho, (double2 *)d_At, (double2 *)d_Bt,
-                     (double2 *)d_Ahs_t, (double2 *)d_Bhs_t, mixed, false, G);
+                     (double2 *)d_Ahs_t, (double2 *)d_Bhs_t, mixed, false, G, gbytes);
 }
 
 // slice planes of the FP64 transfer's solver and products
@@ -729,7 +729,7 @@ static size_t transfer_mixed_ws_bytes(const ia_mesh *mesh, int l, int F, const i
 {
     const int m = mesh->m;
     size_t b = ws_round(8 * (size_t)m * m * F) + ws_round(8 * (size_t)m * l * F) + 3 * ws_round(16 * (size_t)m * l * F) +
-               (with_table ? ws_round(ibem_geom_bytes(mesh, m + l)) : 0);
+               (with_table ? ws_round(ibem_geom_own_bytes(mesh, m + l, F)) : 0);
     if (tc_products(cfg, m))
         b += tc_planes_bytes(m, m, cfg->gemm_slices, false, F) + tc_planes_bytes(l, m, cfg->gemm_slices, true, F) +
              1024;
@@ -752,7 +752,7 @@ static int ibem_transfer_t_mixed(ia_context *ctx, const ia_mesh *mesh, int l, co
     double2 *Y = cur.take<double2>((size_t)m * l * F);
     double2 *R = cur.take<double2>((size_t)m * l * F);
     float4 *Y4 = cur.take<float4>((size_t)m * l * F);
-    const size_t gbytes = ibem_geom_bytes(mesh, m + l);
+    const size_t gbytes = shared_geom ? ibem_geom_bytes(mesh, m + l) : ibem_geom_own_bytes(mesh, m + l, F);
     float2 *G = nullptr;
     bool build_geom = true;
     if (shared_geom) {
@@ -768,7 +768,7 @@ static int ibem_transfer_t_mixed(ia_context *ctx, const ia_mesh *mesh, int l, co
     {
         NvtxRange r("ia.assembly");
         st = ibem_rows(ctx, mesh, l, d_mics, 0, nullptr, F, d_k, cfg->c, cfg->rho, At, Bt, Ahs_t, Ht, true, true, G,
-                       build_geom);
+                       gbytes, build_geom);
     }
     if (st) return st;
     if (ev_rows) IA_CUDA_TRY(cudaEventRecord(ev_rows, ctx->stream));

@@ -256,7 +256,7 @@ __device__ __forceinline__ void write_split_rows(int m, int tid, const cx<dfl> *
 
 template <class R, bool GT>
 __global__ void __launch_bounds__(IBEM_THREADS, GT ? 7 : std::is_same<R, dfl>::value ? 5 : 3) ibem_rows_kernel(
-    int m, int n, int l, int n_ch, int ncolors, int F, const double *__restrict__ nodes, const double *__restrict__ egeo,
+    int m, int n, int l, int n_ch, int row0, int ncolors, int F, const double *__restrict__ nodes, const double *__restrict__ egeo,
     const R *__restrict__ qdat, const R *__restrict__ qnrm, const int *__restrict__ evert,
     const int *__restrict__ color_ptr, const int *__restrict__ adj_ptr, const int *__restrict__ adj, int nq,
     const double *__restrict__ reg,
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(IBEM_THREADS, GT ? 7 : std::is_same<R, dfl>::v
     // with the geometry table the frequency blocks of one row are consecutive
     // CTAs (one 1-D grid), so they read the row's table from L2 together
     const int nfb = (F + FB - 1) / FB;
-    const int row = GT ? (int)(blockIdx.x / nfb) : (int)blockIdx.x;
+    const int row = GT ? row0 + (int)(blockIdx.x / nfb) : (int)blockIdx.x;
     const int f0 = (GT ? (int)(blockIdx.x % nfb) : (int)blockIdx.y) * FB;
     const int mt = m + n_ch;
     FreqBlock fb;
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(IBEM_THREADS, GT ? 7 : std::is_same<R, dfl>::v
             for (int f = 0; f < FB; ++f)
 #pragma unroll
                 for (int v = 0; v < 3; ++v) { a[f][v] = cx_zero<R>(); b[f][v] = cx_zero<R>(); }
-            const float2 *gq = GT ? gtab + (size_t)row * nq * 3 * n + e : nullptr;
+            const float2 *gq = GT ? gtab + (size_t)(row - row0) * nq * 3 * n + e : nullptr;
             regular_element<R, FB, !DF, GT>(qdat, n, e, nq, qnrm[e], qnrm[e + n], qnrm[e + 2 * (size_t)n], xr, yr,
                                             zr, gq, fb, kf, dkf, tab, P, C, cw, a, b, ctr);
             if (!DF) ctr = r_norm(ctr);
@@ -494,15 +494,15 @@ int mesh_creg(ia_context *ctx, ia_mesh *mesh)
 // warp's threads (consecutive elements) load each value coalesced.  The rows
 // kernel then spends its issue slots on the per-frequency work only.  One
 // thread per (row, element).
-__global__ void __launch_bounds__(128) ibem_geom_kernel(int m, int n, int l, int n_ch, int nq, int nblk,
+__global__ void __launch_bounds__(128) ibem_geom_kernel(int m, int n, int l, int n_ch, int row0, int nrow, int nq, int nblk,
                                                         const double *__restrict__ nodes, const double *__restrict__ cp,
                                                         const double *__restrict__ mics, const dfl *__restrict__ qdat,
                                                         const dfl *__restrict__ qnrm, float2 *__restrict__ G)
 {
-    const int row = (int)(blockIdx.x / nblk);
+    const int row = row0 + (int)(blockIdx.x / nblk);
     const int e = (int)(blockIdx.x % nblk) * 128 + (int)threadIdx.x;
     const int mt = m + n_ch;
-    if (e >= n || row >= mt + l) return;
+    if (e >= n || row >= row0 + nrow) return;
     double xo, yo, zo;
     if (row < m) {
         xo = nodes[row]; yo = nodes[row + m]; zo = nodes[row + 2 * m];
@@ -515,11 +515,11 @@ __global__ void __launch_bounds__(128) ibem_geom_kernel(int m, int n, int l, int
     }
     const dfl xr = df_from_double(xo), yr = df_from_double(yo), zr = df_from_double(zo);
     const dfl nx = qnrm[e], ny = qnrm[e + n], nz = qnrm[e + 2 * (size_t)n];
-    [[maybe_unused]] const long long gext = (long long)(mt + l) * nq * 3 * n;
+    [[maybe_unused]] const long long gext = (long long)nrow * nq * 3 * n;
     for (int q = 0; q < nq; ++q) {
         dfl r, invr, ft;
         point_geometry(qdat + (size_t)q * 9 * n + e, n, nx, ny, nz, xr, yr, zr, r, invr, ft);
-        const long long o = ((long long)row * nq + q) * 3 * n + e;
+        const long long o = ((long long)(row - row0) * nq + q) * 3 * n + e;
         if (!IA_IDX_OK(o + 2 * (long long)n, gext)) continue;
         G[o] = make_float2(r.hi, r.lo);
         G[o + n] = make_float2(invr.hi, invr.lo);
@@ -528,21 +528,40 @@ __global__ void __launch_bounds__(128) ibem_geom_kernel(int m, int n, int l, int
 }
 
 // Largest geometry table the double-float assembly uses (per call, in the
-// caller's workspace); above it the rows kernel computes the geometry inline.
+// caller's workspace).  A table that several streams share (the staggered parts
+// of a solve) has to hold every row, and above the limit their rows kernel
+// computes the geometry inline; a call's own table is filled and read in chunks
+// of rows (1962 nodes, 150 microphones, 5 bins: inline 10.1 ms, chunked 7.5; 2
+// bins 4.1 and 3.6).  A single bin would only read each entry once: inline.
 // IA_ASM_GEOM_TABLE=0 selects the inline form at every size.
 constexpr size_t IBEM_GEOM_MAX_BYTES = size_t(1) << 30;
+
+static size_t geom_row_bytes(const ia_mesh *mesh) { return sizeof(float2) * 3 * (size_t)mesh->nq * mesh->n; }
 
 size_t ibem_geom_bytes(const ia_mesh *mesh, int rows)
 {
     const char *e = getenv("IA_ASM_GEOM_TABLE");
     if (e && e[0] == '0') return 0;
-    const size_t b = sizeof(float2) * 3 * (size_t)rows * mesh->nq * mesh->n;
+    const size_t b = geom_row_bytes(mesh) * rows;
     return b <= IBEM_GEOM_MAX_BYTES ? b : 0;
+}
+
+size_t ibem_geom_own_bytes(const ia_mesh *mesh, int rows, int F)
+{
+    const char *e = getenv("IA_ASM_GEOM_TABLE");
+    if (e && e[0] == '0') return 0;
+    const size_t row = geom_row_bytes(mesh), b = row * rows;
+    if (b <= IBEM_GEOM_MAX_BYTES) return b;
+    const size_t fit = IBEM_GEOM_MAX_BYTES / row;
+    if (F < 2 || fit < 1) return 0;
+    // chunks of equal size
+    const size_t chunks = (rows + fit - 1) / fit;
+    return row * ((rows + chunks - 1) / chunks);
 }
 
 int ibem_rows(ia_context *ctx, const ia_mesh *mesh, int l, const double *mics, int n_ch, const double *cp, int F,
               const double *k, double c, double rho, double2 *At, double2 *Bt, double2 *Ahs_t, double2 *Bhs_t,
-              bool df32, bool split_ab, float2 *gtab, bool build_gtab)
+              bool df32, bool split_ab, float2 *gtab, size_t gtab_bytes, bool build_gtab)
 {
     if (mesh->nq > IBEM_MAX_NQ) return IA_ERR_RULE;
     const int m = mesh->m;
@@ -556,27 +575,36 @@ int ibem_rows(ia_context *ctx, const ia_mesh *mesh, int l, const double *mics, i
     const int nfb = (F + FB - 1) / FB;
     dim3 g(rows, nfb);
     if (df32 && gtab) {
-        // the geometry table (ibem_geom_bytes(mesh, rows) bytes), then the rows
-        // kernel reading it, the frequency blocks of a row in consecutive CTAs
+        // the geometry table, then the rows kernel reading it, the frequency
+        // blocks of a row in consecutive CTAs; chunk by chunk where the table
+        // does not hold every row
         const int nblk = (mesh->n + 127) / 128;
-        if (build_gtab) {
-            ibem_geom_kernel<<<(unsigned)rows * nblk, 128, 0, ctx->stream>>>(
-                m, mesh->n, l, n_ch, mesh->nq, nblk, mesh->d_nodes, cp, mics, (const dfl *)mesh->d_qdat_f,
-                (const dfl *)mesh->d_qnrm_f, gtab);
-            IA_LAUNCH_CHECK(ctx);
-        }
+        const size_t fit = gtab_bytes / geom_row_bytes(mesh);
+        const int chunk = fit < (size_t)rows ? (int)fit : rows;
+        if (chunk < 1 || (chunk < rows && !build_gtab)) return IA_ERR_ARG;
         IA_CUDA_TRY(cudaFuncSetAttribute(ibem_rows_kernel<dfl, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          220 * 1024));
-        ibem_rows_kernel<dfl, true><<<(unsigned)rows * nfb, IBEM_THREADS, smem, ctx->stream>>>(
-            m, mesh->n, l, n_ch, mesh->ncolors, F, mesh->d_nodes, mesh->d_egeo, (const dfl *)mesh->d_qdat_f,
-            (const dfl *)mesh->d_qnrm_f, mesh->d_evert, mesh->d_color_ptr, mesh->d_adj_ptr, mesh->d_adj, mesh->nq,
-            mesh->d_reg, mesh->d_sing, mesh->nqs, mics, cp, k, c, rho, coef, red, mesh->d_dftab, split_ab ? 1 : 0,
-            mesh->d_creg, gtab, At, Bt, Ahs_t, Bhs_t);
+        for (int r0 = 0; r0 < rows; r0 += chunk) {
+            const int nr = rows - r0 < chunk ? rows - r0 : chunk;
+            if (build_gtab) {
+                ibem_geom_kernel<<<(unsigned)nr * nblk, 128, 0, ctx->stream>>>(
+                    m, mesh->n, l, n_ch, r0, nr, mesh->nq, nblk, mesh->d_nodes, cp, mics, (const dfl *)mesh->d_qdat_f,
+                    (const dfl *)mesh->d_qnrm_f, gtab);
+                IA_LAUNCH_CHECK(ctx);
+            }
+            ibem_rows_kernel<dfl, true><<<(unsigned)nr * nfb, IBEM_THREADS, smem, ctx->stream>>>(
+                m, mesh->n, l, n_ch, r0, mesh->ncolors, F, mesh->d_nodes, mesh->d_egeo, (const dfl *)mesh->d_qdat_f,
+                (const dfl *)mesh->d_qnrm_f, mesh->d_evert, mesh->d_color_ptr, mesh->d_adj_ptr, mesh->d_adj, mesh->nq,
+                mesh->d_reg, mesh->d_sing, mesh->nqs, mics, cp, k, c, rho, coef, red, mesh->d_dftab, split_ab ? 1 : 0,
+                mesh->d_creg, gtab, At, Bt, Ahs_t, Bhs_t);
+            IA_LAUNCH_CHECK(ctx);
+        }
+        return IA_OK;
     } else if (df32) {
         IA_CUDA_TRY(cudaFuncSetAttribute(ibem_rows_kernel<dfl, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          220 * 1024));
         ibem_rows_kernel<dfl, false><<<g, IBEM_THREADS, smem, ctx->stream>>>(
-            m, mesh->n, l, n_ch, mesh->ncolors, F, mesh->d_nodes, mesh->d_egeo, (const dfl *)mesh->d_qdat_f,
+            m, mesh->n, l, n_ch, 0, mesh->ncolors, F, mesh->d_nodes, mesh->d_egeo, (const dfl *)mesh->d_qdat_f,
             (const dfl *)mesh->d_qnrm_f, mesh->d_evert, mesh->d_color_ptr, mesh->d_adj_ptr, mesh->d_adj, mesh->nq,
             mesh->d_reg, mesh->d_sing, mesh->nqs, mics, cp, k, c, rho, coef, red, mesh->d_dftab, split_ab ? 1 : 0,
             mesh->d_creg, nullptr, At, Bt, Ahs_t, Bhs_t);
@@ -584,7 +612,7 @@ int ibem_rows(ia_context *ctx, const ia_mesh *mesh, int l, const double *mics, i
         IA_CUDA_TRY(cudaFuncSetAttribute(ibem_rows_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          220 * 1024));
         ibem_rows_kernel<double, false><<<g, IBEM_THREADS, smem, ctx->stream>>>(
-            m, mesh->n, l, n_ch, mesh->ncolors, F, mesh->d_nodes, mesh->d_egeo, mesh->d_qdat, mesh->d_qnrm,
+            m, mesh->n, l, n_ch, 0, mesh->ncolors, F, mesh->d_nodes, mesh->d_egeo, mesh->d_qdat, mesh->d_qnrm,
             mesh->d_evert, mesh->d_color_ptr, mesh->d_adj_ptr, mesh->d_adj, mesh->nq, mesh->d_reg, mesh->d_sing,
             mesh->nqs, mics, cp, k, c, rho, coef, red, nullptr, 0, nullptr, nullptr, At, Bt, Ahs_t, Bhs_t);
     }
