@@ -715,6 +715,204 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     if (warp == 2) tc::tmem_dealloc(tmem, 512);
 }
 
+// The FP64 path's product in tiles twice as wide.  An MMA of 48 columns waits on
+// shared memory: it reads 128 + 48 rows of 32 bytes (44 cycles) for 24 cycles of
+// arithmetic.  Here the ten levels are accumulated five at a time, so that five
+// 96-column accumulators fill the 480 TMEM columns (56 cycles for 48): levels 0-4
+// from the first five slices, their integer sums kept in registers (48 per thread,
+// eight warps), then levels 5-9 from all ten.  Stages of 16 K values in the 32-byte
+// swizzle.  Level sums are exact integers, so the results are those of
+// tc_gemm_kernel bit for bit.  256 x 256 x 256 products of
+// 64 bins 616 -> 466 us.
+constexpr int TW_BN = 96, TW_BK = 16, TW_STAGES = 3, TW_THREADS = 256, TW_H = 5;
+constexpr uint32_t TW_A_SLICE = TC_BM * TW_BK * 2, TW_B_SLICE = TW_BN * TW_BK * 2;
+constexpr uint32_t TW_STAGE = TC_SLICES_FP64 * (TW_A_SLICE + TW_B_SLICE);
+constexpr size_t TW_SMEM = (size_t)TW_STAGES * TW_STAGE + 1024;
+
+template <bool REAL>
+__global__ void __launch_bounds__(TW_THREADS, 1)
+    tc_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
+                        int Kp, const int *__restrict__ ea, const int *__restrict__ eb, double alpha, double beta,
+                        typename std::conditional<REAL, double, double2>::type *__restrict__ C, int ldc, long long sC,
+                        int *info)
+{
+    constexpr int S = TC_SLICES_FP64, CPC = REAL ? 1 : 2, HC = TW_BN / 2;   // columns per thread
+    static_assert(S == 2 * TW_H && TW_H * TW_BN <= 512, "two groups of levels in TMEM");
+    extern __shared__ unsigned char tc_smem_raw[];
+    __shared__ __align__(8) uint64_t bar_full[TW_STAGES], bar_empty[TW_STAGES], bar_done[2];
+    __shared__ uint32_t s_tmem;
+    __shared__ volatile int s_abort;
+    __shared__ int s_colexp[TW_BN / CPC];
+    unsigned char *base = reinterpret_cast<unsigned char *>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
+    const uint32_t base_u = tc::smem_u32(base);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int f = blockIdx.z, m0 = blockIdx.y * TC_BM, c0 = blockIdx.x * TW_BN;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < TW_STAGES; ++s) {
+            tc::mbar_init(tc::smem_u32(&bar_full[s]), 1);
+            tc::mbar_init(tc::smem_u32(&bar_empty[s]), 1);
+        }
+        tc::mbar_init(tc::smem_u32(&bar_done[0]), 1);
+        tc::mbar_init(tc::smem_u32(&bar_done[1]), 1);
+        s_abort = 0;
+        tc::mbar_fence_init();
+        tc::prefetch_tmap(&tmA);
+        tc::prefetch_tmap(&tmB);
+    }
+    if (warp == 2) tc::tmem_alloc(tc::smem_u32(&s_tmem), 512);
+    if (threadIdx.x < TW_BN / CPC) {
+        const int n = c0 / CPC + threadIdx.x;
+        s_colexp[threadIdx.x] = n < N ? eb[(size_t)f * N + n] : 0;
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    const int nkb = (Kp + TW_BK - 1) / TW_BK;
+    int issued = 0;   // producer: steps issued over both groups of levels
+
+    const int row = m0 + (warp & 3) * 32 + lane, half = warp >> 2;
+    const int er = row < M ? ea[(size_t)f * M + row] : 0;
+    const double amag = fabs(alpha);
+    bool fast = true;
+    for (int q = 0; q < TW_BN / CPC; ++q) fast &= tc_safe(er + s_colexp[q] - 64);
+    fast = __syncthreads_and(fast) && amag == 1.0;
+    auto *Cf = C + f * sC;
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(half * HC);
+    long long hi[HC];
+#pragma unroll
+    for (int group = 0; group < 2; ++group) {
+        if (warp == 0 && lane == 0) {
+            // producer; after the first group's steps it goes on into the second
+            // group's as far as the stages reach
+            const int end = group ? 2 * nkb : nkb + (TW_STAGES < nkb ? TW_STAGES : nkb);
+            for (int g = issued; g < end && !s_abort; ++g) {
+                const int s = g % TW_STAGES;
+                const uint32_t ph = (uint32_t)(g / TW_STAGES) & 1u;
+                if (g >= TW_STAGES && !tc::mbar_wait(tc::smem_u32(&bar_empty[s]), ph ^ 1u, TC_WAIT_NS)) {
+                    s_abort = 1;
+                    break;
+                }
+                const uint32_t full = tc::smem_u32(&bar_full[s]);
+                const bool second = g >= nkb;
+                const int k = (second ? g - nkb : g) * TW_BK;
+                tc::mbar_arrive_expect_tx(full, second ? TW_STAGE : TW_STAGE / 2);
+                const uint32_t a = base_u + (uint32_t)s * TW_STAGE, b = a + S * TW_A_SLICE;
+                tc::tma_load_4d(a, &tmA, k, m0, 0, f, full);
+                tc::tma_load_4d(b, &tmB, k, c0, 0, f, full);
+                if (second) {
+                    tc::tma_load_4d(a + TW_H * TW_A_SLICE, &tmA, k, m0, TW_H, f, full);
+                    tc::tma_load_4d(b + TW_H * TW_B_SLICE, &tmB, k, c0, TW_H, f, full);
+                }
+                issued = g + 1;
+            }
+        } else if (warp == 1 && lane == 0) {
+            // MMA issuer: level L = i + j accumulates in TMEM columns [96 (L - 5 group), + 96)
+            constexpr uint32_t idesc = tc::idesc_bf16_f32(TC_BM, TW_BN);
+            for (int kb = 0; kb < nkb; ++kb) {
+                const int g = group * nkb + kb, s = g % TW_STAGES;
+                const uint32_t ph = (uint32_t)(g / TW_STAGES) & 1u;
+                if (s_abort || !tc::mbar_wait(tc::smem_u32(&bar_full[s]), ph, TC_WAIT_NS)) {
+                    s_abort = 1;
+                    break;
+                }
+                tc::tc_fence_after();
+                const uint32_t a = base_u + (uint32_t)s * TW_STAGE, b = a + S * TW_A_SLICE;
+#pragma unroll
+                for (int i = 0; i < S; ++i) {
+                    const uint64_t ad = tc::sdesc(a + i * TW_A_SLICE, 256, 6);
+#pragma unroll
+                    for (int j = 0; j + i < S; ++j) {
+                        if ((i + j) / TW_H != group) continue;
+                        const uint64_t bd = tc::sdesc(b + j * TW_B_SLICE, 256, 6);
+                        tc::mma_bf16(tmem + (uint32_t)((i + j - group * TW_H) * TW_BN), ad, bd, idesc,
+                                     (kb | i) != 0 ? 1u : 0u);
+                    }
+                }
+                tc::mma_commit(tc::smem_u32(&bar_empty[s]));
+            }
+            tc::mma_commit(tc::smem_u32(&bar_done[group]));
+        }
+        __syncwarp();
+        if (!tc::mbar_wait(tc::smem_u32(&bar_done[group]), 0, 2 * TC_WAIT_NS)) s_abort = 1;
+        __syncwarp();
+        tc::tc_fence_after();
+        if (group == 0) {
+            // sum_L 64^(4-L) lev_L of this thread's columns, below 2^50
+#pragma unroll
+            for (int ch = 0; ch < HC / 16; ++ch) {
+                uint32_t v[TW_H][16];
+#pragma unroll
+                for (int L = 0; L < TW_H; ++L) tc::tmem_ld16(lane_base + (uint32_t)(L * TW_BN + ch * 16), v[L]);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                    long long acc = 0;
+#pragma unroll
+                    for (int L = 0; L < TW_H; ++L) acc = acc * 64 + (long long)__float2int_rn(__uint_as_float(v[L][q]));
+                    hi[ch * 16 + q] = acc;
+                }
+            }
+            // the second group overwrites the accumulators
+            tc::tc_fence_before();
+            __syncthreads();
+            tc::tc_fence_after();
+        }
+    }
+    __syncthreads();   // s_abort as every thread left it
+    const bool ok = !s_abort;
+    if (!ok && threadIdx.x == 0) {
+        if (info) atomicOr(info + f, IA_INFO_TIMEOUT);
+        // let this CTA's copies in flight land before the CTA ends
+        for (int g = issued - TW_STAGES > 0 ? issued - TW_STAGES : 0; g < issued; ++g)
+            tc::mbar_wait(tc::smem_u32(&bar_full[g % TW_STAGES]), (uint32_t)(g / TW_STAGES) & 1u, TC_WAIT_NS);
+    }
+    auto epilogue = [&](auto FAST) {
+#pragma unroll
+        for (int ch = 0; ch < HC / 16; ++ch) {
+            uint32_t v[TW_H][16];
+#pragma unroll
+            for (int L = 0; L < TW_H; ++L) tc::tmem_ld16(lane_base + (uint32_t)(L * TW_BN + ch * 16), v[L]);
+            tc::tmem_wait_ld();
+            if (!ok || row >= M) continue;
+            auto combine = [&](int q, int cq) -> double {
+                long long lo = 0;
+#pragma unroll
+                for (int L = 0; L < TW_H; ++L) lo = lo * 64 + (long long)__float2int_rn(__uint_as_float(v[L][q]));
+                const double u = tc_round(hi[ch * 16 + q], lo);
+                const int ec = s_colexp[cq];
+                if constexpr (decltype(FAST)::value) return tc_scale(u, er + ec - 64, alpha < 0.0 ? 0x80000000u : 0u);
+                else return (u * (alpha * fp64_scale(er))) * fp64_scale(ec);
+            };
+#pragma unroll
+            for (int q = 0; q < 16 / CPC; ++q) {
+                const int cq = (half * HC + ch * 16) / CPC + q, n = c0 / CPC + cq;
+                if (n < N) {
+                    auto *p = Cf + row + (size_t)n * ldc;
+                    if constexpr (REAL) {
+                        double out = combine(q, cq);
+                        if (beta != 0.0) out = fma(beta, *p, out);
+                        *p = out;
+                    } else {
+                        double2 out = make_double2(combine(2 * q, cq), combine(2 * q + 1, cq));
+                        if (beta != 0.0) {
+                            const double2 old = *p;
+                            out.x = fma(beta, old.x, out.x);
+                            out.y = fma(beta, old.y, out.y);
+                        }
+                        *p = out;
+                    }
+                }
+            }
+        }
+    };
+    if (fast) epilogue(std::true_type{});
+    else epilogue(std::false_type{});
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 2) tc::tmem_dealloc(tmem, 512);
+}
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -738,19 +936,21 @@ int encode_fn(PFN_cuTensorMapEncodeTiled_v12000 *out)
     return IA_OK;
 }
 
-// 4-D map over planes [batch][S][rows][Kp] (BF16), box (32, box_rows, S, 1),
-// 64-byte swizzle
-int make_tmap(CUtensorMap *tm, const __nv_bfloat16 *planes, int Kp, int rows, int S, int batch, int box_rows)
+// 4-D map over planes [batch][S][rows][Kp] (BF16): box (32, box_rows, S, 1) in the
+// 64-byte swizzle, or (16, box_rows, 5, 1) in the 32-byte one (wide)
+int make_tmap(CUtensorMap *tm, const __nv_bfloat16 *planes, int Kp, int rows, int S, int batch, int box_rows,
+              bool wide = false)
 {
     PFN_cuTensorMapEncodeTiled_v12000 enc;
     int st = encode_fn(&enc);
     if (st) return st;
     const cuuint64_t dims[4] = {(cuuint64_t)Kp, (cuuint64_t)rows, (cuuint64_t)S, (cuuint64_t)batch};
     const cuuint64_t strides[3] = {(cuuint64_t)Kp * 2, (cuuint64_t)rows * Kp * 2, (cuuint64_t)S * rows * Kp * 2};
-    const cuuint32_t box[4] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows, (cuuint32_t)S, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)(wide ? TW_BK : TC_BK), (cuuint32_t)box_rows, (cuuint32_t)(wide ? TW_H : S), 1};
     const cuuint32_t es[4] = {1, 1, 1, 1};
     CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16 *>(planes), dims, strides, box,
-                     es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     es, CU_TENSOR_MAP_INTERLEAVE_NONE, wide ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? IA_OK : IA_ERR_CUDA;
 }
@@ -764,6 +964,36 @@ int gemm_launch(ia_context *ctx, const CUtensorMap &ta, const CUtensorMap &tb, c
     dim3 grid(((REAL ? 1 : 2) * N + tc_bn(S) - 1) / tc_bn(S), (M + TC_BM - 1) / TC_BM, batch);
     tc_gemm_kernel<S, REAL><<<grid, TC_THREADS, smem, ctx->stream>>>(ta, tb, M, N, A.Kp, A.e, B.e, alpha, beta, C,
                                                                       ldc, sC, info);
+    IA_LAUNCH_CHECK(ctx);
+    return IA_OK;
+}
+
+// The wide tiles where their waves, at 1.25 times a narrow tile's time (78 against
+// 62 us at K = 256 complex), are the shorter: from about two waves on; below, the
+// narrow tiles spread over more SMs (rank-64 updates of one 642 x 642 matrix: 135
+// against 70 tiles).  The results are the same.
+bool tc_wide(const ia_context *ctx, int M, int ncols, int batch)
+{
+    auto waves = [&](int bn) {
+        const long long t = (long long)((ncols + bn - 1) / bn) * ((M + TC_BM - 1) / TC_BM) * batch;
+        return (t + ctx->sm_count - 1) / ctx->sm_count;
+    };
+    return 5 * waves(TW_BN) < 4 * waves(tc_bn(TC_SLICES_FP64));
+}
+
+template <bool REAL, class TC>
+int gemm_wide_launch(ia_context *ctx, const TcPlanes &A, const TcPlanes &B, int M, int N, double alpha, double beta, TC *C,
+                     int ldc, long long sC, int batch, int *info)
+{
+    CUtensorMap ta, tb;
+    int st = make_tmap(&ta, A.p, A.Kp, A.rows, A.S, batch, TC_BM, true);
+    if (!st) st = make_tmap(&tb, B.p, B.Kp, B.rows, B.S, batch, TW_BN, true);
+    if (st) return st;
+    IA_CUDA_TRY(cudaFuncSetAttribute(tc_gemm_wide_kernel<REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)TW_SMEM));
+    dim3 grid(((REAL ? 1 : 2) * N + TW_BN - 1) / TW_BN, (M + TC_BM - 1) / TC_BM, batch);
+    tc_gemm_wide_kernel<REAL><<<grid, TW_THREADS, TW_SMEM, ctx->stream>>>(ta, tb, M, N, A.Kp, A.e, B.e, alpha, beta, C,
+                                                                          ldc, sC, info);
     IA_LAUNCH_CHECK(ctx);
     return IA_OK;
 }
@@ -874,6 +1104,8 @@ int tc_gemm(ia_context *ctx, const TcPlanes &A, const TcPlanes &B, int M, int N,
 {
     if (M <= 0 || N <= 0 || batch <= 0) return IA_OK;
     if (A.S != B.S || A.Kp != B.Kp || A.R != M || B.R != N || A.rows != M || B.rows != 2 * N) return IA_ERR_ARG;
+    if (A.S == TC_SLICES_FP64 && tc_wide(ctx, M, 2 * N, batch))
+        return gemm_wide_launch<false>(ctx, A, B, M, N, alpha, beta, C, ldc, sC, batch, info);
     CUtensorMap ta, tb;
     int st = make_tmap(&ta, A.p, A.Kp, A.rows, A.S, batch, TC_BM);
     if (!st) st = make_tmap(&tb, B.p, B.Kp, B.rows, B.S, batch, tc_bn(A.S));
@@ -924,6 +1156,8 @@ int tc_gemm_real(ia_context *ctx, const TcPlanes &A, const TcPlanes &B, int M, i
 {
     if (M <= 0 || N <= 0 || batch <= 0) return IA_OK;
     if (A.S != TC_SLICES_FP64 || B.S != A.S || A.Kp != B.Kp || A.rows != M || B.rows != N) return IA_ERR_ARG;
+    if (tc_wide(ctx, M, N, batch))
+        return gemm_wide_launch<true>(ctx, A, B, M, N, alpha, beta, C, ldc, sC, batch, info);
     CUtensorMap ta, tb;
     int st = make_tmap(&ta, A.p, A.Kp, A.rows, A.S, batch, TC_BM);
     if (!st) st = make_tmap(&tb, B.p, B.Kp, B.rows, B.S, batch, tc_bn(A.S));
