@@ -20,6 +20,7 @@
 // whose products use double-float arithmetic on the FP32 pipe.
 #include "df32.cuh"
 #include <cooperative_groups.h>
+#include <cuda_pipeline.h>
 #include "ia_common.cuh"
 #include "ia_internal.h"
 
@@ -545,11 +546,13 @@ static bool rqr_cluster_launch(ia_context *ctx, int rows, int cols, T *Y, T *tau
 // The same explicit factor over column groups: CTA (g, f) forms columns
 // [FQ_COLS g, FQ_COLS (g + 1)) of bin f's Q, a warp per column held in shared
 // memory; each reflector j (from the group's last column down to 0) is staged
-// in shared memory once and applied by every warp whose column c >= j.  The
-// operations per column are rform_q_kernel's, in the same order (bitwise the
-// same Q); a bin's columns spread over cols / FQ_COLS CTAs instead of one,
-// and a reflector is read from L2 once per CTA instead of once per warp.
-constexpr int FQ_COLS = 16;
+// in shared memory once, while the one before is applied, and applied by every
+// warp whose column c >= j.  The operations per column are rform_q_kernel's, in
+// the same order (bitwise the same Q).  Bound by the FP64 pipe, on which a warp's
+// instruction holds its SM sub-partition for 64 cycles: four columns per CTA are
+// one per sub-partition (1280 x 40, 16 bins: 195 us; with 16 columns per CTA, on
+// 48 of 152 SMs, 342).
+constexpr int FQ_COLS = 4;
 
 template <class T>
 __global__ void __launch_bounds__(32 * FQ_COLS) rform_q_group_kernel(int rows, int cols, const T *__restrict__ Y,
@@ -557,27 +560,36 @@ __global__ void __launch_bounds__(32 * FQ_COLS) rform_q_group_kernel(int rows, i
 {
     extern __shared__ __align__(16) unsigned char fq_raw[];
     T *qs = reinterpret_cast<T *>(fq_raw);   // FQ_COLS x rows: the group's columns
-    T *vs = qs + (size_t)FQ_COLS * rows;     // rows: the current reflector
-    const int f = blockIdx.y, c0 = blockIdx.x * FQ_COLS;
+    T *vs = qs + (size_t)FQ_COLS * rows;     // 2 x rows: reflectors, by parity of j
+    // the longest groups (the last columns) of every bin first
+    const int f = blockIdx.x, c0 = (gridDim.y - 1 - blockIdx.y) * FQ_COLS;
     Y += (size_t)f * rows * cols;
     tau += (size_t)f * cols;
     Q += (size_t)f * rows * cols;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int c = c0 + wid;
     T *q = qs + (size_t)wid * rows;
+    auto stage = [&](int j) {
+        T *v = vs + (size_t)(j & 1) * rows;
+        for (int i = j + 1 + (int)threadIdx.x; i < rows; i += blockDim.x)
+            __pipeline_memcpy_async(v + i, Y + i + (size_t)j * rows, sizeof(T));
+        __pipeline_commit();
+    };
+    const int ctop = (c0 + FQ_COLS < cols ? c0 + FQ_COLS : cols) - 1, top = ctop < rows - 1 ? ctop : rows - 1;
+    stage(top);
     for (int i = lane; i < rows; i += 32) q[i] = i == c ? T(1) : T(0);
-    const int ctop = (c0 + FQ_COLS < cols ? c0 + FQ_COLS : cols) - 1;
-    for (int j = ctop < rows - 1 ? ctop : rows - 1; j >= 0; --j) {
-        __syncthreads();   // every warp is done with the previous reflector
-        for (int i = j + 1 + (int)threadIdx.x; i < rows; i += blockDim.x) vs[i] = Y[i + (size_t)j * rows];
-        __syncthreads();
+    for (int j = top; j >= 0; --j) {
+        __pipeline_wait_prior(0);
+        __syncthreads();   // reflector j is here, every warp is done with j + 1
+        if (j > 0) stage(j - 1);
         const T t = tau[j];
         if (t == 0 || c >= cols || j > c) continue;   // H_j leaves e_c alone for j > c
+        const T *v = vs + (size_t)(j & 1) * rows;
         T acc = lane == 0 ? q[j] : T(0);
-        for (int i = j + 1 + lane; i < rows; i += 32) acc = fma(vs[i], q[i], acc);
+        for (int i = j + 1 + lane; i < rows; i += 32) acc = fma(v[i], q[i], acc);
         acc = warp_sum(acc) * t;
         if (lane == 0) q[j] -= acc;
-        for (int i = j + 1 + lane; i < rows; i += 32) q[i] = fma(-vs[i], acc, q[i]);
+        for (int i = j + 1 + lane; i < rows; i += 32) q[i] = fma(-v[i], acc, q[i]);
     }
     __syncwarp();
     if (c < cols)
@@ -604,12 +616,12 @@ static int orthonormalise(ia_context *ctx, int rows, int cols, T *Y, T *tau, T *
         rqr_kernel<T><<<batch, RQR_THREADS, 0, ctx->stream>>>(rows, cols, Y, tau);
     if (st) return st;
     IA_LAUNCH_CHECK(ctx);
-    const size_t fsm = sizeof(T) * (size_t)(FQ_COLS + 1) * rows;
+    const size_t fsm = sizeof(T) * (size_t)(FQ_COLS + 2) * rows;
     if (fsm <= 200 * 1024) {
         if (fsm > 48 * 1024)
             IA_CUDA_TRY(cudaFuncSetAttribute(rform_q_group_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)fsm));
-        dim3 g((cols + FQ_COLS - 1) / FQ_COLS, batch);
+        dim3 g(batch, (cols + FQ_COLS - 1) / FQ_COLS);
         rform_q_group_kernel<T><<<g, 32 * FQ_COLS, fsm, ctx->stream>>>(rows, cols, Y, tau, Q);
     } else {
         rform_q_kernel<T><<<batch, 512, 0, ctx->stream>>>(rows, cols, Y, tau, Q);
