@@ -5,7 +5,7 @@
 // for the update, 2 more for the exact remaining norms of the pivoted form.
 // One CTA per matrix left most SMs idle, and FP64 instructions that are
 // predicated off still take the pipe's time.  Per call: 48 bins of 1280 x 192
-// 73 -> 43 ms, 64 of 256 x 256 46 -> 15, 23 of 642 x 120 16 -> 4.6.  Here the columns of one matrix are dealt cyclically to the
+// 73 -> 40 ms, 64 of 256 x 256 46 -> 14, 23 of 642 x 120 16 -> 4.6.  Here the columns of one matrix are dealt cyclically to the
 // CTAs of a cluster, a warp per column; per step
 //   - every CTA publishes its pivot candidate; one cluster barrier;
 //   - every CTA reads the pivot column's rows (from L2; its owner wrote them
@@ -267,7 +267,11 @@ static size_t zq_smem_bytes(int rows, int cols)
     return sizeof(double2) * (size_t)rows + (sizeof(double) + 2 * sizeof(int)) * (size_t)cols;
 }
 
-bool zqr_ok(int rows, int cols) { return zq_smem_bytes(rows, cols) <= 200 * 1024; }
+constexpr size_t ZQ_SMEM_MAX = 200 * 1024;   // (one CTA per SM)
+// a step's work beside the columns, in columns; time of CTAs that share an SM
+constexpr double ZQ_STEP = 16.0, ZQ_SHARED = 1.5;
+
+bool zqr_ok(int rows, int cols) { return zq_smem_bytes(rows, cols) <= ZQ_SMEM_MAX; }
 
 template <bool PIV>
 static int zqr_launch(ia_context *ctx, int rows, int cols, double2 *A, int lda, long long sA, double2 *tau, int *perm,
@@ -278,14 +282,19 @@ static int zqr_launch(ia_context *ctx, int rows, int cols, double2 *A, int lda, 
                 : rows <= 768  ? zqr_cluster_kernel<24, 2, PIV>
                 : rows <= 1280 ? zqr_cluster_kernel<40, 4, PIV>
                                : zqr_cluster_kernel<0, 1, PIV>;
-    if (smem > 48 * 1024)
-        IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // the largest cluster with a column per warp whose clusters all run at once
-    // (a cluster stays inside one GPC, so c * batch SMs do not always do: 48
-    // clusters of 3 took two waves, 57 ms against 43 with 2)
+    IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZQ_SMEM_MAX));
+    // The cluster size of least waves (cols / c + ZQ_STEP) among those with a
+    // column per warp: a step's columns over the CTAs, plus what each CTA does for
+    // itself (reflector, barrier: as long as about 16 columns of the update: 64
+    // to 256 columns).  A cluster stays inside one GPC, so fewer run at once than c *
+    // batch SMs hold: 46 of 3, 28 of 5, 15 of 8.  Two waves of larger
+    // clusters can then beat one: 48 bins of 1280 x 192 44.3 ms with 2, 56.4 with
+    // 3, 39.6 with 5; 90 bins 79.1 with 1, 59.5 with 3.  Up to 768 rows (and
+    // streamed) two CTAs fit an SM; sharing it costs up to 1.6: 48 bins of 256 x
+    // 256 17.9 ms with 3 (two clusters on shared SMs), 15.4 with 2 (none), 12.1
+    // with 5 (all); 64 bins 15.4 with 2, 14.4 with 4.
     cudaLaunchConfig_t lc = {};
     lc.blockDim = dim3(ZQ_THREADS);
-    lc.dynamicSmemBytes = smem;
     lc.stream = ctx->stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -294,17 +303,29 @@ static int zqr_launch(ia_context *ctx, int rows, int cols, double2 *A, int lda, 
     lc.attrs = at;
     lc.numAttrs = 1;
     int cs = 1;
-    for (int c : {8, 6, 5, 4, 3, 2}) {
-        if (c * batch > ctx->sm_count || c * ZQ_WARPS > cols) continue;
-        int fit = 0;
+    double least = 0.0;
+    for (int c : {8, 6, 5, 4, 3, 2, 1}) {
+        if (c > 1 && c * ZQ_WARPS > cols) continue;
         lc.gridDim = dim3((unsigned)(c * batch));
         at[0].val.clusterDim.x = c;
-        IA_CUDA_TRY(cudaOccupancyMaxActiveClusters(&fit, kern, &lc));
-        if (fit >= batch) {
-            cs = c;
+        int alone = 0, fit = 0;   // clusters at once, a CTA per SM and as many as fit
+        lc.dynamicSmemBytes = ZQ_SMEM_MAX;
+        if (c * batch <= ctx->sm_count) IA_CUDA_TRY(cudaOccupancyMaxActiveClusters(&alone, kern, &lc));
+        const double one = (double)cols / c + ZQ_STEP;
+        if (alone >= batch) {   // no smaller cluster is faster than one wave of these
+            if (!least || one < least) cs = c;
             break;
         }
+        lc.dynamicSmemBytes = smem;
+        IA_CUDA_TRY(cudaOccupancyMaxActiveClusters(&fit, kern, &lc));
+        if (fit < 1) continue;
+        const double cost = one * ((batch + fit - 1) / fit) * (c * fit > ctx->sm_count ? ZQ_SHARED : 1.0);
+        if (!least || cost < least) {
+            least = cost;
+            cs = c;
+        }
     }
+    lc.dynamicSmemBytes = smem;
     lc.gridDim = dim3((unsigned)(cs * batch));
     at[0].val.clusterDim.x = cs;
     IA_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, rows, cols, A, lda, sA, tau, perm));

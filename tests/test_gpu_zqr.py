@@ -70,3 +70,12 @@ def test_wide_solve_qr_degenerate_columns(cuda, ctx, kind):
         assert not x.any() and not s.any() and not info.any()
         return
     _check(ctx, cuda, H, b, lam)
+
+
+# batches whose clusters run in several waves or two CTAs to an SM
+@pytest.mark.parametrize("m,n,F", [(64, 160, 49), (40, 200, 101), (48, 800, 61), (100, 642, 80), (16, 20, 400)])
+def test_wide_solve_qr_waves(cuda, ctx, m, n, F):
+    rng = np.random.default_rng(m * 1000 + F)
+    H = rng.normal(size=(F, m, n)) + 1j * rng.normal(size=(F, m, n))
+    b = rng.normal(size=(F, 1, m)) + 1j * rng.normal(size=(F, 1, m))
+    _check(ctx, cuda, H, b, 0.3 * np.linalg.norm(H[0], 2))
