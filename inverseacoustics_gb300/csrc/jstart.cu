@@ -48,7 +48,7 @@ namespace ia {
 // (measured with the rotations still carried along: the figures below are
 // today's).  Operators above that level gain more: 64 microphones, one bin, the
 // whole ESM solve 4.7 -> 2.5 ms; 192 microphones, 48 bins 170 -> 61 ms; 64 order-15
-// HELS bins (256 x 256) 401 -> 54 to 63 ms, the more the more bins need the FP64
+// HELS bins (256 x 256) 401 -> 51 to 57 ms, the more the more bins need the FP64
 // Jacobi's last sweep.
 constexpr int JS_MIN_N = 64, JS_MAX_N = 256;
 constexpr int JS_FP32_SWEEPS = 12;
