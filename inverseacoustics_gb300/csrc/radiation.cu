@@ -38,11 +38,16 @@ namespace ia {
 //   - evenly spaced wavenumbers: frequencies go in blocks of 2 SR_J + 1 around a
 //     centre, sin(a +- j b) = sin a cos jb +- cos a sin jb giving two outputs
 //     for one multiply and two FMAs, and the centre advances by one rotation
-//     per block.  The step exp(i 9 dk r) is evaluated directly, so after the
-//     at most 7 steps of a chunk the phase error is that of rounding k r.
+//     per block, the step exp(i 9 dk r) evaluated directly.  An output's error is
+//     then that of rounding the largest phase on the way to it, so a chunk runs
+//     from its end of smaller |k|, and a first bin below a quarter of the first
+//     centre is evaluated directly and the centre reached from it (with a sincos
+//     for each, 10 % of the time): relative to its own max|R| no bin loses more
+//     than the factor 4 (a sweep from 1 Hz in either direction: 1e-14, without
+//     the two 1e-12).
 // 21 -> 2.8 FP64 instructions per stored value and half the entries: 64 bins of
-// 1280^2 in 0.59 ms (was 3.13 ms).  Below 4 frequencies, and for unevenly
-// spaced wavenumbers, every phase is evaluated directly.
+// 1280^2 in 0.57 ms (was 3.13 ms).  Below 4 frequencies, for unevenly spaced
+// wavenumbers and across k = 0, every phase is evaluated directly.
 // --------------------------------------------------------------------------
 constexpr int SR_TILE = 16;
 constexpr int SR_J = 4, SR_BLK = 2 * SR_J + 1;
@@ -60,22 +65,25 @@ __global__ void __launch_bounds__(SR_TILE *SR_TILE) sinc_r_kernel(int n, const d
     while ((long long)(ti + 1) * (ti + 2) / 2 <= t) ++ti;
     const int tj = t - (int)((long long)ti * (ti + 1) / 2);
     const int f0 = blockIdx.y * SR_CHUNK, nf = min(SR_CHUNK, F - f0);
-    if (threadIdx.x < nf) sk[threadIdx.x] = kv[f0 + threadIdx.x];
+    // in the order of increasing |k|
+    const bool down = fabs(kv[f0 + nf - 1]) < fabs(kv[f0]);
+    if (threadIdx.x < nf) sk[threadIdx.x] = kv[f0 + (down ? nf - 1 - (int)threadIdx.x : (int)threadIdx.x)];
     __syncthreads();
     const double k0 = sk[0], dk = nf > 1 ? (sk[nf - 1] - k0) / (nf - 1) : 0.0;
     const bool odd_k = threadIdx.x < nf &&
                        !(fabs(sk[threadIdx.x] - (k0 + threadIdx.x * dk)) <= 1e-12 * fabs(sk[threadIdx.x]));
-    const bool uniform = !__syncthreads_or(odd_k) && nf >= 4;
+    const bool uniform = !__syncthreads_or(odd_k) && nf >= 4 && !(k0 * sk[nf - 1] < 0.0);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int i = ti * SR_TILE + (wid & 1) * 8 + (lane & 7), j = tj * SR_TILE + (wid >> 1) * 4 + (lane >> 3);
     if (i >= n || j > i) return;
     const double dx = x[i] - x[j], dy = x[i + n] - x[j + n], dz = x[i + 2 * (size_t)n] - x[j + 2 * (size_t)n];
     const double r = sqrt(dx * dx + dy * dy + dz * dz);
-    const size_t nn = (size_t)n * n;
-    double *lo = R + (size_t)f0 * nn + (size_t)j * n + i, *up = R + (size_t)f0 * nn + (size_t)i * n + j;
+    const size_t nn = (size_t)n * n, ff = f0 + (down ? nf - 1 : 0);
+    const long long step = down ? -(long long)nn : (long long)nn;
+    double *lo = R + ff * nn + (size_t)j * n + i, *up = R + ff * nn + (size_t)i * n + j;
     auto put = [&](int f, double v) {
-        lo[(size_t)f * nn] = v;
-        up[(size_t)f * nn] = v;
+        lo[f * step] = v;
+        up[f * step] = v;
     };
     if (r == 0.0) {
         for (int f = 0; f < nf; ++f) put(f, pref * sk[f] * sk[f]);
@@ -94,11 +102,19 @@ __global__ void __launch_bounds__(SR_TILE *SR_TILE) sinc_r_kernel(int n, const d
         cj[q] = fma(cj[q - 1], cj[0], -sj[q - 1] * sj[0]);
         sj[q] = fma(sj[q - 1], cj[0], cj[q - 1] * sj[0]);
     }
+    const double kc = k0 + SR_J * dk;
+    const bool low = 4.0 * fabs(k0) < fabs(kc);
     double s, c, ss = 0.0, cs = 1.0;
-    sincos((k0 + SR_J * dk) * r, &s, &c);
+    sincos((low ? k0 : kc) * r, &s, &c);
     if (nf > SR_BLK) sincos(SR_BLK * dk * r, &ss, &cs);
     s *= amp;
     c *= amp;
+    if (low) {
+        put(0, k0 * s);
+        const double s1 = fma(s, cj[SR_J - 1], c * sj[SR_J - 1]);
+        c = fma(c, cj[SR_J - 1], -s * sj[SR_J - 1]);
+        s = s1;
+    }
     for (int b = 0;; b += SR_BLK) {
         const int fc = b + SR_J;
         if (fc < nf) put(fc, sk[fc] * s);
@@ -106,7 +122,7 @@ __global__ void __launch_bounds__(SR_TILE *SR_TILE) sinc_r_kernel(int n, const d
         for (int q = 0; q < SR_J; ++q) {
             const int fm = fc - 1 - q, fp = fc + 1 + q;
             const double p = s * cj[q];
-            if (fm < nf) put(fm, sk[fm] * fma(-c, sj[q], p));
+            if (fm < nf && (fm > 0 || !low)) put(fm, sk[fm] * fma(-c, sj[q], p));
             if (fp < nf) put(fp, sk[fp] * fma(c, sj[q], p));
         }
         if (b + SR_BLK >= nf) break;
