@@ -8,9 +8,9 @@
 // the FP64 work is products on the tensor cores (10 BF16 slices, zgemm_tc):
 //   1. FP32 Jacobi of R scaled by a power of two; the rotations are recorded and
 //      then applied to J;
-//   2. J's polar factor in FP64: with D = I - J^H J (|D|_F ~ 2e-4 in FP32),
-//      J <- J + J (D / 2 + 3 D^2 / 8 + D^2 (5 D / 16 + 35 D^2 / 128)), unitary to
-//      |D|^5 (cf. Higham, Functions of Matrices, ch. 8);  M = R J: couplings
+//   2. J's polar factor in FP64: with E = I - J^H J (|E|_F ~ 2e-4 in FP32),
+//      J <- J + J (E / 2 + 3 E^2 / 8 + E^2 (5 E / 16 + 35 E^2 / 128)), unitary to
+//      |E|^5 (cf. Higham, Functions of Matrices, ch. 8);  M = R J: couplings
 //      |m_i^H m_j| / |m_i||m_j| ~ 1e-5;
 //   3. three times: G = M^H M, T_ij = G_ij / (G_jj - G_ii) anti-Hermitian, the
 //      first-order rotation that removes G_ij, with the large entries (near-equal
@@ -18,11 +18,7 @@
 //      I + T, by its series: to T^11 in the first step (|T| <= 0.05), to T^4 in
 //      the second (|T| <= 6e-4), to T^2 in the third (|T| <= 5e-6).  Each step
 //      squares the couplings; the third clears the smallest columns, whose
-//      products the large ones hide before the first.  A step runs
-//      on M D^-1 and D T D^-1, D the column norms: a slice product's error is
-//      relative to the largest entries of a row and a column, which would leave
-//      columns far below the largest with the large ones' rounding (order-15 HELS:
-//      22,000 of 32,640 pairs left to rotate);
+//      products the large ones hide before the first;
 //   4. what is left -- near-equal singular values, columns at the rounding level
 //      of the largest -- in FP64 sweeps over the pairs that G = M^H M shows above
 //      the Jacobi's test, G anew for each: a sweep costs its rotations and a
@@ -52,8 +48,8 @@ namespace ia {
 // Jacobi's last sweep.
 constexpr int JS_MIN_N = 64, JS_MAX_N = 256;
 constexpr int JS_FP32_SWEEPS = 12;
-constexpr double JS_MAX_D = 1e-3;      // largest |J^H J - I|_F: 63/256 |D|^5 = 2.5e-16
-constexpr float JS_MAX_T1 = 0.05f;     // largest |T|_F of the first step: 231/1024 |T|^12 = 6e-17
+constexpr double JS_MAX_D = 1e-3;      // largest |D (I - J^H J) D^-1|_F: 63/256 of its fifth power = 2.5e-16
+constexpr float JS_MAX_T1 = 0.05f;     // largest |D T D^-1|_F of the first step: 231/1024 |T|^12 = 6e-17
 constexpr float JS_MAX_T2 = 6e-4f;     // of the second: 3/8 |T|^5 = 3e-17
 constexpr float JS_MAX_T3 = 5e-6f;     // of the third: |T|^3 / 2 = 6e-17
 // flagged sweeps: they rotate a few pairs at the rounding level
@@ -62,33 +58,68 @@ constexpr int JS_THREADS = 512;
 
 bool jacobi_precondition_ok(int N) { return N >= JS_MIN_N && N <= JS_MAX_N && tc_fp64_ok(N); }
 
-// 2^-e with |R(0, 0)| < 2^e (the pivoted R's largest entry); 1 for a zero or
-// non-finite R(0, 0)
+// The FP32 Jacobi's units: |R(0, 0)| (the pivoted R's largest entry) between 2^54
+// and 2^55, so that squared norms lie below 256 * 2^110 and columns down to 1e-33
+// of the largest still rotate (the squares of 3e-17 of it, in units of R(0, 0),
+// already near FP32's underflow: order-15 HELS then keeps hundreds of unrotated
+// pairs at the rounding level).  1 for a zero or non-finite R(0, 0).
 __device__ __forceinline__ double js_scale(const double2 *R)
 {
     const double a = fmax(fabs(R[0].x), fabs(R[0].y));
     const int e = (int)((__double_as_longlong(a) >> 52) & 0x7FF);
-    return e > 0 && e < 0x7FF ? ldexp(1.0, 1022 - e) : 1.0;
+    return e > 0 && e < 0x7FF ? ldexp(1.0, min(1022 + 55 - e, 1023)) : 1.0;
 }
 
-// Y (N x N FP32) = R's first N rows, scaled
-__global__ void js_init_kernel(int ld, int N, const double2 *__restrict__ R, float2 *__restrict__ Y)
+// exponent of the largest component of a column held by a warp (biased exponents
+// in, this lane's largest): its size as a power of two; 0 for zero and non-finite
+// columns
+__device__ __forceinline__ int js_column_exponent(int e)
+{
+    for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    return e == 0 || e == 0x7FF ? 0 : min(max(e - 1023, -1000), 1000);
+}
+__device__ __forceinline__ int js_biased_exponent(double2 v)
+{
+    return max((__double2hiint(v.x) >> 20) & 0x7FF, (__double2hiint(v.y) >> 20) & 0x7FF);
+}
+
+// Y (N x N FP32) = R's first N rows in the FP32 Jacobi's units, M = R D^-1, E the
+// exponents of D.  A warp per column.
+__global__ void js_init_kernel(int ld, int N, const double2 *__restrict__ R, float2 *__restrict__ Y,
+                               double2 *__restrict__ M, int *__restrict__ E)
+{
+    const int f = blockIdx.y, lane = threadIdx.x & 31, j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (j >= N) return;
+    R += (size_t)f * ld * N;
+    const double sc = js_scale(R);
+    R += (size_t)j * ld;
+    Y += ((size_t)f * N + j) * N;
+    M += ((size_t)f * N + j) * N;
+    int e = 0;
+    for (int i = lane; i < N; i += 32) {
+        const double2 v = R[i];
+        Y[i] = make_float2((float)(v.x * sc), (float)(v.y * sc));
+        e = max(e, js_biased_exponent(v));
+    }
+    e = js_column_exponent(e);
+    const double d = ldexp(1.0, -e);
+    for (int i = lane; i < N; i += 32) M[i] = zscale(R[i], d);
+    if (lane == 0) E[(size_t)f * N + j] = e;
+}
+
+// J = D X D^-1, Jt = D^-1 X D (both from the FP32 X)
+__global__ void js_widen_kernel(int N, const float2 *__restrict__ X, const int *__restrict__ E,
+                                double2 *__restrict__ J, double2 *__restrict__ Jt)
 {
     const int f = blockIdx.y;
-    R += (size_t)f * ld * N;
-    Y += (size_t)f * N * N;
-    const double sc = js_scale(R);
+    const size_t o = (size_t)f * N * N;
+    E += (size_t)f * N;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N * N; e += gridDim.x * blockDim.x) {
-        const int c = e / N, r = e - c * N;
-        const double2 v = R[r + (size_t)c * ld];
-        Y[e] = make_float2((float)(v.x * sc), (float)(v.y * sc));
+        const int c = e / N, r = e - c * N, s = min(max(E[r] - E[c], -1000), 1000);
+        const double2 v = make_double2((double)X[o + e].x, (double)X[o + e].y);
+        J[o + e] = zscale(v, __hiloint2double((1023 + s) << 20, 0));
+        Jt[o + e] = zscale(v, __hiloint2double((1023 - s) << 20, 0));
     }
-}
-
-__global__ void js_widen_kernel(size_t count, const float2 *__restrict__ X, double2 *__restrict__ J)
-{
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < count; e += (size_t)gridDim.x * blockDim.x)
-        J[e] = make_double2((double)X[e].x, (double)X[e].y);
 }
 
 __device__ __forceinline__ double js_block_sum(double v, double *red)
@@ -102,8 +133,8 @@ __device__ __forceinline__ double js_block_sum(double v, double *red)
     return t;
 }
 
-// E = J^H J -> D = I - E; a bin whose |D| is too large (or not a number) gets
-// J = I, D = 0.  One CTA per bin.
+// E = D J^H J D^-1 -> I - E; a bin where that is too large (or not a number) gets
+// J = I, E = 0.  One CTA per bin.
 __global__ void __launch_bounds__(JS_THREADS) js_defect_kernel(int N, double2 *E, double2 *J)
 {
     __shared__ double red[JS_THREADS / 32];
@@ -144,23 +175,18 @@ __device__ __forceinline__ double js_rcp(double x)
 }
 
 // Columns scaled by powers of two to a largest component in [1, 2): X <- X D^-1,
-// E (+)= the exponents of D.  A warp per column.
-__global__ void js_normalize_kernel(int N, int first, double2 *__restrict__ X, int *__restrict__ E)
+// E += the exponents of D.  A warp per column.
+__global__ void js_normalize_kernel(int N, double2 *__restrict__ X, int *__restrict__ E)
 {
     const int f = blockIdx.y, lane = threadIdx.x & 31, j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (j >= N) return;
     X += ((size_t)f * N + j) * N;
-    int e = 0;   // biased exponent of the largest component
-    for (int i = lane; i < N; i += 32) {
-        const double2 v = X[i];
-        const int ex = (int)((__double_as_longlong(v.x) >> 52) & 0x7FF), ey = (int)((__double_as_longlong(v.y) >> 52) & 0x7FF);
-        e = max(e, max(ex, ey));
-    }
-    for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
-    e = e == 0 || e == 0x7FF ? 0 : min(max(e - 1023, -1000), 1000);   // zero and non-finite columns stay
+    int e = 0;
+    for (int i = lane; i < N; i += 32) e = max(e, js_biased_exponent(X[i]));
+    e = js_column_exponent(e);
     const double sc = ldexp(1.0, -e);
     for (int i = lane; i < N; i += 32) X[i] = zscale(X[i], sc);
-    if (lane == 0) E[(size_t)f * N + j] = (first ? 0 : E[(size_t)f * N + j]) + e;
+    if (lane == 0) E[(size_t)f * N + j] += e;
 }
 
 // X <- X D
@@ -173,10 +199,11 @@ __global__ void js_unscale_kernel(int N, double2 *__restrict__ X, const int *__r
     for (int i = lane; i < N; i += 32) X[i] = zscale(X[i], sc);
 }
 
-// G = (M D^-1)^H (M D^-1) -> D T D^-1 in place: T_ij = (D G D)_ij / ((D G D)_jj -
-// (D G D)_ii) where |T_ij| <= theta, the largest of 5e-2, 1e-2 .. 1e-7 that keeps
-// |T|_F <= limit, else 0.  T is exactly anti-Hermitian: each pair is computed
-// once.  One CTA per bin.
+// G = (M D^-1)^H (M D^-1) -> D T D^-1 in place, T_ij = (D G D)_ij / ((D G D)_jj -
+// (D G D)_ii) anti-Hermitian (each pair is computed once).  The larger of the pair's
+// two entries, t = G_ij max(d_i, d_j)^2 / ((D G D)_jj - (D G D)_ii), is kept where
+// |t| <= theta, the largest of 5e-2, 1e-2 .. 1e-7 with |D T D^-1|_F <= limit; the
+// other is -conj(t) times the squared ratio of the sizes.  One CTA per bin.
 constexpr int JS_NT = 7;
 __host__ __device__ constexpr float js_theta2(int q)
 {
@@ -212,7 +239,7 @@ __global__ void __launch_bounds__(JS_THREADS) js_rotation_kernel(int N, float li
         const int j = e / N, i = e - j * N;
         if (i >= j) continue;
         const double2 g = G[e];
-        const double q = js_rcp(js_g[j] - js_g[i]) * w[i] * w[j];
+        const double d = fmax(w[i], w[j]), q = js_rcp(js_g[j] - js_g[i]) * (d * d);
         const double2 t = make_double2(g.x * q, g.y * q);
         const float m = size2(t);
         // a zero gap, a NaN and an infinity fail every comparison
@@ -248,9 +275,12 @@ __global__ void __launch_bounds__(JS_THREADS) js_rotation_kernel(int N, float li
         }
         double2 t = G[e];
         if (!(size2(t) <= keep)) t = make_double2(0.0, 0.0);
-        const double u = w[i] * wi[j], v = w[j] * wi[i];
-        G[e] = zscale(t, u);
-        G[j + (size_t)i * N] = make_double2(-t.x * v, t.y * v);
+        const bool up = w[i] >= w[j];
+        const double u = up ? w[j] * wi[i] : w[i] * wi[j];
+        const double2 small = zscale(t, u * u);
+        G[e] = up ? t : small;
+        const double2 o = up ? small : t;
+        G[j + (size_t)i * N] = make_double2(-o.x, o.y);
     }
 }
 
@@ -302,73 +332,73 @@ int jacobi_precondition_batched(ia_context *ctx, int N, const double2 *R, int ld
     const size_t want = (count + 255) / 256, cap = (size_t)ctx->sm_count * 8;
     const int flat = (int)(want < cap ? want : cap);
     // C = op(A) B + beta C, N x N
-    auto prod = [&](Op opa, const double2 *A, int lda, const double2 *B, double beta, double2 *C) {
-        return zgemm_tc(ctx, opa, OP_N, N, N, N, 1.0, A, lda, (long long)lda * N, B, N, nn, beta, C, N, nn, batch, info,
-                        cur);
+    auto prod = [&](Op opa, const double2 *A, const double2 *B, double beta, double2 *C) {
+        return zgemm_tc(ctx, opa, OP_N, N, N, N, 1.0, A, N, nn, B, N, nn, beta, C, N, nn, batch, info, cur);
     };
     auto combine = [&](double a, const double2 *X, double b, const double2 *Z, double2 *W) -> int {
         js_combine_kernel<<<flat, 256, 0, ctx->stream>>>(count, a, X, b, Z, W);
         IA_LAUNCH_CHECK(ctx);
         return IA_OK;
     };
-    js_init_kernel<<<grid, 256, 0, ctx->stream>>>(ldr, N, R, Y);
+    js_init_kernel<<<cols, 256, 0, ctx->stream>>>(ldr, N, R, Y, M, E);
     IA_LAUNCH_CHECK(ctx);
     if ((st = jacobi_start_batched(ctx, N, Y, Y + count, batch, JS_FP32_SWEEPS, cur))) return st;
-    js_widen_kernel<<<flat, 256, 0, ctx->stream>>>(count, Y + count, J);
+    js_widen_kernel<<<grid, 256, 0, ctx->stream>>>(N, Y + count, E, J, P);
     IA_LAUNCH_CHECK(ctx);
-    // J to its polar factor (M holds the product's second operand), M = R J
-    if ((st = prod(OP_C, J, N, J, 0.0, D))) return st;
+    // J to its polar factor, M = R J
+    double2 *S = reinterpret_cast<double2 *>(Y);   // (Y and J in FP32: N^2 FP64 pairs)
+    if ((st = prod(OP_C, P, J, 0.0, D))) return st;
     js_defect_kernel<<<batch, JS_THREADS, 0, ctx->stream>>>(N, D, J);
     IA_LAUNCH_CHECK(ctx);
-    if ((st = prod(OP_N, D, N, D, 0.0, Q))) return st;
+    if ((st = prod(OP_N, D, D, 0.0, Q))) return st;
     if ((st = combine(0.5, D, 0.375, Q, P))) return st;
-    if ((st = combine(0.3125, D, 35.0 / 128.0, Q, M))) return st;
-    if ((st = prod(OP_N, Q, N, M, 1.0, P))) return st;
-    if ((st = prod(OP_N, J, N, P, 1.0, J))) return st;
-    if ((st = prod(OP_N, R, ldr, J, 0.0, M))) return st;
+    if ((st = combine(0.3125, D, 35.0 / 128.0, Q, S))) return st;
+    if ((st = prod(OP_N, Q, S, 1.0, P))) return st;
+    if ((st = prod(OP_N, J, P, 1.0, J))) return st;
+    if ((st = prod(OP_N, M, J, 0.0, M))) return st;
     const size_t nsm = sizeof(double) * (size_t)N;
     // T of M, on M with its columns scaled
-    auto rotation = [&](float limit, int first) -> int {
-        js_normalize_kernel<<<cols, 256, 0, ctx->stream>>>(N, first, M, E);
+    auto rotation = [&](float limit) -> int {
+        js_normalize_kernel<<<cols, 256, 0, ctx->stream>>>(N, M, E);
         IA_LAUNCH_CHECK(ctx);
-        if ((st = prod(OP_C, M, N, M, 0.0, D))) return st;
+        if ((st = prod(OP_C, M, M, 0.0, D))) return st;
         js_rotation_kernel<<<batch, JS_THREADS, 3 * nsm, ctx->stream>>>(N, limit, E, D);
         IA_LAUNCH_CHECK(ctx);
         return IA_OK;
     };
     // first step: p = (I - T^2)^(-1/2) - I to (T^2)^5, P = T + p + T p
-    if ((st = rotation(JS_MAX_T1, 1))) return st;
+    if ((st = rotation(JS_MAX_T1))) return st;
     {
         // D = T, Q = T^2, J = T^4, P = T^6, then P = 5/16 Q + 35/128 J + 63/256 P
-        double2 *T = D, *S = reinterpret_cast<double2 *>(Y);   // (Y and J in FP32: N^2 FP64 pairs)
-        if ((st = prod(OP_N, T, N, T, 0.0, Q))) return st;
-        if ((st = prod(OP_N, Q, N, Q, 0.0, J))) return st;
-        if ((st = prod(OP_N, Q, N, J, 0.0, P))) return st;
+        double2 *T = D;
+        if ((st = prod(OP_N, T, T, 0.0, Q))) return st;
+        if ((st = prod(OP_N, Q, Q, 0.0, J))) return st;
+        if ((st = prod(OP_N, Q, J, 0.0, P))) return st;
         if ((st = combine(35.0 / 128.0, J, 63.0 / 256.0, P, P))) return st;
         if ((st = combine(5.0 / 16.0, Q, 1.0, P, P))) return st;
         if ((st = combine(0.5, Q, 0.375, J, S))) return st;
-        if ((st = prod(OP_N, J, N, P, 1.0, S))) return st;      // p
+        if ((st = prod(OP_N, J, P, 1.0, S))) return st;      // p
         if ((st = combine(1.0, T, 1.0, S, P))) return st;
-        if ((st = prod(OP_N, T, N, S, 1.0, P))) return st;
-        if ((st = prod(OP_N, M, N, P, 1.0, M))) return st;
+        if ((st = prod(OP_N, T, S, 1.0, P))) return st;
+        if ((st = prod(OP_N, M, P, 1.0, M))) return st;
     }
     // second step: P = T + T^2 / 2 + T^2 (T / 2 + 3 T^2 / 8)
-    if ((st = rotation(JS_MAX_T2, 0))) return st;
-    if ((st = prod(OP_N, D, N, D, 0.0, Q))) return st;
+    if ((st = rotation(JS_MAX_T2))) return st;
+    if ((st = prod(OP_N, D, D, 0.0, Q))) return st;
     if ((st = combine(0.5, D, 0.375, Q, J))) return st;
     if ((st = combine(1.0, D, 0.5, Q, P))) return st;
-    if ((st = prod(OP_N, Q, N, J, 1.0, P))) return st;
-    if ((st = prod(OP_N, M, N, P, 1.0, M))) return st;
+    if ((st = prod(OP_N, Q, J, 1.0, P))) return st;
+    if ((st = prod(OP_N, M, P, 1.0, M))) return st;
     // third step: P = T + T^2 / 2
-    if ((st = rotation(JS_MAX_T3, 0))) return st;
-    if ((st = prod(OP_N, D, N, D, 0.0, Q))) return st;
+    if ((st = rotation(JS_MAX_T3))) return st;
+    if ((st = prod(OP_N, D, D, 0.0, Q))) return st;
     if ((st = combine(1.0, D, 0.5, Q, P))) return st;
-    if ((st = prod(OP_N, M, N, P, 1.0, M))) return st;
+    if ((st = prod(OP_N, M, P, 1.0, M))) return st;
     js_unscale_kernel<<<cols, 256, 0, ctx->stream>>>(N, M, E);
     IA_LAUNCH_CHECK(ctx);
     // sweeps over the pairs above the test
     for (int it = 0; it < JS_FLAG_SWEEPS; ++it) {
-        if ((st = prod(OP_C, M, N, M, 0.0, D))) return st;
+        if ((st = prod(OP_C, M, M, 0.0, D))) return st;
         js_flags_kernel<<<batch, JS_THREADS, nsm, ctx->stream>>>(N, jacobi_tol_fp64(N), D, flags, done);
         IA_LAUNCH_CHECK(ctx);
         if ((st = jacobi_flagged_batched(ctx, N, M, batch, done, flags))) return st;

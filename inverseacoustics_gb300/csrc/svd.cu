@@ -61,7 +61,7 @@ __device__ __forceinline__ bool jacobi_rotation(R a, R b, T g, R tol, R &c, T &s
 }
 
 // jacobi_rotation for a start whose columns span more than FP32's squares can
-// (norms down to 1e-17 of the largest): the modulus of g from scaled parts, so
+// (norms down to 1e-33 of the largest): the modulus of g from scaled parts, so
 // that the rotation is unitary whatever g's size, and no rotation with a column
 // whose squared norm nears the underflow limit (an iteration in FP64 follows)
 __device__ __forceinline__ bool jacobi_rotation_start(float a, float b, float2 g, float tol, float &c, float2 &sp,
