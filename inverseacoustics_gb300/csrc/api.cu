@@ -1031,7 +1031,6 @@ static int fp64_fallback(ia_context *ctx, const ia_config *cfg, int F, int *d_in
     }
     if (!st && !fp64.empty()) {
         const ia_config rc = fp64_config(cfg);
-        const PlainFp64 plain(ctx, true);
         st = redo_bins(ctx, fp64, d_info, ins, outs, redo, &rc);
     }
     if (!st) ctx->last_fallback = (int)(retry.size() + fp64.size());

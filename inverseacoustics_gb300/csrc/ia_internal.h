@@ -38,8 +38,9 @@ namespace ia {
 int ensure_side_stream(ia_context *ctx);
 
 // Scope of an FP64 solve that keeps the plain operation order (FP64 GEMM
-// updates and products, Jacobi from the pivoted R): the IBEM inversion and the
-// FP64 solution of a mixed call's flagged bins.  In a bin whose GCV minimum
+// updates and products, Jacobi from the pivoted R): the IBEM inversion, whether
+// called in FP64 or for the bins that a mixed call hands to it (every entry point's
+// mixed call returns such bins as its FP64 call does).  In a bin whose GCV minimum
 // sits at the bottom of its grid (0.6 % of the sphere's bins at 30 dB:
 // lambda ~ 1e-10 s_1) the solution carries the operator's and the
 // decomposition's rounding times s_1 / lambda, so only the same operations
