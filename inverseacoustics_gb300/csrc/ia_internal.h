@@ -304,8 +304,9 @@ int gcv_beta_batched(ia_context *ctx, int m, int p, int batch, const double *s, 
 // of A^H when n > m, one-sided Jacobi on R with U^H b carried as extra rows,
 // GCV / Tikhonov, x = Q [U_R (phi .* beta); 0].
 size_t wide_solve_ws_bytes(int m, int n, int nrhs, int batch);
-// what the FP64 solve uses on top of that for a preconditioned Jacobi, where
-// the caller's scratch has it
+// the FP64 solve runs the start of the Jacobi (jstart.cu), and needs
+// wide_start_ws_bytes on top of that
+inline bool wide_started(const ia_context *ctx, int m) { return !ctx->plain_fp64 && jacobi_precondition_ok(m); }
 size_t wide_start_ws_bytes(int m, int batch);
 int wide_solve_batched(ia_context *ctx, int m, int n, int batch, const double2 *A, bool transposed, int nrhs,
                        const double2 *b, const ia_config *cfg, double2 *x, double *lambda, double *s_out, int *info,

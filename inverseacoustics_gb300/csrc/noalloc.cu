@@ -70,11 +70,29 @@ extern "C" int ia_solve_batch_noalloc(ia_context *ctx, int m, int n, int F, cons
     int st = noalloc_scratch(&scratch);
     if (st) return st;
     IA_CUDA_TRY(cudaMemsetAsync(d_info, 0, sizeof(int) * (size_t)F, ctx->stream));
-    WsCursor cur{(char *)scratch, 0, (size_t)IA_NOALLOC_SCRATCH_BYTES};
+    // Operators whose Jacobi start fits with one bin take it for every bin, as many
+    // bins at a time as fit with it; the others take the plain order.  The size
+    // decides, not F: a bin's digits do not depend on the bins beside it.
+    auto group_bytes = [&](int g) { return wide_solve_ws_bytes(m, n, nrhs, g) + wide_start_ws_bytes(m, g); };
+    const bool start = wide_started(ctx, m) && group_bytes(1) <= (size_t)IA_NOALLOC_SCRATCH_BYTES;
+    const PlainFp64 plain(ctx, !start);
+    int g = F;
+    if (start) {
+        while (group_bytes(g) > (size_t)IA_NOALLOC_SCRATCH_BYTES) --g;
+        const int groups = (F + g - 1) / g;
+        g = (F + groups - 1) / groups;
+    }
     const int prev = ctx->no_tune;
     ctx->no_tune = 1;
-    st = wide_solve_batched(ctx, m, n, F, (const double2 *)d_H, false, nrhs, (const double2 *)d_b, cfg,
-                            (double2 *)d_x, d_lambda, d_s, d_info, cur);
+    for (int f0 = 0; f0 < F && !st; f0 += g) {
+        const int nf = F - f0 < g ? F - f0 : g;
+        const size_t o = (size_t)f0 * nrhs;
+        WsCursor cur{(char *)scratch, 0, (size_t)IA_NOALLOC_SCRATCH_BYTES};
+        st = wide_solve_batched(ctx, m, n, nf, (const double2 *)d_H + (size_t)f0 * m * n, false, nrhs,
+                                (const double2 *)d_b + o * m, cfg, (double2 *)d_x + o * n,
+                                d_lambda ? d_lambda + o : nullptr, d_s ? d_s + (size_t)f0 * m : nullptr, d_info + f0,
+                                cur);
+    }
     ctx->no_tune = prev;
     return st;
 }

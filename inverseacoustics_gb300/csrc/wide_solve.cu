@@ -777,9 +777,10 @@ int wide_solve_batched(ia_context *ctx, int m, int n, int batch, const double2 *
         build_rh_aug_kernel<<<dim3(blocks, batch), 256, 0, ctx->stream>>>(N, Mr, nrhs, Y, perm, unmoved ? 1 : 0, b, Rg);
         IA_LAUNCH_CHECK(ctx);
     }
-    // the Jacobi starts from R^H K (jstart.cu), which as a rule passes its test
-    const size_t extra = wide_start_ws_bytes(m, batch);
-    const bool started = !ctx->plain_fp64 && extra && cur.off + extra <= cur.cap;
+    // the Jacobi starts from R^H K (jstart.cu), which as a rule passes its test;
+    // by the operator's size alone, so that a bin's digits do not depend on the
+    // scratch or on the batch
+    const bool started = wide_started(ctx, m);
     int *done = nullptr;
     if (started) {
         double2 *M = cur.take<double2>((size_t)N * N * batch);
