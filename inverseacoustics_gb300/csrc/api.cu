@@ -25,24 +25,30 @@ int cuda_status(cudaError_t e)
     return IA_ERR_CUDA;
 }
 
-int ws_reserve(ia_context *ctx, size_t bytes)
+int ws_reserve(ia_context *ctx, size_t bytes, size_t least)
 {
+    if (least == 0 || least > bytes) least = bytes;
     if (bytes <= ctx->ws_bytes) return IA_OK;
-    if (ctx->capturing) return IA_ERR_CAPTURE;
+    if (ctx->capturing) return least <= ctx->ws_bytes ? IA_OK : IA_ERR_CAPTURE;
     if (ctx->ws) {
         cudaError_t e = cudaFreeAsync(ctx->ws, ctx->stream);
         ctx->ws = nullptr;
         ctx->ws_bytes = 0;
         if (e != cudaSuccess) return cuda_status(e);
     }
-    size_t grow = bytes + bytes / 8;
-    cudaError_t e = cudaMallocAsync(&ctx->ws, grow, ctx->stream);
-    if (e != cudaSuccess) {
+    // with room to grow; what was asked for; what the call can do with
+    cudaError_t e = cudaSuccess;
+    for (size_t size : {bytes + bytes / 8, bytes, least}) {
+        e = cudaMallocAsync(&ctx->ws, size, ctx->stream);
+        if (e == cudaSuccess) {
+            ctx->ws_bytes = size;
+            return IA_OK;
+        }
         ctx->ws = nullptr;
-        return cuda_status(e);
+        cudaGetLastError();   // the failure is this call's alone
+        if (e != cudaErrorMemoryAllocation) break;
     }
-    ctx->ws_bytes = grow;
-    return IA_OK;
+    return cuda_status(e);
 }
 
 // ---- built-in quadrature rules ------------------------------------------
@@ -668,12 +674,16 @@ int ia_ibem_assemble_batch(ia_context *ctx, const ia_mesh *mesh, int l, const do
     const size_t gbytes = mixed ? ibem_geom_own_bytes(mesh, mesh->m + n_ch + l, F) : 0;
     if (gbytes) {
         const int st = ws_reserve(ctx, gbytes);
-        if (st) return st;
-        G = reinterpret_cast<float2 *>(ctx->ws);
+        if (st && st != IA_ERR_ALLOC) return st;
+        if (!st) G = reinterpret_cast<float2 *>(ctx->ws);   // no memory for it: the inline form, the same bits
     }
     return ibem_rows(ctx, mesh, l, d_mics, n_ch, d_cp, F, d_k, cfg->c, cfg->rho, (double2 *)d_At, (double2 *)d_Bt,
                      (double2 *)d_Ahs_t, (double2 *)d_Bhs_t, mixed, false, G, gbytes);
 }
+
+// Every ..._ws_bytes below: `least` is what the call can do with where the device
+// has no more: slice planes and starts for a bin at a time, no geometry table of
+// its own.  The results are the same bits.
 
 // slice planes of the FP64 transfer's solver and products
 static size_t transfer_fp64_ws_bytes(int m, int l, int F)
@@ -723,6 +733,7 @@ struct GeomTable {
     float2 *p;
     bool build;
 };
+constexpr GeomTable no_geom_table{nullptr, true};   // the geometry inline
 
 // with_table: the transfer's workspace holds its own geometry table
 static size_t transfer_mixed_ws_bytes(const ia_mesh *mesh, int l, int F, const ia_config *cfg, bool with_table = true)
@@ -826,9 +837,11 @@ int ia_ibem_transfer_batch(ia_context *ctx, const ia_mesh *mesh, int l, const do
     if (!ctx || !mesh || !cfg || F < 1 || l < 1 || !d_mics || !d_k || !d_H || !d_info) return IA_ERR_ARG;
     const int m = mesh->m;
     const bool mixed = cfg->precision == IA_PREC_MIXED;
-    size_t need = ws_round(sizeof(double2) * (size_t)m * m * F) * 2 + ws_round(sizeof(int) * (size_t)m * F) +
-                  ws_round(sizeof(double2) * (size_t)m * l * F) * 2 + (mixed ? transfer_mixed_ws_bytes(mesh, l, F, cfg) : transfer_fp64_ws_bytes(m, l, F));
-    int st = ws_reserve(ctx, need);
+    const size_t base = ws_round(sizeof(double2) * (size_t)m * m * F) * 2 + ws_round(sizeof(int) * (size_t)m * F) +
+                        ws_round(sizeof(double2) * (size_t)m * l * F) * 2;
+    const size_t need = base + (mixed ? transfer_mixed_ws_bytes(mesh, l, F, cfg) : transfer_fp64_ws_bytes(m, l, F));
+    int st = ws_reserve(ctx, need, base + (mixed ? transfer_mixed_ws_bytes(mesh, l, F, cfg, false)
+                                                 : transfer_fp64_ws_bytes(m, l, 1)));
     if (!st) st = clear_info(ctx, d_info, F);
     if (st) return st;
     WsCursor cur{(char *)ctx->ws, 0, ctx->ws_bytes};
@@ -837,7 +850,9 @@ int ia_ibem_transfer_batch(ia_context *ctx, const ia_mesh *mesh, int l, const do
     int *ipiv = cur.take<int>((size_t)m * F);
     double2 *Ahs = cur.take<double2>((size_t)m * l * F);
     double2 *Ht = cur.take<double2>((size_t)m * l * F);
-    if (mixed) st = ibem_transfer_t_mixed(ctx, mesh, l, d_mics, F, d_k, cfg, At, Bt, ipiv, Ahs, Ht, d_info, cur);
+    if (mixed)
+        st = ibem_transfer_t_mixed(ctx, mesh, l, d_mics, F, d_k, cfg, At, Bt, ipiv, Ahs, Ht, d_info, cur, nullptr,
+                                   cur.cap < need ? &no_geom_table : nullptr);
     else st = ibem_transfer_t(ctx, mesh, l, d_mics, F, d_k, cfg, At, Bt, ipiv, Ahs, Ht, d_info, cur);
     if (st) return st;
     return ztranspose_batched(ctx, m, l, Ht, m, (long long)m * l, (double2 *)d_H, l, (long long)m * l, false, F);
@@ -1037,10 +1052,12 @@ static int fp64_fallback(ia_context *ctx, const ia_config *cfg, int F, int *d_in
     return st;
 }
 
-static size_t solve_ws_bytes(int m, int n, int F, int nrhs, const ia_config *cfg)
+static size_t solve_ws_bytes(const ia_context *ctx, int m, int n, int F, int nrhs, const ia_config *cfg,
+                             bool least = false)
 {
     if (use_mixed_wide(m, n, cfg)) return wide_solve_mixed_ws_bytes(m, n, nrhs, F);
-    if (m <= n) return wide_solve_ws_bytes(m, n, nrhs, F) + wide_start_ws_bytes(m, F);
+    if (m <= n)
+        return wide_solve_ws_bytes(m, n, nrhs, F) + (wide_started(ctx, m) ? wide_start_ws_bytes(m, F, least ? 1 : F) : 0);
     const int p = m < n ? m : n;
     const int M = m >= n ? m : n;
     return ws_round(sizeof(double2) * (size_t)M * p * F) + ws_round(sizeof(double2) * (size_t)p * p * F) +
@@ -1052,7 +1069,7 @@ int ia_solve_batch(ia_context *ctx, int m, int n, int F, const ia_complex *d_H, 
                    const ia_config *cfg, ia_complex *d_x, double *d_lambda, double *d_s, int *d_info)
 {
     if (!ctx || !cfg || m < 1 || n < 1 || F < 1 || nrhs < 1 || !d_H || !d_b || !d_x || !d_info) return IA_ERR_ARG;
-    int st = ws_reserve(ctx, solve_ws_bytes(m, n, F, nrhs, cfg));
+    int st = ws_reserve(ctx, solve_ws_bytes(ctx, m, n, F, nrhs, cfg), solve_ws_bytes(ctx, m, n, F, nrhs, cfg, true));
     if (!st) st = clear_info(ctx, d_info, F);
     if (st) return st;
     WsCursor cur{(char *)ctx->ws, 0, ctx->ws_bytes};
@@ -1069,16 +1086,15 @@ int ia_solve_batch(ia_context *ctx, int m, int n, int F, const ia_complex *d_H, 
         });
 }
 
-static size_t ibem_solve_ws_bytes(const ia_mesh *mesh, int l, int F, int nrhs, const ia_config *cfg,
-                                  bool with_table = true)
+// (in FP64 the plain order: no slice planes)
+static size_t ibem_solve_ws_bytes(const ia_context *ctx, const ia_mesh *mesh, int l, int F, int nrhs,
+                                  const ia_config *cfg, bool with_table, bool least = false)
 {
     const bool mixed = cfg->precision == IA_PREC_MIXED;
     const int m = mesh->m;
     return ws_round(sizeof(double2) * (size_t)m * m * F) * 2 + ws_round(sizeof(int) * (size_t)m * F) +
-           ws_round(sizeof(double2) * (size_t)m * l * F) * 2 +
-           (mixed ? solve_ws_bytes(l, m, F, nrhs, cfg) + transfer_mixed_ws_bytes(mesh, l, F, cfg, with_table)
-                  // the transfer's scratch is free again when the solve starts
-                  : std::max(solve_ws_bytes(l, m, F, nrhs, cfg), transfer_fp64_ws_bytes(m, l, F)));
+           ws_round(sizeof(double2) * (size_t)m * l * F) * 2 + solve_ws_bytes(ctx, l, m, F, nrhs, cfg, least) +
+           (mixed ? transfer_mixed_ws_bytes(mesh, l, F, cfg, with_table && !least) : 0);
 }
 
 // the whole IBEM pipeline for F bins on ctx->stream; ev_rows (if given) is
@@ -1129,10 +1145,16 @@ int ia_ibem_solve_batch(ia_context *ctx, const ia_mesh *mesh, int l, const doubl
     }
     const PlainFp64 plain(ctx, cfg->precision != IA_PREC_MIXED);
     const int Fp = F / parts;
-    const size_t need = ibem_solve_ws_bytes(mesh, l, Fp, nrhs, cfg, parts == 1);
+    size_t need = ibem_solve_ws_bytes(ctx, mesh, l, Fp, nrhs, cfg, parts == 1);
     const size_t gshared = parts > 1 && cfg->precision == IA_PREC_MIXED ? ibem_geom_bytes(mesh, m + l) : 0;
-    const size_t goff = ws_round(need * parts);
-    int st = ws_reserve(ctx, goff + gshared);
+    size_t goff = ws_round(need * parts);
+    const size_t want = goff + gshared, lneed = ibem_solve_ws_bytes(ctx, mesh, l, Fp, nrhs, cfg, false, true);
+    int st = ws_reserve(ctx, want, lneed * parts);
+    const bool table = ctx->ws_bytes >= want;
+    if (!table) {
+        need = lneed;
+        goff = 0;
+    }
     if (!st) st = clear_info(ctx, d_info, F);
     if (st) return st;
     const int p = l < m ? l : m;
@@ -1149,7 +1171,7 @@ int ia_ibem_solve_batch(ia_context *ctx, const ia_mesh *mesh, int l, const doubl
     if (parts == 1) {
         WsCursor cur{(char *)ctx->ws, 0, ctx->ws_bytes};
         st = ibem_solve_part(ctx, mesh, l, d_mics, F, d_k, nrhs, (const double2 *)d_p, cfg, (double2 *)d_x, d_lambda,
-                             d_s, d_info, cur, nullptr);
+                             d_s, d_info, cur, nullptr, table ? nullptr : &no_geom_table);
         return st ? st : fallback();
     }
     if ((st = ensure_side_stream(ctx))) return st;
@@ -1165,7 +1187,8 @@ int ia_ibem_solve_batch(ia_context *ctx, const ia_mesh *mesh, int l, const doubl
         ctx->stream = sq;
         ctx->tail_part = q + 1 == parts;
         WsCursor cur{(char *)ctx->ws + need * q, 0, need};
-        const GeomTable geom{reinterpret_cast<float2 *>((char *)ctx->ws + goff), q == 0};
+        const GeomTable geom = table ? GeomTable{reinterpret_cast<float2 *>((char *)ctx->ws + goff), q == 0}
+                                     : no_geom_table;
         st = ibem_solve_part(ctx, mesh, l, d_mics, Fp, d_k + f0, nrhs, (const double2 *)d_p + (size_t)f0 * nrhs * l,
                              cfg, (double2 *)d_x + (size_t)f0 * nrhs * m,
                              d_lambda ? d_lambda + (size_t)f0 * nrhs : nullptr, d_s ? d_s + (size_t)f0 * p : nullptr,
@@ -1191,8 +1214,9 @@ int ia_esm_solve_batch(ia_context *ctx, int l, int m, const double *d_mics, cons
 {
     if (!ctx || !cfg || l < 1 || m < 1 || F < 1 || nrhs < 1 || !d_mics || !d_src || !d_k || !d_p || !d_x || !d_info)
         return IA_ERR_ARG;
-    size_t need = ws_round(sizeof(double2) * (size_t)l * m * F) + solve_ws_bytes(l, m, F, nrhs, cfg);
-    int st = ws_reserve(ctx, need);
+    const size_t op = ws_round(sizeof(double2) * (size_t)l * m * F);
+    int st = ws_reserve(ctx, op + solve_ws_bytes(ctx, l, m, F, nrhs, cfg),
+                        op + solve_ws_bytes(ctx, l, m, F, nrhs, cfg, true));
     if (!st) st = clear_info(ctx, d_info, F);
     if (st) return st;
     WsCursor cur{(char *)ctx->ws, 0, ctx->ws_bytes};
@@ -1220,8 +1244,9 @@ int ia_hels_solve_batch(ia_context *ctx, int l, const double *d_pts, int n_sh, i
     if (!ctx || !cfg || l < 1 || n_sh < 0 || F < 1 || nrhs < 1 || !d_pts || !d_k || !d_p || !d_x || !d_info)
         return IA_ERR_ARG;
     const int nt = (n_sh + 1) * (n_sh + 1);
-    size_t need = ws_round(sizeof(double2) * (size_t)l * nt * F) + solve_ws_bytes(l, nt, F, nrhs, cfg);
-    int st = ws_reserve(ctx, need);
+    const size_t op = ws_round(sizeof(double2) * (size_t)l * nt * F);
+    int st = ws_reserve(ctx, op + solve_ws_bytes(ctx, l, nt, F, nrhs, cfg),
+                        op + solve_ws_bytes(ctx, l, nt, F, nrhs, cfg, true));
     if (!st) st = clear_info(ctx, d_info, F);
     if (st) return st;
     WsCursor cur{(char *)ctx->ws, 0, ctx->ws_bytes};
@@ -1257,7 +1282,8 @@ int ia_radiation_modes_batch(ia_context *ctx, int n, int F, const double *d_R, i
     if (!ctx || !cfg || n < 1 || F < 1 || nmodes < 1 || nmodes > n || !d_R || !d_lambda || !d_modes || !d_info ||
         cfg->mode_iters < 0 || cfg->mode_oversample < 0)
         return IA_ERR_ARG;
-    int st = ws_reserve(ctx, radiation_modes_ws_bytes(n, F, nmodes, cfg));
+    int st = ws_reserve(ctx, radiation_modes_ws_bytes(n, F, nmodes, cfg),
+                        radiation_modes_ws_bytes(n, F, nmodes, cfg, false, true));
     if (!st) st = clear_info(ctx, d_info, F);
     if (st) return st;
     WsCursor cur{(char *)ctx->ws, 0, ctx->ws_bytes};
@@ -1274,7 +1300,7 @@ int ia_esm_design_batch(ia_context *ctx, int l, int m, int F, int nrhs, const do
         return IA_ERR_ARG;
     const int ng = (d_grad_mics != nullptr) + (d_grad_retreat != nullptr) + (d_grad_loglam != nullptr);
     if (ng != 0 && ng != 3) return IA_ERR_ARG;
-    int st = ws_reserve(ctx, esm_design_ws_bytes(l, m, F, nrhs));
+    int st = ws_reserve(ctx, esm_design_ws_bytes(l, m, F, nrhs), esm_design_ws_bytes(l, m, F, nrhs, true));
     if (!st) st = clear_info(ctx, d_info, F);
     if (st) return st;
     WsCursor cur{(char *)ctx->ws, 0, ctx->ws_bytes};
@@ -1291,7 +1317,8 @@ static int bem_modes_entry(ia_context *ctx, const ia_mesh *mesh, int l, const do
         nmodes > mesh->m || !d_mics || !d_k || !d_Ur || !d_sr || !d_Hr || !d_info || cfg->mode_iters < 0 ||
         cfg->mode_oversample < 0)
         return IA_ERR_ARG;
-    int st = ws_reserve(ctx, bem_modes_ws_bytes(mesh, l, n_ch, F, nmodes, cfg, cplx));
+    int st = ws_reserve(ctx, bem_modes_ws_bytes(mesh, l, n_ch, F, nmodes, cfg, cplx),
+                        bem_modes_ws_bytes(mesh, l, n_ch, F, nmodes, cfg, cplx, true));
     if (!st) st = clear_info(ctx, d_info, F);
     if (st) return st;
     WsCursor cur{(char *)ctx->ws, 0, ctx->ws_bytes};

@@ -336,7 +336,8 @@ static int bem_slices(const ia_config *cfg)
     return cfg->gemm_slices < TC_SLICES_MAX ? cfg->gemm_slices + 1 : TC_SLICES_MAX;
 }
 
-size_t bem_modes_ws_bytes(const ia_mesh *mesh, int l, int n_ch, int F, int nm, const ia_config *cfg, bool cplx)
+size_t bem_modes_ws_bytes(const ia_mesh *mesh, int l, int n_ch, int F, int nm, const ia_config *cfg, bool cplx,
+                          bool least)
 {
     const size_t M = mesh->m, MT = M + n_ch, L = l, FF = F;
     size_t b = 4 * ws_round(16 * MT * M * FF) + 4 * ws_round(16 * M * L * FF) + ws_round(4 * M * FF) +
@@ -347,13 +348,18 @@ size_t bem_modes_ws_bytes(const ia_mesh *mesh, int l, int n_ch, int F, int nm, c
             const ComplexModeSub c = complex_mode_sub(cfg, mesh->m, nm);
             const size_t NR = c.nr;
             b += ws_round(32 * M * M * FF) + ws_round(16 * M * NR * FF) + ws_round(8 * NR * FF) +
-                 radiation_modes_ws_bytes(2 * mesh->m, F, c.nr, &c.cfg, true);
+                 radiation_modes_ws_bytes(2 * mesh->m, F, c.nr, &c.cfg, true, least);
         }
-    } else b += ws_round(8 * M * M * FF) + ws_round(8 * nm * FF) + radiation_modes_ws_bytes(mesh->m, F, nm, cfg, true);
-    if (cfg->precision == IA_PREC_MIXED) b += ws_round(ibem_geom_own_bytes(mesh, (int)(MT + L), F));   // assembly geometry
-    if (!bem_mixed_solve(cfg, n_ch))   // slice planes of the FP64 solver and products
-        b += std::max({zlu_ws_bytes(mesh->m, mesh->m, F), zgemm_tc_ws_bytes(l, mesh->m, mesh->m, F),
-                       zgemm_tc_ws_bytes(mesh->m > l ? mesh->m : l, nm, mesh->m, F)});
+    } else
+        b += ws_round(8 * M * M * FF) + ws_round(8 * nm * FF) +
+             radiation_modes_ws_bytes(mesh->m, F, nm, cfg, true, least);
+    if (cfg->precision == IA_PREC_MIXED && !least)
+        b += ws_round(ibem_geom_own_bytes(mesh, (int)(MT + L), F));   // assembly geometry
+    if (!bem_mixed_solve(cfg, n_ch)) {   // slice planes of the FP64 solver and products
+        const int fp = least ? 1 : F;
+        b += std::max({zlu_ws_bytes(mesh->m, mesh->m, fp), zgemm_tc_ws_bytes(l, mesh->m, mesh->m, fp),
+                       zgemm_tc_ws_bytes(mesh->m > l ? mesh->m : l, nm, mesh->m, fp)});
+    }
     if (bem_mixed_solve(cfg, n_ch)) {
         b += 2 * ws_round(8 * M * M * FF) + ws_round(16 * M * M * FF);
         if (tc_products_ok(bem_slices(cfg), mesh->m))
@@ -372,13 +378,13 @@ size_t bem_modes_ws_bytes(const ia_mesh *mesh, int l, int n_ch, int F, int nm, c
 // gemm_slices 0, as double-float CUDA-core GEMMs.  On exit Z (FP64, m x m) is
 // in At's storage.
 static int bem_mixed_z(ia_context *ctx, const ia_mesh *mesh, int l, const double *mics, int F, const double *k,
-                       const ia_config *cfg, double2 *At, double2 *Bt, double2 *A, double2 *B, double2 *Ahs_t,
-                       double2 *Bhs_t, double2 *Ahs, double2 *H, int *ipiv, int *info, WsCursor &cur)
+                       const ia_config *cfg, bool table, double2 *At, double2 *Bt, double2 *A, double2 *B,
+                       double2 *Ahs_t, double2 *Bhs_t, double2 *Ahs, double2 *H, int *ipiv, int *info, WsCursor &cur)
 {
     const int m = mesh->m;
     const long long mm = (long long)m * m, ml = (long long)m * l;
     int st;
-    const size_t gbytes = ibem_geom_own_bytes(mesh, m + l, F);
+    const size_t gbytes = table ? ibem_geom_own_bytes(mesh, m + l, F) : 0;
     float2 *G = gbytes ? cur.take<float2>(gbytes / sizeof(float2)) : nullptr;
     if (cur.off > cur.cap) return IA_ERR_ALLOC;
     if ((st = ibem_rows(ctx, mesh, l, mics, 0, nullptr, F, k, cfg->c, cfg->rho, At, Bt, Ahs_t, Bhs_t, true, true, G, gbytes)))
@@ -450,6 +456,8 @@ int bem_modes_batched(ia_context *ctx, const ia_mesh *mesh, int l, const double 
     const int m = mesh->m, mt = m + n_ch;
     int st;
     const long long mm = (long long)m * m, tm = (long long)mt * m, ml = (long long)m * l;
+    // (a geometry table where the whole workspace is there)
+    const bool table = cur.cap - cur.off >= bem_modes_ws_bytes(mesh, l, n_ch, F, nm, cfg, cplx);
     double2 *At = cur.take<double2>(tm * F), *Bt = cur.take<double2>(tm * F);
     double2 *A = cur.take<double2>(tm * F), *B = cur.take<double2>(tm * F);
     double2 *Ahs_t = cur.take<double2>(ml * F), *Bhs_t = cur.take<double2>(ml * F);
@@ -460,12 +468,13 @@ int bem_modes_batched(ia_context *ctx, const ia_mesh *mesh, int l, const double 
     const bool mixed_z = bem_mixed_solve(cfg, n_ch);
     double2 *Z = At;
     if (mixed_z) {
-        if ((st = bem_mixed_z(ctx, mesh, l, mics, F, k, cfg, At, Bt, A, B, Ahs_t, Bhs_t, Ahs, H, ipiv, info, cur)))
+        if ((st = bem_mixed_z(ctx, mesh, l, mics, F, k, cfg, table, At, Bt, A, B, Ahs_t, Bhs_t, Ahs, H, ipiv, info,
+                              cur)))
             return st;
     } else {
         // collocation rows, then A, B (mt x m), A_hs, B_hs (l x m) column-major
         const bool df = cfg->precision == IA_PREC_MIXED;
-        const size_t gbytes = df ? ibem_geom_own_bytes(mesh, mt + l, F) : 0;
+        const size_t gbytes = df && table ? ibem_geom_own_bytes(mesh, mt + l, F) : 0;
         float2 *G = gbytes ? cur.take<float2>(gbytes / sizeof(float2)) : nullptr;
         if (cur.off > cur.cap) return IA_ERR_ALLOC;
         if ((st = ibem_rows(ctx, mesh, l, mics, n_ch, cp, F, k, cfg->c, cfg->rho, At, Bt, Ahs_t, Bhs_t, df, false, G, gbytes)))

@@ -110,7 +110,8 @@ int cuda_status(cudaError_t e);
     } while (0)
 
 // workspace carving: returns IA_OK / IA_ERR_ALLOC
-int ws_reserve(ia_context *ctx, size_t bytes);
+// (`bytes`, or where the device has no more at least `least`; 0: bytes)
+int ws_reserve(ia_context *ctx, size_t bytes, size_t least = 0);
 struct WsCursor {
     char *base;
     size_t off, cap;
@@ -305,9 +306,10 @@ int gcv_beta_batched(ia_context *ctx, int m, int p, int batch, const double *s, 
 // GCV / Tikhonov, x = Q [U_R (phi .* beta); 0].
 size_t wide_solve_ws_bytes(int m, int n, int nrhs, int batch);
 // the FP64 solve runs the start of the Jacobi (jstart.cu), and needs
-// wide_start_ws_bytes on top of that
+// wide_start_ws_bytes on top of that (group: bins that it works through at a time;
+// as many as the scratch holds, at least one)
 inline bool wide_started(const ia_context *ctx, int m) { return !ctx->plain_fp64 && jacobi_precondition_ok(m); }
-size_t wide_start_ws_bytes(int m, int batch);
+size_t wide_start_ws_bytes(int m, int batch, int group);
 int wide_solve_batched(ia_context *ctx, int m, int n, int batch, const double2 *A, bool transposed, int nrhs,
                        const double2 *b, const ia_config *cfg, double2 *x, double *lambda, double *s_out, int *info,
                        WsCursor &cur);
@@ -377,12 +379,13 @@ int sinc_resistance_batched(ia_context *ctx, int n, const double *x, int F, cons
                             double rho, double *R);
 // leading eigenpairs of the symmetric R, or (gram) of R R^T for a general R:
 // left singular vectors, lambda = squared singular values
-size_t radiation_modes_ws_bytes(int n, int F, int nm, const ia_config *cfg, bool gram = false);
+size_t radiation_modes_ws_bytes(int n, int F, int nm, const ia_config *cfg, bool gram = false, bool least = false);
 int radiation_modes_batched(ia_context *ctx, int n, int F, const double *R, int nm, const ia_config *cfg,
                             double *lambda, double *modes, int *info, WsCursor &cur, bool gram = false);
 // BEM radiation modes (bem_modes.cu)
 // (cplx: Ur is double2 m x nm per frequency, modes of G Z; else double, of Re(G Z))
-size_t bem_modes_ws_bytes(const ia_mesh *mesh, int l, int n_ch, int F, int nm, const ia_config *cfg, bool cplx);
+size_t bem_modes_ws_bytes(const ia_mesh *mesh, int l, int n_ch, int F, int nm, const ia_config *cfg, bool cplx,
+                          bool least = false);
 int bem_modes_batched(ia_context *ctx, const ia_mesh *mesh, int l, const double *mics, int n_ch, const double *cp,
                       int F, const double *k, int nm, const ia_config *cfg, bool cplx, void *Ur, double *sr,
                       double2 *Hr, double2 *Pr, int *info, WsCursor &cur);
@@ -395,7 +398,7 @@ int admm_batched(ia_context *ctx, int l, int m, int F, const double2 *H, int nrh
                  int *info, WsCursor &cur);
 
 // ---- differentiable ESM design (adjoint.cu); gm == nullptr: forward only
-size_t esm_design_ws_bytes(int l, int m, int F, int R);
+size_t esm_design_ws_bytes(int l, int m, int F, int R, bool least = false);
 int esm_design_batched(ia_context *ctx, int l, int m, int F, int R, const double *mics, const double *surf,
                        const double *retreat, const double *k, const double *loglam, const double2 *q,
                        const double2 *noise, double *err, double *gm, double *gd, double *gl, int *info,

@@ -73,7 +73,7 @@ extern "C" int ia_solve_batch_noalloc(ia_context *ctx, int m, int n, int F, cons
     // Operators whose Jacobi start fits with one bin take it for every bin, as many
     // bins at a time as fit with it; the others take the plain order.  The size
     // decides, not F: a bin's digits do not depend on the bins beside it.
-    auto group_bytes = [&](int g) { return wide_solve_ws_bytes(m, n, nrhs, g) + wide_start_ws_bytes(m, g); };
+    auto group_bytes = [&](int g) { return wide_solve_ws_bytes(m, n, nrhs, g) + wide_start_ws_bytes(m, g, g); };
     const bool start = wide_started(ctx, m) && group_bytes(1) <= (size_t)IA_NOALLOC_SCRATCH_BYTES;
     const PlainFp64 plain(ctx, !start);
     int g = F;

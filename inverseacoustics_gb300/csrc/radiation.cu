@@ -972,10 +972,10 @@ __global__ void mode_sign_kernel(int n, int nm, double *__restrict__ X, const do
     if (threadIdx.x == 0 && info && bad) info[f] |= IA_INFO_NONFINITE;
 }
 
-size_t radiation_modes_ws_bytes(int n, int F, int nm, const ia_config *cfg, bool gram)
+// workspace of a group of F bins
+static size_t modes_group_bytes(int n, int F, int nm, const ia_config *cfg, bool gram)
 {
     const size_t b = (size_t)min(n, nm + max(0, cfg->mode_oversample));
-    F = modes_group(n, (int)b, F, cfg, gram);
     const size_t nb = (size_t)n * b * F, bb = b * b * F;
     size_t s = 4 * ws_round(8 * nb) + ws_round(8 * b * F) + ws_round(8 * bb) + 4 * ws_round(16 * bb) +
                ws_round(8 * b * F) + ws_round(8 * b * (size_t)nm * F);
@@ -983,6 +983,12 @@ size_t radiation_modes_ws_bytes(int n, int F, int nm, const ia_config *cfg, bool
         s += ws_round(4 * (size_t)n * n * F) + 3 * ws_round(4 * nb) + ws_round(4 * b * F);
     if (modes_tc(n, cfg)) s += modes_op_bytes(n, (int)b, F, gram);
     return s + 4096;
+}
+
+size_t radiation_modes_ws_bytes(int n, int F, int nm, const ia_config *cfg, bool gram, bool least)
+{
+    const int g = modes_group(n, min(n, nm + max(0, cfg->mode_oversample)), F, cfg, gram);
+    return modes_group_bytes(n, least && modes_tc(n, cfg) ? 1 : g, nm, cfg, gram);
 }
 
 // one group of bins
@@ -1111,7 +1117,9 @@ int radiation_modes_batched(ia_context *ctx, int n, int F, const double *R, int 
                             double *lambda, double *modes, int *info, WsCursor &cur, bool gram)
 {
     const int b = min(n, nm + max(0, cfg->mode_oversample));
-    const int fg = modes_group(n, b, F, cfg, gram);
+    int fg = modes_group(n, b, F, cfg, gram);
+    // a device without the memory: what fits
+    while (modes_tc(n, cfg) && fg > 1 && cur.off + modes_group_bytes(n, fg, nm, cfg, gram) > cur.cap) fg = (fg + 1) / 2;
     for (int f0 = 0; f0 < F; f0 += fg) {
         WsCursor c = cur;
         const int st = radiation_modes_group(ctx, n, min(fg, F - f0), R + (size_t)f0 * n * n, nm, cfg,

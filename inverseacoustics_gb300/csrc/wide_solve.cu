@@ -729,11 +729,9 @@ size_t wide_solve_ws_bytes(int m, int n, int nrhs, int batch)
            ws_round(16 * R * N * F) * 2 + ws_round(16 * N * N * F) + 2 * ws_round(4 * N * F) + 2048;
 }
 
-size_t wide_start_ws_bytes(int m, int batch)
+size_t wide_start_ws_bytes(int m, int batch, int group)
 {
-    if (!jacobi_precondition_ok(m)) return 0;
-    return ws_round(16 * (size_t)m * m * batch) + ws_round(4 * (size_t)batch) + jacobi_precondition_ws_bytes(m, batch) +
-           512;
+    return ws_round(4 * (size_t)batch) + jacobi_precondition_ws_bytes(m, group) + 512;
 }
 
 // FP64 wide solve (Drmac-Veselic preconditioned one-sided Jacobi):
@@ -783,9 +781,23 @@ int wide_solve_batched(ia_context *ctx, int m, int n, int batch, const double2 *
     const bool started = wide_started(ctx, m);
     int *done = nullptr;
     if (started) {
-        double2 *M = cur.take<double2>((size_t)N * N * batch);
         done = cur.take<int>((size_t)batch);
-        if ((st = jacobi_precondition_batched(ctx, N, Rg, N + nrhs, M, done, batch, info, cur))) return st;
+        double2 *M = Y;   // R is in Rg, Y (Mr >= N rows) is free
+        // the largest group of bins that the scratch holds
+        const size_t room = cur.cap > cur.off ? cur.cap - cur.off : 0;
+        int lo = 0, hi = batch;
+        while (lo < hi) {
+            const int g = (lo + hi + 1) / 2;
+            if (jacobi_precondition_ws_bytes(N, g) <= room) lo = g;
+            else hi = g - 1;
+        }
+        if (lo < 1) return IA_ERR_ALLOC;
+        const int groups = (batch + lo - 1) / lo, g = (batch + groups - 1) / groups;
+        for (int f0 = 0; f0 < batch; f0 += g)
+            if ((st = jacobi_precondition_batched(ctx, N, Rg + (size_t)f0 * (N + nrhs) * N, N + nrhs,
+                                                  M + (size_t)f0 * N * N, done + f0, batch - f0 < g ? batch - f0 : g,
+                                                  info ? info + f0 : nullptr, cur)))
+                return st;
         Rg = M;
     }
     const int rows = started ? N : N + nrhs;
