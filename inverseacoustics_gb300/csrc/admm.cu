@@ -418,12 +418,10 @@ static int admm_launch(ia_context *ctx, bool dual, int cs, size_t smem, int bloc
     lc.attrs = at;
     lc.numAttrs = cs > 1 ? 1 : 0;
     if (dual) {
-        IA_CUDA_TRY(cudaFuncSetAttribute(admm_kernel<AR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         200 * 1024));
+        IA_CUDA_TRY(allow_shared(admm_kernel<AR, true>));
         IA_CUDA_TRY(cudaLaunchKernelEx(&lc, admm_kernel<AR, true>, a, cs));
     } else {
-        IA_CUDA_TRY(cudaFuncSetAttribute(admm_kernel<AR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         200 * 1024));
+        IA_CUDA_TRY(allow_shared(admm_kernel<AR, false>));
         IA_CUDA_TRY(cudaLaunchKernelEx(&lc, admm_kernel<AR, false>, a, 1));
     }
     IA_LAUNCH_CHECK(ctx);

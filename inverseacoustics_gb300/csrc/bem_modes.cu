@@ -520,8 +520,7 @@ int bem_modes_batched(ia_context *ctx, const ia_mesh *mesh, int l, const double 
             const size_t smem = sizeof(double2) * ((size_t)m + nm) + (sizeof(double) + sizeof(int)) * (size_t)c.nr;
             if (smem > 227 * 1024) return IA_ERR_TOO_LARGE;
             if (smem > 48 * 1024)
-                IA_CUDA_TRY(cudaFuncSetAttribute(modes_pick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem));
+                IA_CUDA_TRY(allow_shared_all(modes_pick_kernel));
             modes_pick_kernel<<<F, PICK_THREADS, smem, ctx->stream>>>(m, nm, c.nr, V2, lam2, Uc, sr, info);
         } else {
             // FP64 SVD of Y: columns orthogonalised in place, U = Y / sigma

@@ -521,8 +521,7 @@ int getrf_batched(ia_context *ctx, int n, T *A, int lda, long long sA, int *ipiv
     constexpr size_t kPanelSmemMax = 200 * 1024;
     const bool smem_panel = (size_t)n * LU_NB * sizeof(T) <= kPanelSmemMax;
     if (smem_panel)
-        IA_CUDA_TRY(cudaFuncSetAttribute(lu_panel_smem_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kPanelSmemMax));
+        IA_CUDA_TRY(allow_shared<(int)kPanelSmemMax>(lu_panel_smem_kernel<T>));
     for (int k0 = 0; k0 < n; k0 += LU_NB) {
         int kend = k0 + LU_NB < n ? k0 + LU_NB : n;
         int nb = kend - k0;
@@ -787,7 +786,7 @@ int getrs_batched(ia_context *ctx, int n, int nrhs, const T *LU, int lda, long l
         if (smem <= 200 * 1024) {
             auto kern = getrs_fused_kernel<rb, nt>;
             if (smem > 48 * 1024)
-                IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+                IA_CUDA_TRY(allow_shared(kern));
             dim3 gf((nrhs + rb - 1) / rb, batch);
             kern<<<gf, nt, smem, ctx->stream>>>(n, nrhs, LU, lda, sA, ipiv, B, ldb, sB);
             IA_LAUNCH_CHECK(ctx);

@@ -109,6 +109,25 @@ int cuda_status(cudaError_t e);
         if (e__ != cudaSuccess) return ia::cuda_status(e__); \
     } while (0)
 
+// Dynamic shared memory above 48 KB has to be allowed for a kernel, and the limit
+// belongs to the function, not to the launch: set to each launch's own size, it is
+// lowered between another host thread's call and its launch, which then fails.  So
+// it is one value per kernel: BYTES, or all that the static part leaves.
+template <int BYTES = 200 * 1024, class K>
+cudaError_t allow_shared(K kernel)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
+}
+template <class K>
+cudaError_t allow_shared_all(K kernel)
+{
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   227 * 1024 - (int)a.sharedSizeBytes);
+}
+
 // workspace carving: returns IA_OK / IA_ERR_ALLOC
 // (`bytes`, or where the device has no more at least `least`; 0: bytes)
 int ws_reserve(ia_context *ctx, size_t bytes, size_t least = 0);

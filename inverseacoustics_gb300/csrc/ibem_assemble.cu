@@ -582,8 +582,7 @@ int ibem_rows(ia_context *ctx, const ia_mesh *mesh, int l, const double *mics, i
         const size_t fit = gtab_bytes / geom_row_bytes(mesh);
         const int chunk = fit < (size_t)rows ? (int)fit : rows;
         if (chunk < 1 || (chunk < rows && !build_gtab)) return IA_ERR_ARG;
-        IA_CUDA_TRY(cudaFuncSetAttribute(ibem_rows_kernel<dfl, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         220 * 1024));
+        IA_CUDA_TRY(allow_shared<220 * 1024>(ibem_rows_kernel<dfl, true>));
         for (int r0 = 0; r0 < rows; r0 += chunk) {
             const int nr = rows - r0 < chunk ? rows - r0 : chunk;
             if (build_gtab) {
@@ -601,16 +600,14 @@ int ibem_rows(ia_context *ctx, const ia_mesh *mesh, int l, const double *mics, i
         }
         return IA_OK;
     } else if (df32) {
-        IA_CUDA_TRY(cudaFuncSetAttribute(ibem_rows_kernel<dfl, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         220 * 1024));
+        IA_CUDA_TRY(allow_shared<220 * 1024>(ibem_rows_kernel<dfl, false>));
         ibem_rows_kernel<dfl, false><<<g, IBEM_THREADS, smem, ctx->stream>>>(
             m, mesh->n, l, n_ch, 0, mesh->ncolors, F, mesh->d_nodes, mesh->d_egeo, (const dfl *)mesh->d_qdat_f,
             (const dfl *)mesh->d_qnrm_f, mesh->d_evert, mesh->d_color_ptr, mesh->d_adj_ptr, mesh->d_adj, mesh->nq,
             mesh->d_reg, mesh->d_sing, mesh->nqs, mics, cp, k, c, rho, coef, red, mesh->d_dftab, split_ab ? 1 : 0,
             mesh->d_creg, nullptr, At, Bt, Ahs_t, Bhs_t);
     } else {
-        IA_CUDA_TRY(cudaFuncSetAttribute(ibem_rows_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         220 * 1024));
+        IA_CUDA_TRY(allow_shared<220 * 1024>(ibem_rows_kernel<double, false>));
         ibem_rows_kernel<double, false><<<g, IBEM_THREADS, smem, ctx->stream>>>(
             m, mesh->n, l, n_ch, 0, mesh->ncolors, F, mesh->d_nodes, mesh->d_egeo, mesh->d_qdat, mesh->d_qnrm,
             mesh->d_evert, mesh->d_color_ptr, mesh->d_adj_ptr, mesh->d_adj, mesh->nq, mesh->d_reg, mesh->d_sing,

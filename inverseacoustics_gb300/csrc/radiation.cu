@@ -539,7 +539,7 @@ static bool rqr_cluster_launch(ia_context *ctx, int rows, int cols, T *Y, T *tau
     st = IA_OK;
     cudaError_t e = cudaSuccess;
     if (smem > 48 * 1024)
-        e = cudaFuncSetAttribute(rqr_cluster_kernel<T, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = allow_shared(rqr_cluster_kernel<T, CS>);
     if (e == cudaSuccess) {
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3((unsigned)(CS * batch));
@@ -635,8 +635,7 @@ static int orthonormalise(ia_context *ctx, int rows, int cols, T *Y, T *tau, T *
     const size_t fsm = sizeof(T) * (size_t)(FQ_COLS + 2) * rows;
     if (fsm <= 200 * 1024) {
         if (fsm > 48 * 1024)
-            IA_CUDA_TRY(cudaFuncSetAttribute(rform_q_group_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)fsm));
+            IA_CUDA_TRY(allow_shared(rform_q_group_kernel<T>));
         dim3 g(batch, (cols + FQ_COLS - 1) / FQ_COLS);
         rform_q_group_kernel<T><<<g, 32 * FQ_COLS, fsm, ctx->stream>>>(rows, cols, Y, tau, Q);
     } else {
@@ -1087,7 +1086,7 @@ static int radiation_modes_group(ia_context *ctx, int n, int F, const double *R,
     if (rjs <= 200 * 1024) {
         double *Xr = reinterpret_cast<double *>(Ysvd);
         if (rjs > 48 * 1024)
-            IA_CUDA_TRY(cudaFuncSetAttribute(rsym_jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rjs));
+            IA_CUDA_TRY(allow_shared(rsym_jacobi_kernel));
         rsym_jacobi_kernel<<<F, RJ_THREADS, rjs, ctx->stream>>>(b, B, Xr, s, 16, info);
         IA_LAUNCH_CHECK(ctx);
         sort_eig_real_kernel<<<F, 256, sizeof(int) * (size_t)b, ctx->stream>>>(b, s, Xr, Vc);

@@ -79,7 +79,7 @@ int regularize_batched(ia_context *ctx, int m, int n, int p, int batch, const do
     if (int st = check_method(*cfg, p)) return st;
     size_t smem = sizeof(double) * (size_t)p * 2 + sizeof(double2) * (size_t)p + sizeof(double) * (size_t)cfg->gcv_points;
     if (smem > 200 * 1024) return IA_ERR_TOO_LARGE;
-    IA_CUDA_TRY(cudaFuncSetAttribute(regularize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    IA_CUDA_TRY(allow_shared(regularize_kernel));
     dim3 g(batch, nrhs);
     regularize_kernel<<<g, REG_THREADS, smem, ctx->stream>>>(m, n, p, U, s, V, nrhs, b, *cfg, x, lambda);
     IA_LAUNCH_CHECK(ctx);
@@ -127,7 +127,7 @@ int gcv_beta_batched(ia_context *ctx, int m, int p, int batch, const double *s, 
     if (int st = check_method(*cfg, p)) return st;
     size_t smem = sizeof(double) * ((size_t)p * 2 + (size_t)cfg->gcv_points);
     if (smem > 200 * 1024) return IA_ERR_TOO_LARGE;
-    IA_CUDA_TRY(cudaFuncSetAttribute(gcv_beta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    IA_CUDA_TRY(allow_shared(gcv_beta_kernel));
     dim3 g(batch, nrhs);
     gcv_beta_kernel<<<g, REG_THREADS, smem, ctx->stream>>>(m, p, s, nrhs, beta, bnorm2, *cfg, z, lambda);
     IA_LAUNCH_CHECK(ctx);

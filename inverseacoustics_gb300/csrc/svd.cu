@@ -977,7 +977,7 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
     // without accumulator: a half-warp per pair (FP32: every pair of a round at
     // once in 32 warps; FP64: 16 warps, the 128-register budget), Y in shared
     // memory up to the per-CTA limit (an FP64 121 x 120 system fits)
-    const size_t half_smem_max = sizeof(T) <= 8 ? 200 * 1024 : 227 * 1024 - 64;   // 16 B static besides
+    constexpr size_t half_smem_max = sizeof(T) <= 8 ? 200 * 1024 : 227 * 1024 - 64;   // 16 B static besides
     {
         // over a cluster per bin: FP32 for batches that leave most of the GPU
         // idle and for the last part of a staggered pipeline (4x the SMs for
@@ -1013,8 +1013,7 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
                     if (np % c || np / c < 2 || c * batch > ctx->sm_count) continue;
                     configure(c);
                     if (lc.dynamicSmemBytes > 48 * 1024)
-                        IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)lc.dynamicSmemBytes));
+                        IA_CUDA_TRY(allow_shared(kern));
                     int fit = 0;
                     IA_CUDA_TRY(cudaOccupancyMaxActiveClusters(&fit, kern, &lc));
                     if (fit >= batch) {
@@ -1031,8 +1030,7 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
             configure(cs);
             kern = kpl == 17 ? jacobi_cluster_kernel<T, 17> : kpl == 12 ? jacobi_cluster_kernel<T, 12> : kern;
             if (lc.dynamicSmemBytes > 48 * 1024)
-                IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)lc.dynamicSmemBytes));
+                IA_CUDA_TRY(allow_shared(kern));
             IA_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, M, Mdot, N, N + (N & 1), Y, sY, max_sweeps, tol, info, skip,
                                            (const unsigned char *)nullptr, (float4 *)nullptr, (int *)nullptr));
             IA_LAUNCH_CHECK(ctx);
@@ -1045,15 +1043,13 @@ int jacobi_rows_batched(ia_context *ctx, int M, int Mdot, int N, T *Y, T *V, int
         int nws = (pairs + 1) / 2;
         if (nws > wcap) nws = wcap;
         if (nws < 1) nws = 1;
-        IA_CUDA_TRY(cudaFuncSetAttribute(jacobi_half_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)half_smem_max));
+        IA_CUDA_TRY(allow_shared<(int)half_smem_max>(jacobi_half_kernel<T>));
         jacobi_half_kernel<T><<<batch, nws * 32, smem, ctx->stream>>>(M, Mdot, N, Y, sY, max_sweeps, tol, info, skip);
     } else if (M <= 128 && N <= 128 && smem <= 200 * 1024) {
         const int wmax = sizeof(T) <= 8 ? 2 * SVD_MAX_WARPS : SVD_MAX_WARPS;
         int nws = (N + 1) / 2 < wmax ? (N + 1) / 2 : wmax;
         if (nws < 1) nws = 1;
-        IA_CUDA_TRY(cudaFuncSetAttribute(jacobi_smem_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         200 * 1024));
+        IA_CUDA_TRY(allow_shared(jacobi_smem_kernel<T, 4>));
         jacobi_smem_kernel<T, 4><<<batch, nws * 32, smem, ctx->stream>>>(M, Mdot, N, Y, sY, V, sV, max_sweeps, tol,
                                                                          info);
     } else if (M <= 128)
@@ -1113,7 +1109,7 @@ static int jc_launch(ia_context *ctx, int N, T *Y, int batch, int max_sweeps, ty
                           (MODE == JC_FLAGGED ? sizeof(unsigned) * (size_t)N2 * ((P + 31) / 32) : 0);
     at[0].val.clusterDim.x = cs;
     if (lc.dynamicSmemBytes > 48 * 1024)
-        IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lc.dynamicSmemBytes));
+        IA_CUDA_TRY(allow_shared(kern));
     IA_CUDA_TRY(cudaLaunchKernelEx(&lc, kern, N, N, N, N2, Y, (long long)N * N, max_sweeps, tol, (int *)nullptr, skip,
                                    flags, rec, sweeps));
     IA_LAUNCH_CHECK(ctx);
@@ -1153,7 +1149,7 @@ int jacobi_start_batched(ia_context *ctx, int N, float2 *Y, float2 *J, int batch
     auto apply = N2 <= 64    ? jacobi_apply_kernel<1>
                  : N2 <= 128 ? jacobi_apply_kernel<2>
                              : jacobi_apply_kernel<JA_MAX_CHUNKS>;
-    IA_CUDA_TRY(cudaFuncSetAttribute(apply, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    IA_CUDA_TRY(allow_shared(apply));
     for (int f0 = 0; f0 < batch; f0 += fit) {
         const int nf = batch - f0 < fit ? batch - f0 : fit;
         const size_t o = (size_t)f0 * N * N;

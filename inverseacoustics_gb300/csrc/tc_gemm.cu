@@ -62,7 +62,7 @@ constexpr uint64_t TC_WAIT_NS = 2000000000ull;
 constexpr uint32_t TC_A_SLICE = TC_BM * TC_BK * 2;   // bytes of one slice's A tile
 __host__ __device__ constexpr uint32_t tc_b_slice(int S) { return tc_bn(S) * TC_BK * 2; }
 
-size_t tc_smem_bytes(int S) { return (size_t)TC_STAGES * S * (TC_A_SLICE + tc_b_slice(S)) + 1024; }
+constexpr size_t tc_smem_bytes(int S) { return (size_t)TC_STAGES * S * (TC_A_SLICE + tc_b_slice(S)) + 1024; }
 
 // ---------------------------------------------------------------------------
 // slicing
@@ -960,7 +960,7 @@ int gemm_launch(ia_context *ctx, const CUtensorMap &ta, const CUtensorMap &tb, c
                 int M, int N, double alpha, double beta, TC *C, int ldc, long long sC, int batch, int *info)
 {
     const size_t smem = tc_smem_bytes(S);
-    IA_CUDA_TRY(cudaFuncSetAttribute(tc_gemm_kernel<S, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    IA_CUDA_TRY(allow_shared<(int)tc_smem_bytes(S)>(tc_gemm_kernel<S, REAL>));
     dim3 grid(((REAL ? 1 : 2) * N + tc_bn(S) - 1) / tc_bn(S), (M + TC_BM - 1) / TC_BM, batch);
     tc_gemm_kernel<S, REAL><<<grid, TC_THREADS, smem, ctx->stream>>>(ta, tb, M, N, A.Kp, A.e, B.e, alpha, beta, C,
                                                                       ldc, sC, info);
@@ -989,8 +989,7 @@ int gemm_wide_launch(ia_context *ctx, const TcPlanes &A, const TcPlanes &B, int 
     int st = make_tmap(&ta, A.p, A.Kp, A.rows, A.S, batch, TC_BM, true);
     if (!st) st = make_tmap(&tb, B.p, B.Kp, B.rows, B.S, batch, TW_BN, true);
     if (st) return st;
-    IA_CUDA_TRY(cudaFuncSetAttribute(tc_gemm_wide_kernel<REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)TW_SMEM));
+    IA_CUDA_TRY(allow_shared<(int)TW_SMEM>(tc_gemm_wide_kernel<REAL>));
     dim3 grid(((REAL ? 1 : 2) * N + TW_BN - 1) / TW_BN, (M + TC_BM - 1) / TC_BM, batch);
     tc_gemm_wide_kernel<REAL><<<grid, TW_THREADS, TW_SMEM, ctx->stream>>>(ta, tb, M, N, A.Kp, A.e, B.e, alpha, beta, C,
                                                                           ldc, sC, info);
@@ -1005,8 +1004,7 @@ int slice_launch(ia_context *ctx, const SliceOp<Src> &a, const SliceOp<Src> *b, 
     const size_t smem1 = sizeof(Src) * SL1_RB * (size_t)sl1_stride(Kp >> 1);
     if (smem1 <= 200 * 1024) {
         if (smem1 > 48 * 1024)
-            IA_CUDA_TRY(cudaFuncSetAttribute(tc_slice1_kernel<Src, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem1));
+            IA_CUDA_TRY(allow_shared(tc_slice1_kernel<Src, S>));
         dim3 grid((rmax + SL1_RB - 1) / SL1_RB, batch, b ? 2 : 1);
         tc_slice1_kernel<Src, S><<<grid, SL1_THREADS, smem1, ctx->stream>>>(a, b ? *b : a, K, Kp);
         IA_LAUNCH_CHECK(ctx);
@@ -1142,7 +1140,7 @@ int tc_slice_real(ia_context *ctx, bool role_b, Op op, const double *X, int ld, 
     if (cur.off > cur.cap) return IA_ERR_ALLOC;
     const size_t smem = sizeof(double) * SL1_RB * (size_t)slr_stride(Kp);
     if (smem > 48 * 1024)
-        IA_CUDA_TRY(cudaFuncSetAttribute(tc_slice_real_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        IA_CUDA_TRY(allow_shared(tc_slice_real_kernel));
     // view V(r, k): the A role reads rows of op(A), the B role columns of op(B)
     const bool rcontig = role_b ? op != OP_N : op == OP_N;
     tc_slice_real_kernel<<<dim3((R + SL1_RB - 1) / SL1_RB, batch), SL1_THREADS, smem, ctx->stream>>>(

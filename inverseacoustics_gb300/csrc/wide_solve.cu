@@ -480,7 +480,7 @@ static int qr_launch_t(ia_context *ctx, int rows, int cols, T *A, int lda, long 
         const size_t csm = qr_cluster_smem(rows, cols);
         if (!B && rows <= 1 + 32 * QR_KPL && cols >= 2 * QRC_CS && csm <= 227 * 1024 &&
             (4 * QRC_CS * batch <= ctx->sm_count || ctx->tail_part)) {
-            IA_CUDA_TRY(cudaFuncSetAttribute(qr_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
+            IA_CUDA_TRY(allow_shared_all(qr_cluster_kernel));
             cudaLaunchConfig_t lc = {};
             lc.gridDim = dim3((unsigned)(QRC_CS * batch));
             lc.blockDim = dim3(QRC_THREADS);
@@ -503,16 +503,14 @@ static int qr_launch_t(ia_context *ctx, int rows, int cols, T *A, int lda, long 
         const size_t smem = sizeof(T) * (size_t)rows + piv;
         if (smem > 48 * 1024) {
             if (smem > 227 * 1024) return IA_ERR_TOO_LARGE;
-            IA_CUDA_TRY(cudaFuncSetAttribute(qr_kernel<T, QR_KPL, PIV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem));
+            IA_CUDA_TRY(allow_shared_all(qr_kernel<T, QR_KPL, PIV>));
         }
         qr_kernel<T, QR_KPL, PIV><<<batch, QR_THREADS, smem, ctx->stream>>>(rows, cols, A, lda, sA, tau, nrhs, B,
                                                                            ldb, sB, perm);
     } else {
         if (piv > 48 * 1024) {
             if (piv > 227 * 1024) return IA_ERR_TOO_LARGE;
-            IA_CUDA_TRY(cudaFuncSetAttribute(qr_kernel<T, 0, PIV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)piv));
+            IA_CUDA_TRY(allow_shared_all(qr_kernel<T, 0, PIV>));
         }
         qr_kernel<T, 0, PIV><<<batch, QR_THREADS, piv, ctx->stream>>>(rows, cols, A, lda, sA, tau, nrhs, B, ldb, sB,
                                                                      perm);
@@ -1571,8 +1569,7 @@ int herm_jacobi_batched(ia_context *ctx, int N, double2 *S, double2 *X, double *
             smem_cap = 1;
     }
     if (smem_s <= smem_cap && N < 65536) {
-        IA_CUDA_TRY(cudaFuncSetAttribute(herm_jacobi_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem_s));
+        IA_CUDA_TRY(allow_shared_all(herm_jacobi_kernel<true>));
         herm_jacobi_kernel<true><<<batch, HJ_THREADS, smem_s, ctx->stream>>>(N, S, X, LAM, max_sweeps, info);
         IA_LAUNCH_CHECK(ctx);
         return IA_OK;
@@ -1581,8 +1578,7 @@ int herm_jacobi_batched(ia_context *ctx, int N, double2 *S, double2 *X, double *
                         sizeof(int) * (size_t)N2 + sizeof(double) * (size_t)N;
     if (smem > 227 * 1024 - 512) return IA_ERR_TOO_LARGE;
     if (smem > 48 * 1024)
-        IA_CUDA_TRY(cudaFuncSetAttribute(herm_jacobi_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+        IA_CUDA_TRY(allow_shared_all(herm_jacobi_kernel<false>));
     herm_jacobi_kernel<false><<<batch, HJ_THREADS, smem, ctx->stream>>>(N, S, X, LAM, max_sweeps, info);
     IA_LAUNCH_CHECK(ctx);
     return IA_OK;

@@ -364,14 +364,13 @@ __global__ void __launch_bounds__(32 * ZT_RB) zlu_trsm_kernel(int nb, const doub
         if (lane + 32 * h < nb) x[lane + 32 * h] = v[h];
 }
 
-static size_t zt_smem_bytes() { return sizeof(double2) * (size_t)ZLU_NB * (ZT_LD + 1); }
+static constexpr size_t zt_smem_bytes() { return sizeof(double2) * (size_t)ZLU_NB * (ZT_LD + 1); }
 
 template <bool UPPER>
 static int ztrsm(ia_context *ctx, int nb, const double2 *T, int ldt, long long sT, double2 *X, int ldx, long long sX,
                  int ncols, int batch)
 {
-    IA_CUDA_TRY(cudaFuncSetAttribute(zlu_trsm_kernel<UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)zt_smem_bytes()));
+    IA_CUDA_TRY(allow_shared<(int)zt_smem_bytes()>(zlu_trsm_kernel<UPPER>));
     zlu_trsm_kernel<UPPER><<<dim3((ncols + ZT_RB - 1) / ZT_RB, batch), 32 * ZT_RB, zt_smem_bytes(), ctx->stream>>>(
         nb, T, ldt, sT, X, ldx, sX, ncols);
     IA_LAUNCH_CHECK(ctx);
@@ -460,7 +459,7 @@ int zgetrf_ws(ia_context *ctx, int n, double2 *A, int lda, long long sA, int *ip
               WsCursor scratch, bool plain)
 {
     if (!zlu_ok(ctx, n)) return zgetrf_batched(ctx, n, A, lda, sA, ipiv, info, batch);
-    IA_CUDA_TRY(cudaFuncSetAttribute(zlu_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZP_SMEM_MAX));
+    IA_CUDA_TRY(allow_shared<(int)ZP_SMEM_MAX>(zlu_panel_kernel));
     int st;
     const bool small = plain || (n > ZLU_NB && n <= ZLU_SMALL_N);
     const int NB = small ? ZLU_NB / 2 : ZLU_NB;

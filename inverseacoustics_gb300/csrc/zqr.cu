@@ -282,7 +282,7 @@ static int zqr_launch(ia_context *ctx, int rows, int cols, double2 *A, int lda, 
                 : rows <= 768  ? zqr_cluster_kernel<24, 2, PIV>
                 : rows <= 1280 ? zqr_cluster_kernel<40, 4, PIV>
                                : zqr_cluster_kernel<0, 1, PIV>;
-    IA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ZQ_SMEM_MAX));
+    IA_CUDA_TRY(allow_shared<(int)ZQ_SMEM_MAX>(kern));
     // The cluster size of least waves (cols / c + ZQ_STEP) among those with a
     // column per warp: a step's columns over the CTAs, plus what each CTA does for
     // itself (reflector, barrier: as long as about 16 columns of the update: 64
