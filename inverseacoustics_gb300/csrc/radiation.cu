@@ -34,7 +34,7 @@ namespace ia {
 //     and (j, i), which also makes R exactly symmetric.  A warp covers 8 rows x
 //     4 columns, so both stores fill whole 32-byte sectors without staging.
 //   - r, 1/r and the two or three sincos of an entry serve up to SR_CHUNK
-//     frequencies.
+//     frequencies (fewer for few radiators).
 //   - evenly spaced wavenumbers: frequencies go in blocks of 2 SR_J + 1 around a
 //     centre, sin(a +- j b) = sin a cos jb +- cos a sin jb giving two outputs
 //     for one multiply and two FMAs, and the centre advances by one rotation
@@ -46,7 +46,7 @@ namespace ia {
 //     than the factor 4 (a sweep from 1 Hz in either direction: 1e-14, without
 //     the two 1e-12).
 // 21 -> 2.8 FP64 instructions per stored value and half the entries: 64 bins of
-// 1280^2 in 0.57 ms (was 3.13 ms).  Below 4 frequencies, for unevenly spaced
+// 1280^2 in 0.56 ms (was 3.13 ms).  Below 4 frequencies, for unevenly spaced
 // wavenumbers and across k = 0, every phase is evaluated directly.
 // --------------------------------------------------------------------------
 constexpr int SR_TILE = 16;
@@ -54,7 +54,7 @@ constexpr int SR_J = 4, SR_BLK = 2 * SR_J + 1;
 constexpr int SR_CHUNK = 8 * SR_BLK;
 
 __global__ void __launch_bounds__(SR_TILE *SR_TILE) sinc_r_kernel(int n, const double *__restrict__ x, int F,
-                                                                  const double *__restrict__ kv, double pref,
+                                                                  const double *__restrict__ kv, int chunk, double pref,
                                                                   double *__restrict__ R)
 {
     __shared__ double sk[SR_CHUNK];
@@ -64,15 +64,18 @@ __global__ void __launch_bounds__(SR_TILE *SR_TILE) sinc_r_kernel(int n, const d
     while ((long long)ti * (ti + 1) / 2 > t) --ti;
     while ((long long)(ti + 1) * (ti + 2) / 2 <= t) ++ti;
     const int tj = t - (int)((long long)ti * (ti + 1) / 2);
-    const int f0 = blockIdx.y * SR_CHUNK, nf = min(SR_CHUNK, F - f0);
-    // in the order of increasing |k|
-    const bool down = fabs(kv[f0 + nf - 1]) < fabs(kv[f0]);
-    if (threadIdx.x < nf) sk[threadIdx.x] = kv[f0 + (down ? nf - 1 - (int)threadIdx.x : (int)threadIdx.x)];
+    const int f0 = blockIdx.y * chunk, nf = min(chunk, F - f0);
+    if (threadIdx.x < nf) sk[threadIdx.x] = kv[f0 + threadIdx.x];
     __syncthreads();
-    const double k0 = sk[0], dk = nf > 1 ? (sk[nf - 1] - k0) / (nf - 1) : 0.0;
+    // in the order of increasing |k|
+    const bool down = fabs(sk[nf - 1]) < fabs(sk[0]);
+    const double *ks = down ? sk + nf - 1 : sk;
+    const int kd = down ? -1 : 1;
+    auto kf = [&](int f) { return ks[kd * f]; };
+    const double k0 = kf(0), k1 = kf(nf - 1), dk = nf > 1 ? (k1 - k0) / (nf - 1) : 0.0;
     const bool odd_k = threadIdx.x < nf &&
-                       !(fabs(sk[threadIdx.x] - (k0 + threadIdx.x * dk)) <= 1e-12 * fabs(sk[threadIdx.x]));
-    const bool uniform = !__syncthreads_or(odd_k) && nf >= 4 && !(k0 * sk[nf - 1] < 0.0);
+                       !(fabs(kf(threadIdx.x) - (k0 + threadIdx.x * dk)) <= 1e-12 * fabs(kf(threadIdx.x)));
+    const bool uniform = !__syncthreads_or(odd_k) && nf >= 4 && !(k0 * k1 < 0.0);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int i = ti * SR_TILE + (wid & 1) * 8 + (lane & 7), j = tj * SR_TILE + (wid >> 1) * 4 + (lane >> 3);
     if (i >= n || j > i) return;
@@ -86,13 +89,13 @@ __global__ void __launch_bounds__(SR_TILE *SR_TILE) sinc_r_kernel(int n, const d
         up[f * step] = v;
     };
     if (r == 0.0) {
-        for (int f = 0; f < nf; ++f) put(f, pref * sk[f] * sk[f]);
+        for (int f = 0; f < nf; ++f) put(f, pref * kf(f) * kf(f));
         return;
     }
     // omega^2 rho A^2/(4 pi c) sin(kr)/(kr) = k (c rho A^2/(4 pi)) sin(kr)/r
     const double amp = pref / r;
     if (!uniform) {
-        for (int f = 0; f < nf; ++f) put(f, amp * sk[f] * sin(sk[f] * r));
+        for (int f = 0; f < nf; ++f) put(f, amp * kf(f) * sin(kf(f) * r));
         return;
     }
     double cj[SR_J], sj[SR_J];
@@ -117,13 +120,13 @@ __global__ void __launch_bounds__(SR_TILE *SR_TILE) sinc_r_kernel(int n, const d
     }
     for (int b = 0;; b += SR_BLK) {
         const int fc = b + SR_J;
-        if (fc < nf) put(fc, sk[fc] * s);
+        if (fc < nf) put(fc, kf(fc) * s);
 #pragma unroll
         for (int q = 0; q < SR_J; ++q) {
             const int fm = fc - 1 - q, fp = fc + 1 + q;
             const double p = s * cj[q];
-            if (fm < nf && (fm > 0 || !low)) put(fm, sk[fm] * fma(-c, sj[q], p));
-            if (fp < nf) put(fp, sk[fp] * fma(c, sj[q], p));
+            if (fm < nf && (fm > 0 || !low)) put(fm, kf(fm) * fma(-c, sj[q], p));
+            if (fp < nf) put(fp, kf(fp) * fma(c, sj[q], p));
         }
         if (b + SR_BLK >= nf) break;
         const double s1 = fma(s, cs, c * ss);
@@ -138,12 +141,16 @@ int sinc_resistance_batched(ia_context *ctx, int n, const double *x, int F, cons
     if (n <= 0 || F <= 0) return IA_OK;
     const double pref = c * rho * area * area * IA_INV4PI;
     const long long nt = (n + SR_TILE - 1) / SR_TILE;
-    const int chunks = (F + SR_CHUNK - 1) / SR_CHUNK;
+    // frequencies per CTA: fewer while the tiles leave SMs idle (4 radiators, 64 bins
+    // unevenly spaced: 64 us in one chunk, 18 in chunks of a block)
+    int chunk = SR_CHUNK;
+    while (chunk > SR_BLK && nt * (nt + 1) / 2 * ((F + chunk - 1) / chunk) < ctx->sm_count) chunk /= 2;
+    const int chunks = (F + chunk - 1) / chunk;
     for (int c0 = 0; c0 < chunks; c0 += 65535) {   // grid.y limit
         const int nc = min(65535, chunks - c0);
-        const int fo = c0 * SR_CHUNK;
+        const int fo = c0 * chunk;
         sinc_r_kernel<<<dim3((unsigned)(nt * (nt + 1) / 2), nc), SR_TILE * SR_TILE, 0, ctx->stream>>>(
-            n, x, F - fo, k + fo, pref, R + (size_t)fo * n * n);
+            n, x, F - fo, k + fo, chunk, pref, R + (size_t)fo * n * n);
         IA_LAUNCH_CHECK(ctx);
     }
     return IA_OK;

@@ -13,14 +13,14 @@ pytestmark = pytest.mark.gpu
 C, RHO = 343.0, 1.21
 
 
+@pytest.mark.parametrize("n", [35, 290])   # chunks of 9 bins, of 72
 @pytest.mark.parametrize("f0,f1,F", [(1.0, 2000.0, 64), (2000.0, 1.0, 64), (10000.0, 20.0, 64), (0.01, 2000.0, 30),
                                      (2000.0, 20.0, 200), (20.0, 2000.0, 150), (0.0, 900.0, 9), (900.0, 0.0, 9),
                                      (-100.0, 2000.0, 70), (-1.0, -2000.0, 40), (3000.0, 1.0, 4), (5.0, 5.0, 12)])
-def test_sinc_resistance_each_bin_to_its_size(cuda, ctx, f0, f1, F):
+def test_sinc_resistance_each_bin_to_its_size(cuda, ctx, f0, f1, F, n):
     from inverseacoustics_gb300 import api
     import torch
     rng = np.random.default_rng(F)
-    n = 35
     x = np.ascontiguousarray(rng.uniform(-0.16, 0.16, (3, n)))
     x[:, 20] = x[:, 4]
     x[:, 21] = x[:, 5] + 1e-4
