@@ -675,15 +675,15 @@ int ia_ibem_assemble_batch(ia_context *ctx, const ia_mesh *mesh, int l, const do
     if (gbytes) {
         const int st = ws_reserve(ctx, gbytes);
         if (st && st != IA_ERR_ALLOC) return st;
-        if (!st) G = reinterpret_cast<float2 *>(ctx->ws);   // no memory for it: the inline form, the same bits
+        if (!st) G = reinterpret_cast<float2 *>(ctx->ws);   // no memory for it: the inline form
     }
     return ibem_rows(ctx, mesh, l, d_mics, n_ch, d_cp, F, d_k, cfg->c, cfg->rho, (double2 *)d_At, (double2 *)d_Bt,
                      (double2 *)d_Ahs_t, (double2 *)d_Bhs_t, mixed, false, G, gbytes);
 }
 
 // Every ..._ws_bytes below: `least` is what the call can do with where the device
-// has no more: slice planes and starts for a bin at a time, no geometry table of
-// its own.  The results are the same bits.
+// has no more: slice planes and starts for a bin at a time (the same bits), no
+// geometry table of its own (equal to the double-float assembly's rounding).
 
 // slice planes of the FP64 transfer's solver and products
 static size_t transfer_fp64_ws_bytes(int m, int l, int F)
