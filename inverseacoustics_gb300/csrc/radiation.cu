@@ -141,10 +141,19 @@ int sinc_resistance_batched(ia_context *ctx, int n, const double *x, int F, cons
     if (n <= 0 || F <= 0) return IA_OK;
     const double pref = c * rho * area * area * IA_INV4PI;
     const long long nt = (n + SR_TILE - 1) / SR_TILE;
-    // frequencies per CTA: fewer while the tiles leave SMs idle (4 radiators, 64 bins
-    // unevenly spaced: 64 us in one chunk, 18 in chunks of a block)
+    // frequencies per CTA: fewer where the tiles leave SMs idle, by the CTAs of the
+    // fullest SM and a CTA's time in frequencies (12 us for 9, 30 for 72: 30 + chunk).
+    // 4 radiators, 64 bins unevenly spaced: 64 us in one chunk, 18 in chunks of a
+    // block; 130 radiators, 128 bins 30 us in chunks of 72, 34 of 36.
     int chunk = SR_CHUNK;
-    while (chunk > SR_BLK && nt * (nt + 1) / 2 * ((F + chunk - 1) / chunk) < ctx->sm_count) chunk /= 2;
+    long long least = 0;
+    for (int c = SR_CHUNK; c >= SR_BLK; c /= 2) {
+        const long long ctas = nt * (nt + 1) / 2 * ((F + c - 1) / c);
+        const long long cost = (ctas + ctx->sm_count - 1) / ctx->sm_count * (30 + min(c, F));
+        if (least && cost >= least) continue;
+        least = cost;
+        chunk = c;
+    }
     const int chunks = (F + chunk - 1) / chunk;
     for (int c0 = 0; c0 < chunks; c0 += 65535) {   // grid.y limit
         const int nc = min(65535, chunks - c0);
