@@ -242,7 +242,7 @@ int df_hi_batched(ia_context *ctx, size_t count, const float4 *in, float2 *out);
 #define TC_SLICES_MIN 6
 #define TC_SLICES_MAX 8
 #define TC_SLICES_DEFAULT 7
-#define TC_SLICES_FP64 10   // the FP64 path's products: rounding below an FP64 GEMM's
+#define TC_SLICES_FP64 10   // the FP64 path's products: 59 bits below a row's and a column's largest entry
 struct TcPlanes {
     __nv_bfloat16 *p;   // [batch][S][rows][Kp] BF16 digits
     int *e;             // [batch][R] power-of-two scale exponents

@@ -35,17 +35,15 @@
 
 namespace ia {
 
-// Sizes that take the start.  Solves of N x 4 N operators whose singular values
-// fall to the rounding level (the start's worst case: the tail's pairs still
-// rotate), GB300, without and with it: N = 48, 1 bin 3.33 / 3.46 ms, 150 bins
-// 7.95 / 9.04 ms; 64: 5.07 / 4.85 and 16.2 / 15.7 ms, 512 bins 62.1 / 49.9 ms;
-// 120: 17.9 / 15.0, 92 / 77 and 355 / 261 ms; 256: 104 / 87, 985 / 807 and
-// 3438 / 2822 ms.  The upper end is the recorded rotations' 128 slots.
-// (measured with the rotations still carried along: the figures below are
-// today's).  Operators above that level gain more: 64 microphones, one bin, the
-// whole ESM solve 4.7 -> 2.5 ms; 192 microphones, 48 bins 170 -> 61 ms; 64 order-15
-// HELS bins (256 x 256) 401 -> 51 to 57 ms, the more the more bins need the FP64
-// Jacobi's last sweep.
+// Sizes that take the start.  GCV solves of N x 4 N operators whose singular values
+// fall to the rounding level (the start's worst case: the tail's pairs still rotate),
+// without and with it, ms: N = 64, 1 bin 4.74 / 2.54, 150 bins 14.7 / 6.0, 512 bins
+// 55.7 / 19.5; 120: 15.7 / 6.3, 77.7 / 26.1, 308 / 90; 192: 43.4 / 14.7, 310 / 83;
+// 256: 88 / 27.6, 851 / 176; monopole operators gain more (64: 512 bins 55.5 / 17.4;
+// 120: 266 / 54).  Below 64 it would pay too (48: 3.15 / 2.08, 512 bins 26.7 / 11.3;
+// 40: 2.50 / 1.91, 17.7 / 9.3): the line is where an earlier form of the start was
+// level, and small arrays keep the digits they have.  The upper end is the recorded
+// rotations' 128 slots.
 constexpr int JS_MIN_N = 64, JS_MAX_N = 256;
 constexpr int JS_FP32_SWEEPS = 12;
 constexpr double JS_MAX_D = 1e-3;      // largest |D (I - J^H J) D^-1|_F: 63/256 of its fifth power = 2.5e-16
